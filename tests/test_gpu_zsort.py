@@ -94,3 +94,18 @@ def test_apply_zsort_errors(ob):
     assert ob.apply_zsort(tns, sid2, torch.zeros(50, device="cuda")).shape == (50,)
     with pytest.deprecated_call():
         ob.apply_zsort_(tns, sid, torch.zeros(100, device="cuda"))
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 256, 257, 1023])
+@pytest.mark.parametrize("rows,dtype", [(1, torch.float32), (3, torch.float32), (5, torch.float32), (3, torch.uint8),
+                                        (3, torch.int16), (3, torch.float64), (6, torch.float64), (16, torch.uint8)])
+def test_short_rows_at_warp_and_block_edges(ob, n, rows, dtype):
+    """Rows of one to four words of every width, and of one more, at the edges
+    of a warp's and a block's rows; both directions."""
+    x = uniform(n, 3, 907 + n)
+    tns, sid = built(ob, x, 0.2)
+    perm = tns.trees[sid - 1].arrays()["perm"].long() - 1
+    a = (torch.arange(rows * n, device="cuda") % 251).reshape(rows, n).to(dtype)
+    y = ob.apply_zsort(tns, sid, a)
+    assert torch.equal(y, a[:, perm])
+    assert torch.equal(ob.api._zsort_rows(tns, sid, y, 1), a)
