@@ -46,3 +46,20 @@ def test_sort_of_6_5m_keys_with_ties(ob, oracle_mod):
     tns, sid = gpu_run(ob, x, r)
     ot = oracle_mod.build_tree(x, r, nthreads=0)
     assert np.array_equal(tns.trees[sid - 1].arrays()["perm"].cpu().numpy(), ot.perm)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("ndims", [2, 3])
+@pytest.mark.parametrize("n", [1, 5, 2047, 2049, 10_001])
+def test_sort_of_coordinates_off_a_16_byte_boundary(ob, oracle_mod, n, ndims, dtype):
+    """Coordinates that start one point into an array (an address that is no
+    multiple of 16 for float32 3D and 2D and float64 3D): the wide loads and
+    copies of the digit counts and the first pass do not apply."""
+    whole = np.random.default_rng(n).random((n + 1, ndims)).astype(dtype)
+    x = np.ascontiguousarray(whole[1:])
+    r = dtype(0.03)
+    tns = ob.TNS(torch.float32 if dtype == np.float32 else torch.float64, ndims=ndims)
+    ob.set_search_radius_(tns, r)
+    sid = ob.add_point_set_(tns, torch.from_numpy(whole).cuda().t()[:, 1:])
+    ob.run_(tns)
+    assert_tree_equal(tns.trees[sid - 1], oracle_mod.build_tree(x, r))
