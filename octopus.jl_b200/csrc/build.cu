@@ -263,10 +263,9 @@ __global__ void __launch_bounds__(kThreads) k_gather(const T* __restrict__ coord
 // ---------------------------------------------------------- 5. topology --
 // Number of leading D-bit digits (of Dims<D>::bits) two keys share.
 template <int D, class K> __device__ __forceinline__ int common_levels(K a, K b) {
-    const uint64_t x = (uint64_t)(a ^ b);
-    if (x == 0) return Dims<D>::bits;
-    const int hb = 63 - __clzll((long long)x);
-    return Dims<D>::bits - 1 - hb / D;
+    // the highest differing bit, -1 for equal keys
+    const int hb = sizeof(K) == 4 ? 31 - __clz((int)(a ^ b)) : 63 - __clzll((long long)(a ^ b));
+    return Dims<D>::bits - (int)((unsigned)(hb + D) / (unsigned)D);
 }
 
 // Same, where keys of different clouds share no level (-1).
@@ -284,11 +283,21 @@ template <int D, class K> __device__ __forceinline__ int slot_digit(K key, int s
     return (int)((v >> shd) & (uint64_t)(Dims<D>::nch - 1));
 }
 
-constexpr int kMarkTile = kThreads;  // positions per block in mark / emit
+// Each warp of mark / emit takes kStrips consecutive strips of 32 positions
+// (both passes and their scan, 16M uniform / 1M lattice points: 342 / 41 us
+// with one position per thread and the keys and counters in shared memory,
+// 243 / 35 us with 1 strip, 198 / 32 with 2, 191 / 36 with 4).
+constexpr int kStrips = 2;
+constexpr int kMarkTile = kThreads * kStrips;  // positions per block
 
 // lohi[k] = lo | hi << 8: the levels whose node starts at position k are
 // lo..hi (empty when lo > hi); hi is the level of the leaf containing k
 // (src/cpu/build_cpu.jl:146: leaf iff count <= 32 or level >= max_levels).
+// Also counts the block's nodes per level.
+//
+// A lane holds the same lane of kStrips + 2 consecutive strips, so the levels
+// that positions j and j + 32 share are one comparison of two of its
+// registers.  Bound by instructions.
 template <int D, class K>
 __global__ void __launch_bounds__(kThreads) k_mark(const K* __restrict__ skeys, int64_t n,
                                                    uint16_t* __restrict__ lohi, int32_t* __restrict__ blockcnt,
@@ -297,53 +306,48 @@ __global__ void __launch_bounds__(kThreads) k_mark(const K* __restrict__ skeys, 
     pdl_trigger();
     constexpr int MAXLEV = Dims<D>::bits;
     constexpr int NLEV = MAXLEV + 1;
-    __shared__ K sk[kMarkTile + 64];
-    __shared__ int8_t sc[kMarkTile + 32];
-    __shared__ int32_t wcnt[NLEV][kThreads / 32];
-    const int64_t base = (int64_t)blockIdx.x * kMarkTile;
-    for (int i = threadIdx.x; i < kMarkTile + 64; i += kThreads) {
-        const int64_t p = base - 32 + i;
-        sk[i] = (p >= 0 && p < n) ? skeys[p] : K(0);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kMarkTile + 32; i += kThreads) {
-        const int64_t j = base - 32 + i;
-        sc[i] = (j >= 0 && j + 32 <= n - 1) ? (int8_t)common_levels_b<D, K>(sk[i], sk[i + 32], bt) : (int8_t)-1;
-    }
-    __syncthreads();
-    const int64_t k = base + threadIdx.x;
+    static_assert(NLEV <= 32, "one counter per lane");
+    __shared__ int32_t cnt[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    // max of sc[x .. x + 32] for x = threadIdx.x: the suffix maximum of the
-    // warp's first 32 entries from this lane on, with the prefix maximum of
-    // the next 32 up to this lane
-    int sa = sc[threadIdx.x], pb = sc[threadIdx.x + 32];
+    if (threadIdx.x < 32) cnt[threadIdx.x] = 0;
+    __syncthreads();
+    const int64_t base = (int64_t)blockIdx.x * kMarkTile + w * (32 * kStrips) + lane;
+    // key[i]: position base + 32 (i - 1)
+    K key[kStrips + 2];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int a = __shfl_down_sync(0xffffffffu, sa, o);
-        const int b = __shfl_up_sync(0xffffffffu, pb, o);
-        if (lane + o < 32) sa = max(sa, a);
-        if (lane >= o) pb = max(pb, b);
+    for (int i = 0; i < kStrips + 2; ++i) {
+        const int64_t p = base + 32 * (i - 1);
+        key[i] = p >= 0 && p < n ? skeys[p] : K(0);
     }
-    int lo = 1, hi = 0;
-    if (k < n) {
-        lo = (k == 0) ? 0 : common_levels_b<D, K>(sk[threadIdx.x + 31], sk[threadIdx.x + 32], bt) + 1;
-        hi = min(max(sa, pb) + 1, MAXLEV);
-        lohi[k] = (uint16_t)(lo | (hi << 8));
+    // share[i]: levels shared by the positions of key[i] and key[i + 1]
+    int share[kStrips + 1];
+#pragma unroll
+    for (int i = 0; i < kStrips + 1; ++i) {
+        const int64_t p = base + 32 * (i - 1);
+        share[i] = p >= 0 && p + 32 < n ? common_levels_b<D, K>(key[i], key[i + 1], bt) : -1;
     }
-    // per-level node counts of the warp, over the levels its positions span
-    const int wlo = warp_min(lo <= hi ? lo : NLEV), whi = warp_max(lo <= hi ? hi : -1);
-    if (lane < NLEV && (lane < wlo || lane > whi)) wcnt[lane][w] = 0;
-    for (int L = wlo; L <= whi; ++L) {
-        const unsigned b = __ballot_sync(0xffffffffu, lo <= L && L <= hi);
-        if (lane == 0) wcnt[L][w] = __popc(b);
+#pragma unroll
+    for (int r = 0; r < kStrips; ++r) {
+        const int64_t k = base + 32 * r;
+        // the maximum over the 33 positions k - 32 .. k: the suffix of the
+        // strip before, with the prefix of this one (a shuffle past the end
+        // returns the lane's own value)
+        int sa = share[r], pb = share[r + 1];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            sa = max(sa, __shfl_down_sync(0xffffffffu, sa, o));
+            pb = max(pb, __shfl_up_sync(0xffffffffu, pb, o));
+        }
+        const K up = __shfl_up_sync(0xffffffffu, key[r + 1], 1), last = __shfl_sync(0xffffffffu, key[r], 31);
+        if (k < n) {
+            const int lo = k == 0 ? 0 : common_levels_b<D, K>(lane ? up : last, key[r + 1], bt) + 1;
+            const int hi = min(max(sa, pb) + 1, MAXLEV);
+            lohi[k] = (uint16_t)(lo | (hi << 8));
+            for (int L = lo; L <= hi; ++L) atomicAdd(&cnt[L], 1);
+        }
     }
     __syncthreads();
-    if (threadIdx.x < NLEV) {
-        int s = 0;
-#pragma unroll
-        for (int j = 0; j < kThreads / 32; ++j) s += wcnt[threadIdx.x][j];
-        blockcnt[(int64_t)threadIdx.x * nblocks + blockIdx.x] = s;
-    }
+    if (threadIdx.x < NLEV) blockcnt[(int64_t)threadIdx.x * nblocks + blockIdx.x] = cnt[threadIdx.x];
 }
 
 // Node (L, k) -> BFS id.  Writes nrange[id] = {k, L}, first_child[id] = the
@@ -359,65 +363,78 @@ __global__ void __launch_bounds__(kThreads) k_emit_ids(int64_t n, const uint16_t
     pdl_wait();
     pdl_trigger();
     constexpr int NLEV = Dims<D>::bits + 1;
-    __shared__ int32_t wpre[NLEV][kThreads / 32];
+    constexpr int NW = kThreads / 32;
+    // per warp and level: its nodes, then the next id
+    __shared__ int32_t next[NW][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t k = (int64_t)blockIdx.x * kMarkTile + threadIdx.x;
-    int lo = 1, hi = 0;
-    if (k < n) {
-        const uint16_t v = lohi[k];
-        lo = v & 0xff;
-        hi = v >> 8;
-    }
-    const int wlo = warp_min(lo <= hi ? lo : NLEV), whi = warp_max(lo <= hi ? hi : -1);
-    if (lane < NLEV && (lane < wlo || lane > whi)) wpre[lane][w] = 0;
-    for (int L = wlo; L <= whi; ++L) {
-        const unsigned b = __ballot_sync(0xffffffffu, lo <= L && L <= hi);
-        if (lane == 0) wpre[L][w] = __popc(b);
-    }
-    __syncthreads();
-    if (threadIdx.x < NLEV) {
-        int run = 0;
+    const int64_t base = (int64_t)blockIdx.x * kMarkTile + w * (32 * kStrips) + lane;
+    next[w][lane] = 0;
+    int v[kStrips + 1];  // lo | hi << 8 of this lane's positions, and of the position after the last strip
 #pragma unroll
-        for (int j = 0; j < kThreads / 32; ++j) {
-            const int c = wpre[threadIdx.x][j];
-            wpre[threadIdx.x][j] = run;
-            run += c;
-        }
-    }
+    for (int r = 0; r < kStrips; ++r) v[r] = base + 32 * r < n ? lohi[base + 32 * r] : 1;
+    v[kStrips] = lane == 0 && base + 32 * kStrips < n ? lohi[base + 32 * kStrips] : 1;
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < kStrips; ++r)
+        for (int L = v[r] & 0xff; L <= v[r] >> 8; ++L) atomicAdd(&next[w][L], 1);
     __syncthreads();
     if (hdr->n_nodes > capacity) {
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&hdr->status, (int)DF_NODE_OVERFLOW);
         return;
     }
-    int32_t prev = -1;
-    for (int L = whi; L >= wlo; --L) {
-        const bool in = lo <= L && L <= hi;
-        const unsigned b = __ballot_sync(0xffffffffu, in);
-        if (in) {
-            const int32_t id = (int32_t)(blockoff[(int64_t)L * nblocks + blockIdx.x] + wpre[L][w] +
-                                         __popc(b & lanemask_lt()));
-            nrange[id] = make_int2((int)k, L);
-            first_child[id] = L < hi ? prev : -1;
-            if (L == 0 && bt.n_clouds) bt.croot[cloud_of_position(bt, k)] = id;
-            prev = id;
+    if (threadIdx.x < NLEV) {
+        int32_t run = (int32_t)blockoff[(int64_t)threadIdx.x * nblocks + blockIdx.x];
+#pragma unroll
+        for (int j = 0; j < NW; ++j) {
+            const int32_t c = next[j][threadIdx.x];
+            next[j][threadIdx.x] = run;
+            run += c;
         }
     }
-    // Node ends.  A level-L node ends where the level-L key prefix changes,
-    // so the nodes holding position k that end at k + 1 are those of levels
+    __syncthreads();
+    // Node ends.  A level-L node ends where the level-L key prefix changes, so
+    // the nodes holding position k that end at k + 1 are those of levels
     // lo(k + 1) .. hi(k) (every level at the end of the array).  The level-L
-    // node holding k is the last one starting at or before k: its id is k's
-    // inclusive rank among the level-L starts, minus one.
-    int nlo = __shfl_down_sync(0xffffffffu, lo, 1);  // lo(k + 1)
-    if (lane == 31 && k + 1 < n) nlo = lohi[k + 1] & 0xff;
-    if (k + 1 >= n) nlo = 0;
-    const bool ends = k < n && nlo <= hi;
-    const int elo = warp_min(ends ? nlo : NLEV), ehi = warp_max(ends ? hi : -1);
-    for (int L = elo; L <= ehi; ++L) {
-        const unsigned b = __ballot_sync(0xffffffffu, lo <= L && L <= hi);
-        if (ends && nlo <= L && L <= hi) {
-            const int32_t id = (int32_t)(blockoff[(int64_t)L * nblocks + blockIdx.x] + wpre[L][w] +
-                                         __popc(b & lanemask_lt()) + (int)((b >> lane) & 1u) - 1);
-            node_end[id] = (int32_t)(k + 1);
+    // node holding k is the last one starting at or before k.
+    int nlo[kStrips], from = NLEV, to = -1;
+#pragma unroll
+    for (int r = 0; r < kStrips; ++r) {
+        const int64_t k = base + 32 * r;
+        const int nv = __shfl_down_sync(0xffffffffu, v[r], 1), nv0 = __shfl_sync(0xffffffffu, v[r + 1], 0);
+        nlo[r] = k >= n ? NLEV : k + 1 == n ? 0 : (lane == 31 ? nv0 : nv) & 0xff;
+        const int lo = min(v[r] & 0xff, nlo[r]), hi = v[r] >> 8;
+        if (lo <= hi) {
+            from = min(from, lo);
+            to = max(to, hi);
+        }
+    }
+    from = __reduce_min_sync(0xffffffffu, from);
+    to = __reduce_max_sync(0xffffffffu, to);
+    // All strips of a level together, levels downward (a node's first child is
+    // the next level's node at the same position).
+    int32_t prev[kStrips];
+#pragma unroll
+    for (int r = 0; r < kStrips; ++r) prev[r] = -1;
+    for (int L = to; L >= from; --L) {
+        unsigned b[kStrips];
+#pragma unroll
+        for (int r = 0; r < kStrips; ++r)
+            b[r] = __ballot_sync(0xffffffffu, (v[r] & 0xff) <= L && L <= v[r] >> 8);
+        int32_t first = next[w][L];
+#pragma unroll
+        for (int r = 0; r < kStrips; ++r) {
+            const int64_t k = base + 32 * r;
+            const int hi = v[r] >> 8;
+            const bool in = b[r] >> lane & 1u;
+            const int32_t id = first + __popc(b[r] & lanemask_lt());  // of a node starting here
+            if (in) {
+                nrange[id] = make_int2((int)k, L);
+                first_child[id] = L < hi ? prev[r] : -1;
+                if (L == 0 && bt.n_clouds) bt.croot[cloud_of_position(bt, k)] = id;
+                prev[r] = id;
+            }
+            if (nlo[r] <= L && L <= hi) node_end[in ? id : id - 1] = (int32_t)(k + 1);
+            first += __popc(b[r]);
         }
     }
 }

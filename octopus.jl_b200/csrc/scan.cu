@@ -96,25 +96,36 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_final(const In* in, int64
     }
 }
 
-// Short inputs in one launch: each thread sums, then writes, its own run of
-// consecutive elements (reading each element before writing it, so `in` and
-// `out` may alias).
+// Short inputs in one launch of one block: all inputs staged in shared memory
+// (so `in` and `out` may alias), then each thread's kSmallItems consecutive
+// ones.
 template <class In, class Out>
-__global__ void __launch_bounds__(kSmallScanThreads) k_scan_small(const In* in, int64_t n, Out* out,
+__global__ void __launch_bounds__(kSmallScanThreads) k_scan_small(const In* in, int n, Out* out,
                                                                   int64_t* __restrict__ d_total) {
     pdl_wait();
     pdl_trigger();
     __shared__ int64_t sm[kSmallScanThreads / 32 + 1];
-    const int64_t per = (n + kSmallScanThreads - 1) / kSmallScanThreads;
-    const int64_t b = (int64_t)threadIdx.x * per;
+    __shared__ In stage[kSmallScan];
+#pragma unroll
+    for (int it = 0; it < kSmallItems; ++it) {
+        const int j = it * kSmallScanThreads + threadIdx.x;
+        if (j < n) stage[j] = in[j];
+    }
+    __syncthreads();
+    const int b = threadIdx.x * kSmallItems;
+    In v[kSmallItems];
     int64_t sum = 0;
-    for (int64_t i = b; i < b + per && i < n; ++i) sum += in[i];
+#pragma unroll
+    for (int it = 0; it < kSmallItems; ++it) {
+        v[it] = b + it < n ? stage[b + it] : In(0);
+        sum += v[it];
+    }
     int64_t tot;
     int64_t run = block_exclusive_scan<int64_t>(sum, sm, &tot);
-    for (int64_t i = b; i < b + per && i < n; ++i) {
-        const In x = in[i];
-        out[i] = (Out)run;
-        run += x;
+#pragma unroll
+    for (int it = 0; it < kSmallItems; ++it) {
+        if (b + it < n) out[b + it] = (Out)run;
+        run += v[it];
     }
     if (threadIdx.x == 0) {
         out[n] = (Out)tot;
@@ -132,7 +143,7 @@ int exclusive_scan(const In* in, Out* out, int64_t n, int64_t* d_total, int64_t*
         return 0;
     }
     if (n <= kSmallScan) {
-        launch_pdl(k_scan_small<In, Out>, 1, kSmallScanThreads, 0, s, in, n, out, d_total);
+        launch_pdl(k_scan_small<In, Out>, 1, kSmallScanThreads, 0, s, in, (int)n, out, d_total);
         return 1;
     }
     const int ntiles = div_up(n, kScanTile);
