@@ -301,7 +301,9 @@ constexpr int kMarkTile = kThreads * kStrips;  // positions per block
 template <int D, class K>
 __global__ void __launch_bounds__(kThreads) k_mark(const K* __restrict__ skeys, int64_t n,
                                                    uint16_t* __restrict__ lohi, int32_t* __restrict__ blockcnt,
-                                                   int nblocks, Batch bt) {
+                                                   int nblocks, uint8_t* __restrict__ dstart,
+                                                   int32_t* __restrict__ bvh_arrive, int n_arrive, OctHeader* hdr,
+                                                   Batch bt) {
     pdl_wait();
     pdl_trigger();
     constexpr int MAXLEV = Dims<D>::bits;
@@ -343,6 +345,13 @@ __global__ void __launch_bounds__(kThreads) k_mark(const K* __restrict__ skeys, 
             const int lo = k == 0 ? 0 : common_levels_b<D, K>(lane ? up : last, key[r + 1], bt) + 1;
             const int hi = min(max(sa, pb) + 1, MAXLEV);
             lohi[k] = (uint16_t)(lo | (hi << 8));
+            // the search layout's flags and counters start at zero (sections 6, 7)
+            dstart[k] = 0;
+            if (k < n_arrive) bvh_arrive[k] = 0;
+            if (k == 0) {
+                hdr->n_groups = 0;
+                hdr->asc_key = 0;
+            }
             for (int L = lo; L <= hi; ++L) atomicAdd(&cnt[L], 1);
         }
     }
@@ -430,7 +439,6 @@ __global__ void __launch_bounds__(kThreads) k_emit_ids(int64_t n, const uint16_t
             if (in) {
                 nrange[id] = make_int2((int)k, L);
                 first_child[id] = L < hi ? prev[r] : -1;
-                if (L == 0 && bt.n_clouds) bt.croot[cloud_of_position(bt, k)] = id;
                 prev[r] = id;
             }
             if (nlo[r] <= L && L <= hi) node_end[in ? id : id - 1] = (int32_t)(k + 1);
@@ -439,6 +447,15 @@ __global__ void __launch_bounds__(kThreads) k_emit_ids(int64_t n, const uint16_t
     }
 }
 
+// What climbing the tree needs of a node, in one 16-byte load: its parent (-1
+// for a root; written by the parent's thread), its first child, and its
+// numbers of children (bits 0-7) and internal children (8-15), kLinkFull when
+// it covers its whole point set.
+struct alignas(16) NodeLink {
+    int32_t parent, pad, first, meta;
+};
+constexpr int kLinkFull = 1 << 16;
+
 // Completes node `id`: its last position (from the end k_emit_ids left in
 // `arrive`, which is then reset for the refit), its occupied child slots and
 // the children's parent links.
@@ -446,9 +463,9 @@ template <class T, int D, class K>
 __global__ void __launch_bounds__(kThreads) k_emit_nodes(const K* __restrict__ skeys, int64_t n, int64_t capacity,
                                                          const int32_t* __restrict__ first_child_in,
                                                          TNode<T, D>* __restrict__ tnode, int2* __restrict__ nrange,
-                                                         int32_t* __restrict__ parent, int32_t* __restrict__ arrive,
-                                                         int32_t* __restrict__ chain, const int64_t* __restrict__ blockoff,
-                                                         int nblocks, const OctHeader* hdr, Batch bt) {
+                                                         NodeLink* __restrict__ link, int32_t* __restrict__ arrive,
+                                                         const int64_t* __restrict__ blockoff, int nblocks,
+                                                         OctHeader* hdr, Batch bt) {
     pdl_wait();
     pdl_trigger();
     constexpr int BITS = Dims<D>::bits;
@@ -470,6 +487,7 @@ __global__ void __launch_bounds__(kThreads) k_emit_nodes(const K* __restrict__ s
     }
     const int64_t e = arrive[id];  // the end written by k_emit_ids
     TNode<T, D> nd;
+    int inner = 0;  // internal children
     if (first_child < 0) {
         nd.a = (int32_t)k;
         nd.b = (int32_t)(e - k);
@@ -484,7 +502,8 @@ __global__ void __launch_bounds__(kThreads) k_emit_nodes(const K* __restrict__ s
             const int64_t cs = nrange[c].x;
             if (cs >= e) break;
             slots |= 1u << slot_digit<D, K>(skeys[cs], shd, bt);
-            parent[c] = (int32_t)id;
+            inner += first_child_in[c] >= 0;
+            link[c].parent = (int32_t)id;
         }
         nd.a = first_child;
         nd.b = -(int32_t)slots;
@@ -498,10 +517,6 @@ __global__ void __launch_bounds__(kThreads) k_emit_nodes(const K* __restrict__ s
         } else {
 #pragma unroll
             for (int d = 0; d < D; ++d) { nd.lo[d] = (T)hdr->gmin[d]; nd.hi[d] = (T)hdr->gmax[d]; }
-            // Full-range nodes form the root's chain: chain[L] = id, and
-            // chain[32 + L] = 1 when the node's only child sits in slot 0.
-            chain[L] = (int32_t)id;
-            chain[32 + L] = (nd.b == -1) ? 1 : 0;
         }
     } else {
 #pragma unroll
@@ -510,216 +525,409 @@ __global__ void __launch_bounds__(kThreads) k_emit_nodes(const K* __restrict__ s
     tnode[id] = nd;
     nrange[id] = make_int2((int)k, (int)(e - 1));
     arrive[id] = 0;
-    if (L == 0) parent[id] = -1;  // a root (one per cloud in a batch)
+    // the first node (in level-major order) whose first slot is empty: no
+    // ascending unit lies above it (section 6)
+    if (nd.b < 0 && !((unsigned)(-nd.b) & 1u) && 0x7fffffff - (int32_t)id > *(volatile int32_t*)&hdr->asc_key)
+        atomicMax(&hdr->asc_key, 0x7fffffff - (int32_t)id);
+    link[id].first = first_child;
+    link[id].meta = (nd.b < 0 ? __popc((unsigned)(-nd.b)) : 0) | inner << 8 | (k == s0 && e == s1 ? kLinkFull : 0);
+    if (L == 0) link[id].parent = -1;  // a root (one per cloud in a batch)
 }
 
-// ------------------------------------------------------------- 6. refit --
-// Leaves fold their points (src/cpu/refit_cpu.jl:39-48); the last child to
-// arrive at a parent folds the children (src/cpu/refit_cpu.jl:50-60).  No
-// thread waits: a thread that is not last simply stops.
-template <class T, int D>
-__global__ void __launch_bounds__(kThreads) k_refit(int64_t capacity, int64_t n, TNode<T, D>* tnode,
-                                                    const int2* __restrict__ nrange, const int32_t* __restrict__ parent,
-                                                    int32_t* arrive, const SPt<T, D>* __restrict__ spts,
-                                                    const OctHeader* hdr, Batch bt) {
-    pdl_wait();
-    pdl_trigger();
-    const int64_t nn = hdr->n_nodes;
-    const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (nn > capacity || id >= nn) return;
-    const int32_t a = tnode[id].a, b = tnode[id].b;
-    if (b <= 0) return;
-    T lo[D], hi[D];
-#pragma unroll
-    for (int d = 0; d < D; ++d) { lo[d] = T(INFINITY); hi[d] = T(-INFINITY); }
-    for (int32_t m = a; m < a + b; ++m) {
-        const SPt<T, D> p = spts[m];
-#pragma unroll
-        for (int d = 0; d < D; ++d) { lo[d] = jl_min(lo[d], p.x[d]); hi[d] = jl_max(hi[d], p.x[d]); }
-    }
-#pragma unroll
-    for (int d = 0; d < D; ++d) { tnode[id].lo[d] = lo[d]; tnode[id].hi[d] = hi[d]; }
-    int32_t node = (int32_t)id;
-    while (true) {
-        const int32_t p = parent[node];
-        if (p < 0) break;
-        const int2 rg = nrange[p];
-        int64_t s0 = 0, s1 = n;
-        if (bt.n_clouds) {
-            const int c = cloud_of_position(bt, rg.x);
-            s0 = bt.coff[c];
-            s1 = bt.coff[c + 1];
-        }
-        if (rg.x == s0 && (int64_t)rg.y == s1 - 1) break;  // bounds preset from the set's reduce
-        const int32_t pa = tnode[p].a, pb = tnode[p].b;
-        const int nc = __popc((unsigned)(-pb));
-        // Release this node's bounds and, for the last arrival, acquire its
-        // siblings' (one acquire-release read-modify-write, no full fences).
-        const int old = cuda::atomic_ref<int32_t, cuda::thread_scope_device>(arrive[p]).fetch_add(
-            1, cuda::memory_order_acq_rel);
-        if (old != nc - 1) break;
-#pragma unroll
-        for (int d = 0; d < D; ++d) { lo[d] = T(INFINITY); hi[d] = T(-INFINITY); }
-        for (int c = 0; c < nc; ++c) {
-            const TNode<T, D>* cn = tnode + pa + c;
-#pragma unroll
-            for (int d = 0; d < D; ++d) {
-                lo[d] = jl_min(lo[d], __ldcg(&cn->lo[d]));
-                hi[d] = jl_max(hi[d], __ldcg(&cn->hi[d]));
-            }
-        }
-#pragma unroll
-        for (int d = 0; d < D; ++d) { tnode[p].lo[d] = lo[d]; tnode[p].hi[d] = hi[d]; }
-        node = p;
-    }
-}
-
-// ------------------------------------------------------- 7. query groups --
-// A query group is a run of consecutive sibling leaves holding at most gmax
-// (<= 32, a tuned shape) points in total (a leaf of more than gmax points is
-// cut into chunks of gmax).  Siblings share a parent box, so a
-// group's points are spatially compact; a window of 32 consecutive sorted
-// positions can instead straddle a jump of the Morton curve and span the
-// whole domain.  Each node counts the groups formed under it, a warp reserves
-// room for its nodes' groups with one atomic on hdr->n_groups, and each node
-// writes its groups there.  The groups' order does not matter: every result
-// is per query point.
+// ------------------------------------- 6. leaf bounds and visiting order --
+// Visiting order: the reference's search pushes a node's children in slot
+// order onto a stack, so it visits them last slot first, except below an
+// internal node whose first slot is empty, which it scans as one leaf in
+// ascending position order (src/cpu/iterator_cpu.jl:74-116).  The order does
+// not depend on the query.  For a point at sorted position k let [s, e) be the
+// range of its unit: the highest such node above it, or else its leaf.  The
+// units of a point set holding positions [c0, c1) are visited in descending,
+// the points inside a unit in ascending position order, so the point's
+// visiting position is c0 + (c1 - e) + (k - s).  Each leaf copies its points
+// there (dpts), which makes everything a search meets one after another
+// contiguous in memory and ascending, and folds their bounds
+// (src/cpu/refit_cpu.jl:39-48).
 //
-// Each group also gets the node its traversal may start from (gstart, when
-// given): the deepest strict ancestor S of the group's parent P whose Morton
-// cell contains every cell within kStartMargin cells of P's cell.  The cell
-// size is the radius, so every point within the radius of a point of the group
-// (one cell, plus one for the rounding of the two binnings) lies in S's cell,
-// hence in S's subtree: a search from S meets every neighbor the search from
-// the root meets, and in the same order, since a depth-first search restricted
-// to a subtree visits it in the subtree's own order.  Bit 30 carries the
-// ascending-order flag that S's stack entry has in the search from the root
-// (some strict ancestor with its first child slot empty); -1 = start at the
-// root.  The test reads keys and topology only, so it holds for as long as the
-// keys do (the bounds-only refit keeps it).
-constexpr int kStartMargin = 2;
+// The same pass makes the chunks: a chunk is a run of sibling leaves of at
+// most gmax (<= 32, a tuned shape) points in total, or a piece of gmax points
+// of a larger leaf.  Siblings share a parent box, so a chunk's points are
+// spatially compact; 32 consecutive positions can instead straddle a jump of
+// the curve and span the whole domain.  dstart[p] = point count of the chunk
+// starting at visiting position p (kPiece set for a piece), else 0; a run's
+// box and dstart index go to rbox at the run's first leaf's node, dnode[p].
+//
+// A team of eight lanes per internal node handles its leaf children one after
+// another, eight points per load; the unit, the runs and the box of a node
+// whose children are all leaves are found once per node.  Warps take nodes
+// ids in strides (ids are level-major, so the internal nodes are
+// clustered).  Bounded below by 32n bytes read and written; bound by the
+// latency of a node's dependent loads.
+constexpr int kTeam = 8;
+// points per lane in flight (float: 32 per team, a whole leaf of at most 32)
+template <class T> constexpr int kTeamPtsOf = sizeof(T) == 4 ? 4 : 2;
+constexpr int kPiece = 0x80;
 
-template <int D, class K>
-__device__ __forceinline__ uint64_t axis_cell(K key, int d) {
-    return D == 3 ? compact_by_3((uint64_t)key >> d) : compact_by_2((uint64_t)key >> d);
+// This warp's next internal node (or any node of `todo`) for each team, -1 when none is left.
+__device__ __forceinline__ int32_t team_pick(unsigned& todo, int32_t id) {
+    const int team = (threadIdx.x & 31) / kTeam;
+    int pick = -1;
+#pragma unroll
+    for (int t = 0; t < 32 / kTeam; ++t) {
+        if (todo && t == team) pick = __ffs(todo) - 1;
+        todo &= todo - 1;
+    }
+    const int32_t q = __shfl_sync(0xffffffffu, id, pick & 31);
+    return pick < 0 ? -1 : q;
 }
 
-template <class T, int D, class K>
-__global__ void __launch_bounds__(kThreads) k_groups(const TNode<T, D>* __restrict__ tnode, int64_t capacity,
-                                                     int2* __restrict__ groups, int64_t group_cap,
-                                                     const int32_t* __restrict__ chain,
-                                                     const int32_t* __restrict__ parent, OctHeader* hdr, int gmax,
-                                                     const K* __restrict__ skeys, const int2* __restrict__ nrange,
-                                                     int32_t* __restrict__ gstart) {
+// Box of a team's lanes on order keys (integer min/max follow Julia's
+// min/max of finite values, -0.0 below +0.0), in every lane.
+template <class T, int D>
+__device__ __forceinline__ void team_fold(unsigned mask, typename OrdKey<T>::I* lo, typename OrdKey<T>::I* hi) {
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+#pragma unroll
+        for (int o = kTeam / 2; o > 0; o >>= 1) {
+            lo[d] = min(lo[d], __shfl_xor_sync(mask, lo[d], o));
+            hi[d] = max(hi[d], __shfl_xor_sync(mask, hi[d], o));
+        }
+    }
+}
+
+template <class T, int D>
+__device__ __forceinline__ void store_bounds(TNode<T, D>* nd, const typename OrdKey<T>::I* lo,
+                                             const typename OrdKey<T>::I* hi) {
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+        nd->lo[d] = OrdKey<T>::value(lo[d]);
+        nd->hi[d] = OrdKey<T>::value(hi[d]);
+    }
+}
+
+template <class T, int D>
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1) k_layout(int64_t capacity, int64_t n, TNode<T, D>* __restrict__ tnode,
+                                                     const int2* __restrict__ nrange,
+                                                     const NodeLink* __restrict__ link,
+                                                     const SPt<T, D>* __restrict__ spts, SPt<T, D>* __restrict__ dpts,
+                                                     uint8_t* __restrict__ dstart, int32_t* __restrict__ dnode,
+                                                     TNode<float, D>* __restrict__ rbox, int gmax,
+                                                     const OctHeader* hdr,
+                                                     Batch bt) {
     pdl_wait();
     pdl_trigger();
+    using K = OrdKey<T>;
+    using I = typename K::I;
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int kTeamPts = kTeamPtsOf<T>;
     const int64_t nn = hdr->n_nodes;
-    const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id == 0 && nn <= capacity) {
-        // The DFS may start at the first chain node that is not an internal
-        // node with a single child in slot 0: every node above it covers all
-        // points (its box holds every query) and keeps descending order.
-        int L = 0;
-        while (L < 32 && chain[32 + L] == 1) ++L;
-        hdr->dfs_start = chain[L];
-    }
-    if (nn > capacity || (int64_t)blockIdx.x * blockDim.x >= nn) return;  // block-uniform
-    const bool live = id < nn;
-    // pass 0 counts the node's groups, pass 1 writes them from `out`.
-    int64_t out = 0;
-    int32_t ng = 0;
-    int32_t start = -1;  // the traversal start of this node's groups
-    for (int pass = 0; pass < 2; ++pass) {
-        ng = 0;
-        if (pass && gstart && live && ng == 0) {
-            const TNode<T, D> nd = tnode[id];
-            if (nd.b <= 0) {
-                // P = this node: its level (depth) and the ancestors' chain
-                constexpr int BITS = Dims<D>::bits;
-                int32_t anc[BITS + 2];
-                int depth = 0;
-                for (int32_t a = (int32_t)id; a >= 0 && depth < BITS + 2; a = parent[a]) anc[depth++] = a;
-                const int lp = depth - 1;  // anc[0] = P at level lp, anc[lp] = root
-                const K kp = skeys[nrange[id].x];
-                constexpr int64_t cmax = (1LL << BITS) - 1;
-                int la = -1;  // deepest level whose cell holds P's cell +- kStartMargin
-                for (int L = lp - 1; L >= 1 && la < 0; --L) {
-                    const int sh = BITS - L;
-                    bool ok = true;
+    // After a sort whose wait ran out the ranges mean nothing (the build fails).
+    if (nn > capacity || (hdr->status & DF_TIMEOUT)) return;
+    const int32_t asc_min = 0x7fffffff - hdr->asc_key;  // no node above (before) this id is scanned ascending
+    const int lane = threadIdx.x & 31, sub = lane & (kTeam - 1);
+    const unsigned team = 0xffu << (lane & ~(kTeam - 1));
+    const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
+    const int64_t warp = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    for (int64_t base = warp; base < nn; base += warps * 32) {
+        const int64_t id = base + warps * lane;
+        bool work = false;  // internal nodes, and roots that are leaves
+        if (id < nn) work = tnode[id].b <= 0 || (bt.n_clouds ? link[id].parent < 0 : id == 0);
+        unsigned todo = __ballot_sync(0xffffffffu, work);
+        while (todo) {
+            // The warp's four teams run in step (every shuffle is warp-wide, a
+            // team without a node idles): a team of its own mask would execute
+            // alone.
+            const int32_t q = team_pick(todo, (int32_t)id);
+            const int32_t qa = q >= 0 ? tnode[q].a : 0, qb = q >= 0 ? tnode[q].b : 0;
+            const bool internal = qb < 0;
+            const int nc = q < 0 ? 0 : internal ? __popc((unsigned)(-qb)) : 1;
+            const int32_t ch0 = internal ? qa : q;  // first child's id (a leaf root is its own)
+            int32_t ca = 0, cb = 0;
+            if (sub < nc) {
+                ca = tnode[ch0 + sub].a;
+                cb = tnode[ch0 + sub].b;
+            }
+            const unsigned leaf_m = __ballot_sync(FULL, cb > 0), inner_m = __ballot_sync(FULL, sub < nc && cb <= 0);
+            if (leaf_m == 0) continue;
+            const int2 rg = q >= 0 ? nrange[q] : make_int2(0, 0);
+            int32_t c0 = 0, c1 = (int32_t)n;
+            if (bt.n_clouds && q >= 0) {
+                const int c = cloud_of_position(bt, rg.x);
+                c0 = (int32_t)bt.coff[c];
+                c1 = (int32_t)bt.coff[c + 1];
+            }
+            bool asc = false;
+            int32_t up_shift = 0;  // the shift of an ascending unit
+            if (internal && (leaf_m & team)) {
+                for (int32_t u = q; u >= asc_min; u = link[u].parent) {
+                    if (!((unsigned)(-tnode[u].b) & 1u)) {
+                        const int2 ur = nrange[u];
+                        up_shift = c0 + (c1 - (ur.y + 1)) - ur.x;
+                        asc = true;
+                    }
+                }
+            }
+            // (the children's points lie between the node's first and last: on their way to L2 at once)
+            if ((leaf_m & team) && rg.y - rg.x < 1024)
+                for (int32_t p = rg.x + 8 * sub; p <= rg.y; p += 8 * kTeam)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(spts + p));
+            I nlo[D], nhi[D], rlo[D], rhi[D];  // boxes of the node and of the open run
+            auto clear = [](I* lo, I* hi) {
+#pragma unroll
+                for (int d = 0; d < D; ++d) { lo[d] = K::kMaxKey; hi[d] = K::kMinKey; }
+            };
+            clear(nlo, nhi);
+            clear(rlo, rhi);
+            int32_t run_first = 0, run_count = 0, run_id = 0;
+            auto close = [&]() {
+                if (run_count && sub == 0) {
+                    // outside an ascending unit the run's last leaf is visited first
+                    const int32_t p = asc ? run_first + up_shift : c0 + (c1 - (run_first + run_count));
+                    dstart[p] = (uint8_t)run_count;
+                    dnode[p] = run_id;
+                    TNode<float, D> nd;
 #pragma unroll
                     for (int d = 0; d < D; ++d) {
-                        const int64_t c = (int64_t)axis_cell<D, K>(kp, d);
-                        const int64_t plo = (c >> (BITS - lp)) << (BITS - lp);
-                        const int64_t phi = plo + (1LL << (BITS - lp)) - 1;
-                        const int64_t slo = (c >> sh) << sh, shi = slo + (1LL << sh) - 1;
-                        int64_t nlo = plo - kStartMargin, nhi = phi + kStartMargin;
-                        nlo = nlo < 0 ? 0 : nlo;
-                        nhi = nhi > cmax ? cmax : nhi;
-                        ok = ok && nlo >= slo && nhi <= shi;
+                        nd.lo[d] = float_below(K::value(rlo[d]));
+                        nd.hi[d] = float_above(K::value(rhi[d]));
                     }
-                    if (ok) la = L;
+                    nd.a = p;
+                    nd.b = run_count;
+                    rbox[run_id] = nd;
                 }
-                if (la >= 1) {
-                    const int32_t sid = anc[lp - la];
-                    bool casc = false;  // a strict ancestor of S with its first slot empty
-                    for (int j = lp - la + 1; j <= lp; ++j) casc = casc || !(((unsigned)(-tnode[anc[j]].b)) & 1u);
-                    start = sid | (casc ? (1 << 30) : 0);
-                }
-            }
-        }
-        auto emit = [&](int32_t first, int32_t count) {
-            if (pass && out + ng < group_cap) {
-                groups[out + ng] = make_int2(first, count);
-                if (gstart) gstart[out + ng] = start;
-            }
-            ++ng;
-        };
-        if (live) {
-            const TNode<T, D> nd = tnode[id];
-            if (nd.b > 0) {
-                // Only a leaf root (one per cloud in a batch) forms groups of
-                // its own; other leaves are grouped by their parent.
-                if (parent[id] < 0)
-                    for (int32_t c0 = 0; c0 < nd.b; c0 += gmax) emit(nd.a + c0, min(gmax, nd.b - c0));
-            } else {
-                const int nc = __popc((unsigned)(-nd.b));
-                int32_t gfirst = 0, gcount = 0;
-                for (int j = 0; j < nc; ++j) {
-                    const TNode<T, D> c = tnode[nd.a + j];
-                    if (c.b <= 0) {  // internal child: close the open group
-                        if (gcount) emit(gfirst, gcount);
-                        gcount = 0;
-                    } else if (c.b > gmax) {
-                        if (gcount) emit(gfirst, gcount);
-                        gcount = 0;
-                        for (int32_t c0 = 0; c0 < c.b; c0 += gmax) emit(c.a + c0, min(gmax, c.b - c0));
-                    } else {
-                        if (gcount + c.b > gmax) {
-                            emit(gfirst, gcount);
-                            gcount = 0;
-                        }
-                        if (gcount == 0) gfirst = c.a;
-                        gcount += c.b;
-                    }
-                }
-                if (gcount) emit(gfirst, gcount);
-            }
-        }
-        if (pass == 0) {
-            int incl = ng;
-            const int lane = threadIdx.x & 31;
+                run_count = 0;
+                clear(rlo, rhi);
+            };
+            __syncwarp();
+            const int ncw = __reduce_max_sync(FULL, nc);
+            for (int j = 0; j < ncw; ++j) {
+                const int32_t a = __shfl_sync(FULL, ca, j, kTeam);
+                const int32_t b = max(__shfl_sync(FULL, cb, j, kTeam), 0);  // 0: no leaf here
+                const int bw = __reduce_max_sync(FULL, b);
+                const int32_t shift = asc ? up_shift : c0 + (c1 - (a + b)) - a;
+                I lo[D], hi[D];
+                clear(lo, hi);
+                for (int32_t m = sub; m - sub < bw; m += kTeamPts * kTeam) {
+                    SPt<T, D> p[kTeamPts];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
+                    for (int t = 0; t < kTeamPts; ++t)
+                        if (m + t * kTeam < b) p[t] = spts[a + m + t * kTeam];
+#pragma unroll
+                    for (int t = 0; t < kTeamPts; ++t) {
+                        if (m + t * kTeam < b) {
+                            dpts[a + m + t * kTeam + shift] = p[t];
+#pragma unroll
+                            for (int d = 0; d < D; ++d) {
+                                const I k = K::key(K::bits(p[t].x[d]));
+                                lo[d] = min(lo[d], k);
+                                hi[d] = max(hi[d], k);
+                            }
+                        }
+                    }
+                }
+                __syncwarp();
+                team_fold<T, D>(FULL, lo, hi);
+                if (b > 0 && sub == 0) store_bounds<T, D>(tnode + ch0 + j, lo, hi);
+                if (b == 0 || b > gmax || run_count + b > gmax) close();  // (an internal child ends the run too)
+                if (b > gmax) {
+                    for (int32_t c = sub * gmax; c < b; c += kTeam * gmax)
+                        dstart[a + c + shift] = (uint8_t)(kPiece | min(gmax, b - c));
+                } else if (b > 0) {
+                    if (run_count == 0) {
+                        run_first = a;
+                        run_id = ch0 + j;
+                    }
+                    run_count += b;
+#pragma unroll
+                    for (int d = 0; d < D; ++d) { rlo[d] = min(rlo[d], lo[d]); rhi[d] = max(rhi[d], hi[d]); }
+                }
+#pragma unroll
+                for (int d = 0; d < D; ++d) { nlo[d] = min(nlo[d], lo[d]); nhi[d] = max(nhi[d], hi[d]); }
             }
-            const int tot = __shfl_sync(0xffffffffu, incl, 31);
-            unsigned long long base = 0;
-            if (lane == 31 && tot) base = atomicAdd((unsigned long long*)&hdr->n_groups, (unsigned long long)tot);
-            base = __shfl_sync(0xffffffffu, base, 31);
-            out = (int64_t)base + incl - ng;
-            if (tot == 0) return;  // warp-uniform
+            close();
+            // (a node covering its whole set already has that set's bounds)
+            if (internal && (inner_m & team) == 0 && sub == 0 && !(rg.x == c0 && rg.y == c1 - 1))
+                store_bounds<T, D>(tnode + q, nlo, nhi);
+            __syncwarp();
         }
+    }
+}
+
+// --------------------------------------------- 7. node bounds and chunks --
+// One launch, two kinds of blocks that do not depend on each other (both need
+// only section 6).
+//
+// Node bounds: a team of eight lanes climbs from each internal node whose
+// children are all leaves; at a parent, the last internal child to arrive
+// folds the boxes of all its children, one per lane
+// (src/cpu/refit_cpu.jl:50-60).  No thread waits: a team that is not last
+// stops.  Only internal children count as arrivals, so the acquire-release
+// counters (whose acquire drops the SM's L1) are an eighth of the nodes.
+//
+// Chunks: one warp per span of kSpan visiting positions lists the chunks that
+// start in it (contiguous in the chunk array, at a place reserved with one
+// atomic; the spans' order there affects no result), one lane per chunk, with
+// their boxes from section 6 (a piece's from its points), and folds the
+// span's.  The last warp to finish among 32 spans folds their boxes into the
+// next level, and so on up.
+constexpr int kSpansPerBlock = kThreads / 32;
+
+// A level costs three dependent round trips: the release of the team's box
+// with the counter, the sibling boxes, and in their shade the next link.
+template <class T, int D>
+__device__ __forceinline__ void fold_nodes(int64_t warp, int64_t warps, int64_t nn, TNode<T, D>* tnode,
+                                           const NodeLink* __restrict__ link, int32_t* arrive) {
+    using K = OrdKey<T>;
+    using I = typename K::I;
+    const int lane = threadIdx.x & 31, sub = lane & (kTeam - 1);
+    const unsigned team = 0xffu << (lane & ~(kTeam - 1));
+    for (int64_t base = warp; base < nn; base += warps * 32) {
+        const int64_t id = base + warps * lane;
+        // nodes whose children are all leaves: their boxes are done (section 6)
+        const int meta0 = id < nn ? link[id].meta : 0;
+        unsigned todo = __ballot_sync(0xffffffffu, meta0 != 0 && (meta0 & (0xff00 | kLinkFull)) == 0);
+        while (todo) {
+            const int32_t q0 = team_pick(todo, (int32_t)id);
+            int32_t q = q0 >= 0 ? link[q0].parent : -1;
+            NodeLink lk;
+            if (q >= 0) lk = link[q];
+            while (q >= 0 && !(lk.meta & kLinkFull)) {  // (a full node's bounds come from the set's reduce)
+                const int nc = lk.meta & 0xff, inner = lk.meta >> 8 & 0xff;
+                const int32_t up = lk.parent;
+                NodeLink next;
+                if (up >= 0) next = link[up];
+                int old = 0;
+                if (sub == 0)
+                    old = cuda::atomic_ref<int32_t, cuda::thread_scope_device>(arrive[q]).fetch_add(
+                        1, cuda::memory_order_acq_rel);
+                old = __shfl_sync(team, old, 0, kTeam);
+                if (old != inner - 1) break;
+                __syncwarp(team);  // lane 0's acquire covers the team's reads
+                const TNode<T, D>* ch = tnode + lk.first + sub;
+                I lo[D], hi[D];
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    lo[d] = sub < nc ? K::key(K::bits(__ldcg(&ch->lo[d]))) : K::kMaxKey;
+                    hi[d] = sub < nc ? K::key(K::bits(__ldcg(&ch->hi[d]))) : K::kMinKey;
+                }
+                team_fold<T, D>(team, lo, hi);
+                if (sub == 0) store_bounds<T, D>(tnode + q, lo, hi);
+                q = up;
+                lk = next;
+            }
+            __syncwarp();
+        }
+    }
+}
+
+template <class T, int D>
+__global__ void __launch_bounds__(kThreads) k_fold_chunks(int span_blocks, int64_t n, int64_t capacity,
+                                                          TNode<T, D>* tnode, const NodeLink* __restrict__ link,
+                                                          int32_t* arrive, const SPt<T, D>* __restrict__ dpts,
+                                                          const uint8_t* __restrict__ dstart,
+                                                          const int32_t* __restrict__ dnode,
+                                                          const TNode<float, D>* __restrict__ rbox, int64_t chunk_cap,
+                                                          const __grid_constant__ Bvh<D> bv,
+                                                          int32_t* __restrict__ bvh_arrive, OctHeader* hdr) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ uint32_t list_sm[kSpansPerBlock][kSpan];  // (offset in the span << 8) | dstart
+    const int64_t nn = hdr->n_nodes;
+    if (nn > capacity || (hdr->status & DF_TIMEOUT)) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if ((int)blockIdx.x >= span_blocks) {
+        fold_nodes<T, D>((int64_t)(blockIdx.x - span_blocks) * (kThreads / 32) + w,
+                         (int64_t)(gridDim.x - span_blocks) * (kThreads / 32), nn, tnode, link, arrive);
+        return;
+    }
+    int32_t node = blockIdx.x * kSpansPerBlock + w;
+    if (node >= bv.cnt[0]) return;
+    const int64_t s0 = (int64_t)node * kSpan;
+    uint32_t* list = list_sm[w];
+    // this lane's PL positions: which start chunks
+    constexpr int PL = kSpan / 32;
+    alignas(PL) uint8_t c[PL];
+    const int64_t l0 = s0 + PL * lane;
+    if (s0 + kSpan <= n) {
+#pragma unroll
+        for (int j = 0; j < PL; j += 8) *reinterpret_cast<uint2*>(c + j) = *reinterpret_cast<const uint2*>(dstart + l0 + j);
+    } else {
+#pragma unroll
+        for (int j = 0; j < PL; ++j) c[j] = l0 + j < n ? dstart[l0 + j] : 0;
+    }
+    int mine = 0;
+#pragma unroll
+    for (int j = 0; j < PL; ++j) mine += c[j] != 0;
+    const int incl = warp_inclusive_scan(mine);
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    int at = incl - mine;
+#pragma unroll
+    for (int j = 0; j < PL; ++j)
+        if (c[j]) list[at++] = (uint32_t)(((PL * lane + j) << 8) | c[j]);
+    int32_t cbase = 0;
+    if (lane == 0) cbase = (int32_t)atomicAdd((unsigned long long*)&hdr->n_groups, (unsigned long long)total);
+    cbase = __shfl_sync(0xffffffffu, cbase, 0);
+    __syncwarp();
+    float slo[D], shi[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) { slo[d] = INFINITY; shi[d] = -INFINITY; }
+    for (int k = 0; k < total; k += 32) {
+        const uint32_t v = k + lane < total ? list[k + lane] : 0;
+        const int32_t first = (int32_t)(s0 + (v >> 8));
+        const int cnt = (int)(v & (kPiece - 1));
+        TNode<float, D> nd;
+#pragma unroll
+        for (int d = 0; d < D; ++d) { nd.lo[d] = INFINITY; nd.hi[d] = -INFINITY; }
+        nd.a = first;
+        nd.b = cnt;
+        if (v && !(v & kPiece)) nd = rbox[dnode[first]];
+        for (unsigned pm = __ballot_sync(0xffffffffu, (v & kPiece) != 0); pm; pm &= pm - 1) {
+            const int j = __ffs(pm) - 1;
+            const int32_t f = __shfl_sync(0xffffffffu, first, j);
+            const int m = __shfl_sync(0xffffffffu, cnt, j);
+            SPt<T, D> p;
+            if (lane < m) p = dpts[f + lane];
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                const float lo = box_min(lane < m ? float_below(p.x[d]) : INFINITY);
+                const float hi = box_max(lane < m ? float_above(p.x[d]) : -INFINITY);
+                if (lane == j) { nd.lo[d] = lo; nd.hi[d] = hi; }
+            }
+        }
+        if (v && (int64_t)cbase + k + lane < chunk_cap) bv.chunk[cbase + k + lane] = nd;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            slo[d] = min(slo[d], box_min(nd.lo[d]));
+            shi[d] = max(shi[d], box_max(nd.hi[d]));
+        }
+    }
+    auto store_box = [&](TNode<float, D>* out, int32_t a, int32_t b) {
+        TNode<float, D> nd;
+#pragma unroll
+        for (int d = 0; d < D; ++d) { nd.lo[d] = slo[d]; nd.hi[d] = shi[d]; }
+        nd.a = a;
+        nd.b = b;
+        *out = nd;
+    };
+    if (lane == 0) store_box(bv.lev[0] + node, cbase, total);
+    for (int l = 1; l <= bv.top; ++l) {
+        const int32_t up = node >> 5;
+        const int need = min(32, bv.cnt[l - 1] - 32 * up);
+        int old = 0;
+        if (lane == 0)
+            old = cuda::atomic_ref<int32_t, cuda::thread_scope_device>(bvh_arrive[up]).fetch_add(
+                1, cuda::memory_order_acq_rel);
+        old = __shfl_sync(0xffffffffu, old, 0);
+        if (old != need - 1) return;
+        __syncwarp();
+        const TNode<float, D>* ch = bv.lev[l - 1] + 32 * up + lane;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            slo[d] = box_min(lane < need ? __ldcg(&ch->lo[d]) : INFINITY);
+            shi[d] = box_max(lane < need ? __ldcg(&ch->hi[d]) : -INFINITY);
+        }
+        if (lane == 0) store_box(bv.lev[l] + up, 0, 0);
+        bvh_arrive += bv.cnt[l];
+        node = up;
     }
 }
 
@@ -807,24 +1015,6 @@ __global__ void __launch_bounds__(kThreads) k_cloud_bounds(const T* __restrict__
         for (int d = 0; d < D; ++d) { p[d] = (double)smin[0][d]; p[3 + d] = (double)smax[0][d]; }
         p[6] = snan ? 1.0 : 0.0;
     }
-}
-
-// Each cloud's DFS starts below its root's single-child chain (children in
-// slot 0 only), whose nodes all cover the whole cloud.
-template <class T, int D>
-__global__ void k_cloud_start(const TNode<T, D>* __restrict__ tnode, Batch bt, int64_t capacity,
-                              const OctHeader* hdr) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= bt.n_clouds || hdr->n_nodes > capacity) return;
-    int32_t node = bt.croot[c];
-    if (node >= 0) {
-        for (int it = 0; it < 64; ++it) {
-            const TNode<T, D> nd = tnode[node];
-            if (nd.b != -1) break;
-            node = nd.a;
-        }
-    }
-    bt.cstart[c] = node;
 }
 
 __global__ void k_gather_edge_offsets(const int64_t* __restrict__ offsets, const int64_t* __restrict__ coff,
@@ -998,8 +1188,7 @@ __global__ void __launch_bounds__(kThreads) k_moved_rank(const int64_t* __restri
 template <class T, int D, class K>
 __device__ __forceinline__ void put_sorted(int64_t pos, K key, int32_t idx, const T* __restrict__ coords,
                                            K* __restrict__ okeys, int32_t* __restrict__ operm,
-                                           SPt<T, D>* __restrict__ spts, int32_t* __restrict__ iperm) {
-    iperm[idx] = (int32_t)pos;
+                                           SPt<T, D>* __restrict__ spts) {
     okeys[pos] = key;
     operm[pos] = idx;
     SPt<T, D> sp;
@@ -1022,8 +1211,7 @@ __global__ void __launch_bounds__(kThreads) k_resort_merge(int64_t n, const int6
                                                            const K* __restrict__ mk1, const int32_t* __restrict__ mv1,
                                                            const K* __restrict__ mk2, const int32_t* __restrict__ mv2,
                                                            const T* __restrict__ coords, K* __restrict__ okeys,
-                                                           int32_t* __restrict__ operm, SPt<T, D>* __restrict__ spts,
-                                                           int32_t* __restrict__ iperm) {
+                                                           int32_t* __restrict__ operm, SPt<T, D>* __restrict__ spts) {
     pdl_wait();
     pdl_trigger();
     __shared__ int wsum[kThreads / 32];
@@ -1033,14 +1221,14 @@ __global__ void __launch_bounds__(kThreads) k_resort_merge(int64_t n, const int6
     if (m > cap) {
         // Too many changed keys for a merge (the caller sorts afresh): keep
         // the previous order, so that what follows reads a valid permutation.
-        if (p < n) put_sorted<T, D, K>(p, keys[p], perm[p], coords, okeys, operm, spts, iperm);
+        if (p < n) put_sorted<T, D, K>(p, keys[p], perm[p], coords, okeys, operm, spts);
         return;
     }
     // Sorted changed keys: ranked across chunks when there are several.
     const K* __restrict__ mk = m > kChunk ? mk2 : mk1;
     const int32_t* __restrict__ mv = m > kChunk ? mv2 : mv1;
     if (m == n) {  // every key changed: the sorted changed keys are the result
-        if (p < n) put_sorted<T, D, K>(p, mk[p], mv[p], coords, okeys, operm, spts, iperm);
+        if (p < n) put_sorted<T, D, K>(p, mk[p], mv[p], coords, okeys, operm, spts);
         return;
     }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1090,27 +1278,30 @@ __global__ void __launch_bounds__(kThreads) k_resort_merge(int64_t n, const int6
             sn = count_below(mk, mv, m, keys[q], perm[q]);
     }
     const int64_t ui = p - (changed_before[blockIdx.x] + before);  // rank among unchanged keys
-    put_sorted<T, D, K>(ui + s, key, idx, coords, okeys, operm, spts, iperm);
-    for (int64_t j = s; j < sn; ++j) put_sorted<T, D, K>(j + ui + 1, mk[j], mv[j], coords, okeys, operm, spts, iperm);
+    put_sorted<T, D, K>(ui + s, key, idx, coords, okeys, operm, spts);
+    for (int64_t j = s; j < sn; ++j) put_sorted<T, D, K>(j + ui + 1, mk[j], mv[j], coords, okeys, operm, spts);
     if (ui == 0)
-        for (int64_t j = 0; j < s; ++j) put_sorted<T, D, K>(j, mk[j], mv[j], coords, okeys, operm, spts, iperm);
+        for (int64_t j = 0; j < s; ++j) put_sorted<T, D, K>(j, mk[j], mv[j], coords, okeys, operm, spts);
 }
 
-// Bounds-only step (no key changed): the topology is kept; reset the refit
-// arrival counters and preset the full-range nodes from this build's reduce.
+// Bounds-only step (no key changed): the topology is kept; reset the
+// counters of sections 6 and 7 (chunk starts stay where they are) and preset
+// the full-range nodes from this build's reduce.
 template <class T, int D>
 __global__ void __launch_bounds__(kThreads) k_refit_prepare(int64_t nn, int64_t n, TNode<T, D>* __restrict__ tnode,
                                                             const int2* __restrict__ nrange,
-                                                            int32_t* __restrict__ arrive, OctHeader* hdr,
-                                                            int64_t n_groups, int32_t dfs_start) {
+                                                            int32_t* __restrict__ arrive,
+                                                            int32_t* __restrict__ bvh_arrive, int n_arrive,
+                                                            int32_t asc_key, OctHeader* hdr) {
     pdl_wait();
     pdl_trigger();
     const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (id == 0) {
         hdr->n_nodes = nn;
-        hdr->n_groups = n_groups;
-        hdr->dfs_start = dfs_start;
+        hdr->n_groups = 0;
+        hdr->asc_key = asc_key;
     }
+    for (int64_t k = id; k < n_arrive; k += (int64_t)gridDim.x * blockDim.x) bvh_arrive[k] = 0;
     if (id >= nn) return;
     arrive[id] = 0;
     const int2 rg = nrange[id];
@@ -1157,6 +1348,29 @@ void guard_check(Ctx& ctx, const DevBuf& b, size_t bytes, OctHeader* hdr) {
     ctx.kernel_launches += 1;
 }
 
+// Bounds, visiting order, chunks and box hierarchy (sections 6 and 7) of the
+// tree whose topology was just launched; `nodes` bounds its node count.
+template <class T, int D>
+void launch_layout(Ctx& ctx, Tree& t, int64_t n, int64_t node_cap, int64_t chunk_cap, int64_t nodes, int gmax) {
+    OctHeader* hdr = t.hdr.as<OctHeader>();
+    {
+        PhaseTimer pt_(ctx, PH_REFIT);
+        // a grid that fills the device; warps take further nodes in turn
+        const int64_t blocks = std::min<int64_t>(div_up(nodes, kThreads), 148 * 8);
+        launch_pdl(k_layout<T, D>, blocks, kThreads, 0, ctx.stream, node_cap, n, t.tnode.as<TNode<T, D>>(),
+            t.nrange.as<int2>(), t.link.as<NodeLink>(), t.spts.as<SPt<T, D>>(), t.dpts.as<SPt<T, D>>(),
+            t.dstart.as<uint8_t>(), t.dnode.as<int32_t>(), t.rbox.as<TNode<float, D>>(), gmax, hdr, t.batch());
+    }
+    PhaseTimer pt_(ctx, PH_GROUPS);
+    const int span_blocks = div_up(n, kSpan * kSpansPerBlock);
+    const int64_t fold_blocks = std::min<int64_t>(div_up(nodes, kThreads), 148 * 16);
+    launch_pdl(k_fold_chunks<T, D>, span_blocks + fold_blocks, kThreads, 0, ctx.stream, span_blocks, n, node_cap,
+        t.tnode.as<TNode<T, D>>(), t.link.as<NodeLink>(), t.arrive.as<int32_t>(), t.dpts.as<SPt<T, D>>(), t.dstart.as<uint8_t>(), t.dnode.as<int32_t>(), t.rbox.as<TNode<float, D>>(), chunk_cap,
+        t.search_layout<D>(),
+        t.bvh_arrive.as<int32_t>(), hdr);
+    ctx.kernel_launches += 2;
+}
+
 template <class T, int D, class K>
 int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_t moved = -1, int prev = -1) {
     const Batch bt = t.batch();
@@ -1170,6 +1384,15 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
 
     if ((err = ensure(t.spts, (size_t)n * sizeof(SPt<T, D>))) || (err = ensure(t.iperm, (size_t)n * 4)))
         return cuda_status(ctx, err, "allocating points");
+    int32_t lev[kBvhLevels];
+    int64_t bvh_nodes = 0;
+    t.bvh_levels(n, lev, &bvh_nodes);
+    const int n_arrive = (int)(bvh_nodes - lev[0]);
+    if ((err = ensure(t.dpts, (size_t)n * sizeof(SPt<T, D>))) || (err = ensure(t.dstart, (size_t)n)) ||
+        (err = ensure(t.dnode, (size_t)n * 4)) ||
+        (err = ensure(t.bvh, (size_t)bvh_nodes * sizeof(TNode<float, D>))) ||
+        (err = ensure(t.bvh_arrive, (size_t)n_arrive * 4)))
+        return cuda_status(ctx, err, "allocating the search layout");
     OctHeader* hdr = t.hdr.as<OctHeader>();
     const K* skeys;
     const int32_t* perm;
@@ -1244,14 +1467,13 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
             }
             {
                 PhaseTimer pt_(ctx, PH_REFIT);
-                const int nb = div_up(t.n_nodes, kThreads);
-                launch_pdl(k_refit_prepare<T, D>, nb, kThreads, 0, s, t.n_nodes, n, t.tnode.as<TNode<T, D>>(),
-                    t.nrange.as<int2>(), t.arrive.as<int32_t>(), hdr, t.n_groups, t.dfs_start);
-                launch_pdl(k_refit<T, D>, nb, kThreads, 0, s, t.capacity, n, t.tnode.as<TNode<T, D>>(),
-                    t.nrange.as<int2>(), t.parent.as<int32_t>(), t.arrive.as<int32_t>(), t.spts.as<SPt<T, D>>(), hdr,
-                    bt);
-                ctx.kernel_launches += 2;
+                launch_pdl(k_refit_prepare<T, D>, div_up(t.n_nodes, kThreads), kThreads, 0, s, t.n_nodes, n,
+                    t.tnode.as<TNode<T, D>>(), t.nrange.as<int2>(), t.arrive.as<int32_t>(),
+                    t.bvh_arrive.as<int32_t>(), n_arrive, t.asc_key, hdr);
+                ctx.kernel_launches += 1;
             }
+            // the chunk array's capacity is that of the build that made it
+            launch_layout<T, D>(ctx, t, n, t.capacity, t.n_groups, t.n_nodes, t.group_cap);
             if ((err = cudaGetLastError())) return cuda_status(ctx, err, "bounds refit");
             t.last_path = 2;
             t.sorted_buf = sorted;
@@ -1287,9 +1509,9 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
             }
             launch_pdl(k_resort_merge<T, D, K>, nb, kThreads, 0, s, n, &hdr->n_moved, mcap, kp, vp,
                 t.rflag.as<uint8_t>(), t.roff.as<int64_t>(), mk, mv, t.mkeys2.as<K>(), t.mvals2.as<int32_t>(), coords,
-                ok, ov, t.spts.as<SPt<T, D>>(), t.iperm.as<int32_t>());
+                ok, ov, t.spts.as<SPt<T, D>>());
             ctx.kernel_launches += 1;
-            t.iperm_valid = true;
+            t.iperm_valid = false;
         }
         skeys = ok;
         perm = ov;
@@ -1318,59 +1540,40 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
         const int64_t cap = t.capacity;
         const size_t gcap = (size_t)(cap + n / gmax + 2);
         if ((err = ensure_g(ctx, t.tnode, (size_t)cap * sizeof(TNode<T, D>))) ||
-            (err = ensure_g(ctx, t.nrange, (size_t)cap * 8)) || (err = ensure_g(ctx, t.parent, (size_t)cap * 4)) ||
+            (err = ensure_g(ctx, t.nrange, (size_t)cap * 8)) || (err = ensure_g(ctx, t.link, (size_t)cap * sizeof(NodeLink))) ||
             (err = ensure_g(ctx, t.arrive, (size_t)cap * 4)) || (err = ensure_g(ctx, t.fchild, (size_t)cap * 4)) ||
             (err = ensure(t.scan_tmp, (size_t)scan_tmp_elems(nbc) * 8)) ||
-            (err = ensure_g(ctx, t.groups, gcap * 8)) || (err = ensure(t.gstart, gcap * 4)) ||
-            (err = ensure(t.chain, 64 * 4)))
+            (err = ensure_g(ctx, t.rbox, (size_t)cap * sizeof(TNode<float, D>))) ||
+            (err = ensure_g(ctx, t.chunk, gcap * sizeof(TNode<float, D>))))
             return cuda_status(ctx, err, "allocating node arrays");
-        if ((err = cudaMemsetAsync(t.chain.p, 0xff, 64 * 4, s)) ||
-            (err = cudaMemsetAsync(&hdr->n_groups, 0, sizeof(int64_t), s)))
-            return cuda_status(ctx, err, "chain reset");
         if ((err = guard_fill(ctx, t.tnode, (size_t)cap * sizeof(TNode<T, D>))) ||
-            (err = guard_fill(ctx, t.nrange, (size_t)cap * 8)) || (err = guard_fill(ctx, t.parent, (size_t)cap * 4)) ||
+            (err = guard_fill(ctx, t.nrange, (size_t)cap * 8)) || (err = guard_fill(ctx, t.link, (size_t)cap * sizeof(NodeLink))) ||
             (err = guard_fill(ctx, t.arrive, (size_t)cap * 4)) || (err = guard_fill(ctx, t.fchild, (size_t)cap * 4)) ||
-            (err = guard_fill(ctx, t.groups, gcap * 8)))
+            (err = guard_fill(ctx, t.rbox, (size_t)cap * sizeof(TNode<float, D>))) ||
+            (err = guard_fill(ctx, t.chunk, gcap * sizeof(TNode<float, D>))))
             return cuda_status(ctx, err, "node array guards");
-        if (bt.n_clouds && (err = cudaMemsetAsync(bt.croot, 0xff, (size_t)bt.n_clouds * 4, s)))
-            return cuda_status(ctx, err, "cloud root reset");
         {
         PhaseTimer pt_(ctx, PH_TOPOLOGY);
         launch_pdl(k_mark<D, K>, nblocks, kThreads, 0, s, skeys, n, t.lohi.as<uint16_t>(), t.blockcnt.as<int32_t>(),
-            nblocks, bt);
+            nblocks, t.dstart.as<uint8_t>(), t.bvh_arrive.as<int32_t>(), n_arrive, hdr, bt);
         ctx.kernel_launches += exclusive_scan_i32_i64(t.blockcnt.as<int32_t>(), t.blockoff.as<int64_t>(), nbc,
                                                       &hdr->n_nodes, t.scan_tmp.as<int64_t>(), s);
         launch_pdl(k_emit_ids<D>, nblocks, kThreads, 0, s, n, t.lohi.as<uint16_t>(), t.blockoff.as<int64_t>(), nblocks,
             cap, t.fchild.as<int32_t>(), t.nrange.as<int2>(), t.arrive.as<int32_t>(), hdr, bt);
         launch_pdl(k_emit_nodes<T, D, K>, div_up(cap, kThreads), kThreads, 0, s, skeys, n, cap, t.fchild.as<int32_t>(),
-            t.tnode.as<TNode<T, D>>(), t.nrange.as<int2>(), t.parent.as<int32_t>(), t.arrive.as<int32_t>(),
-            t.chain.as<int32_t>(), t.blockoff.as<int64_t>(), nblocks, hdr, bt);
+            t.tnode.as<TNode<T, D>>(), t.nrange.as<int2>(), t.link.as<NodeLink>(), t.arrive.as<int32_t>(),
+            t.blockoff.as<int64_t>(), nblocks, hdr, bt);
         ctx.kernel_launches += 3;
         }
-        {
-        PhaseTimer pt_(ctx, PH_REFIT);
-        launch_pdl(k_refit<T, D>, div_up(cap, kThreads), kThreads, 0, s, cap, n, t.tnode.as<TNode<T, D>>(),
-            t.nrange.as<int2>(), t.parent.as<int32_t>(), t.arrive.as<int32_t>(), t.spts.as<SPt<T, D>>(), hdr, bt);
-        ctx.kernel_launches += 1;
-        }
-        {
-            PhaseTimer pt_(ctx, PH_GROUPS);
-            launch_pdl(k_groups<T, D, K>, div_up(cap, kThreads), kThreads, 0, s, t.tnode.as<TNode<T, D>>(), cap,
-                t.groups.as<int2>(), (int64_t)gcap, t.chain.as<int32_t>(), t.parent.as<int32_t>(), hdr, gmax, skeys,
-                t.nrange.as<int2>(), bt.n_clouds ? nullptr : t.gstart.as<int32_t>());
-            ctx.kernel_launches += 1;
-            if (bt.n_clouds) {
-                k_cloud_start<T, D><<<div_up(bt.n_clouds, 128), 128, 0, s>>>(t.tnode.as<TNode<T, D>>(), bt, cap, hdr);
-                ctx.kernel_launches += 1;
-            }
-        }
+        launch_layout<T, D>(ctx, t, n, cap, (int64_t)gcap, cap, gmax);
         if (ctx.guard_check) {
             guard_check(ctx, t.tnode, (size_t)cap * sizeof(TNode<T, D>), hdr);
             guard_check(ctx, t.nrange, (size_t)cap * 8, hdr);
-            guard_check(ctx, t.parent, (size_t)cap * 4, hdr);
+            guard_check(ctx, t.link, (size_t)cap * sizeof(NodeLink), hdr);
             guard_check(ctx, t.arrive, (size_t)cap * 4, hdr);
             guard_check(ctx, t.fchild, (size_t)cap * 4, hdr);
-            guard_check(ctx, t.groups, gcap * 8, hdr);
+            guard_check(ctx, t.rbox, (size_t)cap * sizeof(TNode<float, D>), hdr);
+            guard_check(ctx, t.chunk, gcap * sizeof(TNode<float, D>), hdr);
             if (moved == -1) {
                 for (int b = 0; b < 2; ++b) guard_check(ctx, t.keys[b], (size_t)n * sizeof(K), hdr);
                 guard_check(ctx, t.vals[0], (size_t)n * 4, hdr);
@@ -1397,7 +1600,7 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
         }
         t.n_nodes = t.hdr_host->n_nodes;
         t.n_groups = t.hdr_host->n_groups;
-        t.dfs_start = t.hdr_host->dfs_start;
+        t.asc_key = t.hdr_host->asc_key;
         t.sorted_buf = sorted;
         t.perm_dev = perm;
         t.skeys_dev = skeys;
@@ -1535,8 +1738,8 @@ int build_batch_typed(Ctx& ctx, Tree& t, const T* coords, int64_t n, const int64
     cudaStream_t s = ctx.stream;
     cudaError_t err;
     if ((err = ensure(t.hdr, sizeof(OctHeader))) || (err = ensure(t.b_coff, (size_t)(nc + 1) * 8)) ||
-        (err = ensure(t.b_cparam, (size_t)nc * kCloudParams * 8)) || (err = ensure(t.b_croot, (size_t)nc * 4)) ||
-        (err = ensure(t.b_cstart, (size_t)nc * 4)) || (err = ensure(t.b_cbounds, (size_t)nc * 8 * 8)) ||
+        (err = ensure(t.b_cparam, (size_t)nc * kCloudParams * 8)) ||
+        (err = ensure(t.b_cbounds, (size_t)nc * 8 * 8)) ||
         (err = ensure(t.b_eoff, (size_t)(nc + 1) * 8)))
         return cuda_status(ctx, err, "allocating batch arrays");
     if (!t.hdr_host) {

@@ -173,10 +173,10 @@ struct DeviceGuard {
 
 void release_tree(oct::Tree& t) {
     using oct::release;
-    for (auto* b : {&t.b_coff, &t.b_cparam, &t.b_croot, &t.b_cstart, &t.b_cbounds, &t.b_eoff})
+    for (auto* b : {&t.b_coff, &t.b_cparam, &t.b_cbounds, &t.b_eoff})
         release(*b);
     for (auto* b : {&t.keys[0], &t.keys[1], &t.vals[0], &t.vals[1], &t.hist, &t.sort_tmp, &t.look, &t.spts, &t.spts_tmp, &t.tnode, &t.nrange,
-                    &t.parent, &t.fchild, &t.arrive, &t.groups, &t.gstart, &t.chain, &t.lohi, &t.blockcnt, &t.blockoff, &t.scan_tmp, &t.partials, &t.hdr,
+                    &t.link, &t.fchild, &t.arrive, &t.dpts, &t.dstart, &t.dnode, &t.rbox, &t.chunk, &t.bvh, &t.bvh_arrive, &t.lohi, &t.blockcnt, &t.blockoff, &t.scan_tmp, &t.partials, &t.hdr,
                     &t.morton, &t.v_first, &t.v_last, &t.v_children, &t.v_bmin, &t.v_bmax, &t.v_perm, &t.iperm,
                     &t.rflag, &t.rcnt, &t.roff, &t.mkeys, &t.mvals, &t.mkeys2, &t.mvals2})
         release(*b);
@@ -227,7 +227,7 @@ OCT_API int oct_ctx_destroy(oct_ctx* ctx) {
     DeviceGuard g(ctx->c.device);
     cudaStreamSynchronize(ctx->c.stream);
     using oct::release;
-    for (auto* b : {&ctx->c.counts, &ctx->c.offsets, &ctx->c.scan_tmp, &ctx->c.total, &ctx->c.dkeys[0],
+    for (auto* b : {&ctx->c.counts, &ctx->c.qpos, &ctx->c.offsets, &ctx->c.scan_tmp, &ctx->c.total, &ctx->c.dkeys[0],
                     &ctx->c.dkeys[1], &ctx->c.dvals[0], &ctx->c.dvals[1], &ctx->c.dhist, &ctx->c.dsort_tmp, &ctx->c.droff,
                     &ctx->c.dsoff, &ctx->c.dstatus, &ctx->c.dredge, &ctx->c.dterm, &ctx->c.dseg, &ctx->c.tstats, &ctx->c.recs, &ctx->c.rcount, &ctx->c.gflag})
         release(*b);

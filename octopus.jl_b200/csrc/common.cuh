@@ -57,6 +57,24 @@ template <class T, int D> struct alignas(16) TNode {
     int32_t b;
 };
 
+// Search layout of a built tree: the points in the order in which the
+// reference's depth-first search visits them, cut into chunks of at most 32
+// (runs of sibling leaves) with their boxes (TNode: a = first position, b =
+// count; in float for every element type, a Float64 box rounded outward: the
+// box tests only have to keep what may be near), under a hierarchy of boxes with fan-out 32 over fixed spans of
+// positions.  lev[0] holds one node per kSpan positions (a = first chunk
+// starting in the span, b = number of such chunks); lev[l] one node per 32 of
+// lev[l - 1].
+constexpr int kSpanShift = 9;
+constexpr int kSpan = 1 << kSpanShift;
+constexpr int kBvhLevels = 4;
+template <int D> struct Bvh {
+    TNode<float, D>* chunk = nullptr;
+    TNode<float, D>* lev[kBvhLevels] = {};
+    int32_t cnt[kBvhLevels] = {};
+    int32_t top = 0;  // highest level built: the first with at most 64 nodes, or the last
+};
+
 // Per-tree device header, copied to pinned host memory at the end of a build.
 struct OctHeader {
     int32_t status;
@@ -67,9 +85,9 @@ struct OctHeader {
     double gmax[3];
     int32_t n_blocks_done;
     int32_t pad;
-    int64_t n_groups;
-    int32_t dfs_start;  // first node of the DFS below the root's single-child chain
+    int64_t n_groups;   // chunks of the search layout
     int32_t guard_bad;  // canary bytes found overwritten (guard-check mode)
+    int32_t asc_key;    // 2^31 - 1 - the first node whose first child slot is empty (0: none)
     int64_t n_moved;    // refit mode: keys that changed since the previous build
 };
 
@@ -90,6 +108,23 @@ __device__ __forceinline__ unsigned long long mul2_rn(unsigned long long a, unsi
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
+__device__ __forceinline__ unsigned long long add2_rn(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long fma2_rn(unsigned long long a, unsigned long long b,
+                                                      unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+// min(|a|, |b|, |c|) in one instruction.
+__device__ __forceinline__ float min3_abs(float a, float b, float c) {
+    float d;
+    asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
     return ((unsigned long long)__float_as_uint(hi) << 32) | __float_as_uint(lo);
 }
@@ -106,8 +141,6 @@ struct Batch {
     int32_t kbits = 0;
     const int64_t* coff = nullptr;   // [n_clouds + 1]
     const double* cparam = nullptr;  // [n_clouds * kCloudParams], values exact in the element type
-    int32_t* croot = nullptr;        // [n_clouds] root node id (-1 for an empty cloud)
-    int32_t* cstart = nullptr;       // [n_clouds] first DFS node of each cloud's tree
 };
 
 // Cloud containing input (== sorted) position i: binary search of coff.
@@ -172,6 +205,24 @@ __device__ __forceinline__ T box_gap2(const T* qlo, const T* qhi, const T* lo, c
     }
     return acc;
 }
+
+// Minimum / maximum of a warp's values, in every lane (which zero a tie
+// keeps is unspecified: for boxes, not for the reference's bounds).
+__device__ __forceinline__ float box_min(float v) {
+    float m;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(m) : "f"(v));
+    return m;
+}
+__device__ __forceinline__ float box_max(float v) {
+    float m;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(m) : "f"(v));
+    return m;
+}
+// Values rounded down / up to float.
+__device__ __forceinline__ float float_below(float v) { return v; }
+__device__ __forceinline__ float float_above(float v) { return v; }
+__device__ __forceinline__ float float_below(double v) { return __double2float_rd(v); }
+__device__ __forceinline__ float float_above(double v) { return __double2float_ru(v); }
 
 // Morton interleave, src/morton.jl:13-23 and :50-58.
 __host__ __device__ __forceinline__ uint64_t split_by_3(uint64_t x) {

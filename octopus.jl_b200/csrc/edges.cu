@@ -1,25 +1,20 @@
-// Fixed-radius traversal and flat-COO edge construction.
+// Fixed-radius search and flat-COO edge construction.
 //
 // Replaces _count_edges_kernel! / _fill_edges_kernel_{3d,2d}! /
 // _build_edges_cuda! (ext/OctopusCUDAExt.jl:262-415) and reproduces the CPU
 // path's output exactly (src/cpu/edges_cpu.jl:36-247):
 //
-//   * One warp serves one query group of the query set's tree: a run of
-//     sibling leaves with at most 32 points (built with the tree), so the
-//     group's box is compact.  The warp walks the target tree once, depth first, with
-//     the box of its 32 queries: children are tested in slot order and
-//     pushed in that order onto a shared-memory stack, so leaves pop in the
-//     same order as the reference's per-query DFS
-//     (src/cpu/iterator_cpu.jl:74-116).  The group box test is conservative
-//     (box_gap2), so every leaf a single query would visit is visited, and
-//     the exact per-pair test d2 = ((dx*dx + dy*dy) + dz*dz) <= r*r decides
-//     membership.  Each query therefore emits its neighbors in the
-//     reference's order: leaves in DFS order, points in ascending sorted
-//     position inside a leaf.  An internal node whose first child slot is
-//     empty counts as a leaf in the reference (src/cpu/iterator_cpu.jl:87),
-//     so its subtree is walked in ascending slot order, which lists its
-//     points in ascending position exactly as the reference's leaf loop.
-//   * Leaf points are staged in shared memory and broadcast to the 32 lanes.
+//   * The build lays the points out in the order in which the reference's
+//     depth-first search visits them (build.cu sections 6 and 7), so each
+//     query's neighbors, in the reference's order, are the in-radius points
+//     in ascending position of that layout, whatever structure finds them.
+//   * One warp serves one chunk of the query set's layout (at most 32 points,
+//     a run of sibling leaves).  It walks the box hierarchy over the target's
+//     layout, one lane per child box (fan-out 32), in ascending position,
+//     down to the target chunks.  The box tests are conservative
+//     (boxes_near), and the exact per-pair test
+//     d2 = ((dx*dx + dy*dy) + dz*dz) <= r*r decides membership.
+//   * Target points are staged in shared memory and broadcast to the 32 lanes.
 //   * counts -> int64 exclusive scan -> fill at the per-query cursor.
 
 #include <algorithm>
@@ -31,11 +26,11 @@
 namespace oct {
 
 constexpr int kEdgeWarps = 4;
+// Blocks of k_edges per SM: the most that leave it without spills (Float32 count
+// of 1M lattice points with 7 / 8 / 10: 269 / 260 / 290 us).
+template <class T> constexpr int kEdgeBlocks = sizeof(T) == 4 ? 8 : 5;
 constexpr int kEdgeThreads = kEdgeWarps * 32;
-constexpr int kStage = 32;  // staged hits per lane, and points per leaf sub-chunk
-constexpr int kMultiPop = 4;     // most internal nodes expanded together (the tuned multi_pop is <= this)
-constexpr int kMultiLimit = 64;  // stack depth up to which they are
-constexpr int kMaxSeg = 16;      // most leaves sharing one chunk (the tuned max_seg is <= this)
+constexpr int kStage = 32;  // staged hits per lane, and points per chunk
 
 // The three passes of k_edges.
 enum EdgePass {
@@ -49,23 +44,22 @@ enum EdgePass {
 enum TraversalStat {
     TS_GROUPS = 0,     // query groups (warps)
     TS_QUERIES,        // query points
-    TS_EXPANSIONS,     // internal-node expansion rounds
-    TS_CHILDREN,       // child boxes tested
-    TS_CHUNKS,         // leaf chunks staged
+    TS_EXPANSIONS,     // rounds of box tests (up to 32 boxes each)
+    TS_CHILDREN,       // boxes tested
+    TS_CHUNKS,         // target chunks staged
     TS_TARGETS,        // target points staged
     TS_STEPS,          // pair-loop steps executed (four targets each)
     TS_PAIR_TESTS,     // query-target distance tests issued (steps x 4 x queries of the group)
     TS_HITS,           // pairs within the radius (self pair excluded when asked)
     TS_CYCLES_TOTAL,   // SM cycles of the warps, summed
-    TS_CYCLES_LEAF,    // ... of which in leaf chunks (staging and pair tests)
+    TS_CYCLES_LEAF,    // ... of which in target chunks (staging and pair tests)
     TS_CYCLES_PAIRS,   // ... of which in the pair loop
     TS_NUM
 };
 
-// A hit record: the sorted position of a leaf's first point (of a leaf's
-// 32-point part, for a larger leaf) and the bit mask of its points within the
-// radius of one query.  A query's records, in order, list its neighbors in
-// the reference's order.
+// A hit record: the visiting position of a target chunk's first point and the
+// bit mask of the chunk's points within the radius of one query.  A query's
+// records, in order, list its neighbors in the reference's order.
 constexpr int kMaxRecords = 65000;  // per query: the record count is stored in 16 bits
 constexpr uint16_t kOverflowMark = 0xffff;  // record count of the queries of an overflowed group
 
@@ -86,131 +80,291 @@ __device__ __forceinline__ void write_edge(int64_t k, const SPt<T, D>& t, const 
     rdist[k] = mul_rn(sqrt_rn(d2), inv_r);
 }
 
-// Starts moving the line holding p into L1 (no value is returned; p must lie
-// inside an allocation).
-__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
-
-// The per-group traversal starts of a tree searched against itself (not a
-// batch), else null (every group starts at the root).
-__host__ __forceinline__ const int32_t* own_start(const Tree& q, const Tree& t) {
-    return (&q == &t && !t.n_clouds) ? t.gstart.as<int32_t>() : nullptr;
-}
-
-// Radius and index base of the point set (cloud) holding sorted position p.
+// Radius and index base of the point set (cloud) holding position p (sorted
+// and visiting positions of a cloud share one range).
 template <class T>
-__device__ __forceinline__ void cloud_params(const Batch& bt, int64_t p, T& r2, T& inv_r, int32_t& start_node,
-                                             int32_t& base) {
+__device__ __forceinline__ void cloud_params(const Batch& bt, int64_t p, T& r2, T& inv_r, int32_t& base) {
     if (bt.n_clouds) {
         const int c = cloud_of_position(bt, p);
         const double* cp = bt.cparam + (size_t)c * kCloudParams;
         r2 = (T)cp[4];
         inv_r = (T)cp[5];
-        start_node = bt.cstart[c];
         base = (int32_t)bt.coff[c];
     }
 }
 
+// sqrt to within 2^-22 of its value (the slack of the bounds it goes into is 2^-20)
+__device__ __forceinline__ float sqrt_near(float a) {
+    float s;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(s) : "f"(a));
+    return s;
+}
+__device__ __forceinline__ double sqrt_near(double a) { return sqrt_rn(a); }
+
+// The pair test of one staged chunk of targets against the warp's queries.
+//
+// EXACT: d2 in the reference's operation order, packed differences and
+// squares for two float targets at a time and scalar sums (packed
+// add.rn.f32x2 sums after the packed squares changed results, as a fused
+// multiply-add would).  About ten issue slots per target.
+//
+// FAST decides the same test from another expression.  With c the middle of
+// the query chunk's box, t' = t - c and q' = q - c rounded to the element
+// type, and |t'|^2 stored beside the target,
+//     d = (|t'|^2 + (|q'|^2 - r2)) - 2 q' . t'
+// by fused multiply-adds: half an addition, 3/2 multiply-adds, one funnel
+// shift collecting the sign and half a three-way minimum per target.  Every
+// coordinate and intermediate is bounded through the boxes: a target that
+// passed the box test has |t - c| <= half extent + r per axis.  With
+// S = 2 (sum h^2 + sum (h + r)^2) + r2, which bounds every intermediate,
+// u the unit roundoff: the coordinates' rounding contributes 2 u S, the two
+// squared norms 3 u S, the sums and multiply-adds 4 u S, and the reference's
+// own rounding of d2 near r2 5 u S, so the sign of d decides as the reference
+// does whenever |d| > 14 u S.  eps = 32 u S leaves more than a factor of two;
+// a chunk with a smaller |d| in any lane (about 0.4% of them at 28 neighbors
+// per point) is tested again by EXACT.  Groups whose box is large against r
+// (eps above 2^-11 r2: the uncertain shell would be met too often) and
+// radii near the ends of the type's range use EXACT alone.
+template <class T> struct PairConst;
+template <> struct PairConst<float> {
+    static constexpr float eps = 1.0f / (1 << 19);  // 32 u
+    static constexpr float shell = 1.0f / (1 << 11);
+    static constexpr float slack = 1.0f / (1 << 20);
+    static constexpr float tiny = 1e-30f, huge = 1e36f, far = 1e38f;
+};
+template <> struct PairConst<double> {
+    static constexpr double eps = 1.0 / (1ULL << 48);  // 32 u
+    static constexpr double shell = 1.0 / (1 << 11);
+    static constexpr double slack = 1.0 / (1 << 20);
+    static constexpr double tiny = 1e-290, huge = 1e290, far = 1e300;
+};
+
+// Whether the boxes (or points: lo == hi) are near enough for pairs within r:
+// the per-axis gaps, squared and summed in float by fused multiply-adds,
+// against lim = r2 (1 + 2^-20) + tiny.  A pair of points inside with d2 <= r2
+// has per-axis gaps of at most its own differences, and the roundings of the
+// two sums (4 u each) are far inside the bound's slack, so no such pair is
+// lost.
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+template <int D>
+__device__ __forceinline__ bool boxes_near(const float* qlo, const float* qhi, const float* lo, const float* hi,
+                                           float lim) {
+    float acc = 0.f;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+        const float g = max3(__fsub_rn(lo[d], qhi[d]), __fsub_rn(qlo[d], hi[d]), 0.f);
+        acc = d == 0 ? __fmul_rn(g, g) : __fmaf_rn(g, g, acc);
+    }
+    return acc <= lim;
+}
+
+// Bits of the targets (those of `keep`) within the radius of query q; sx[d] =
+// the targets' coordinates.
+template <int D>
+__device__ __forceinline__ unsigned pairs_exact(const float (*sx)[32], unsigned keep, const float* q, float r2) {
+    unsigned hm = 0;
+    unsigned long long P[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) P[d] = pack2(q[d], q[d]);
+    // one bit per step of four targets with a target kept
+    for (unsigned km = (keep | keep >> 1 | keep >> 2 | keep >> 3) & 0x11111111u; km; km &= km - 1) {
+        const int j = __ffs(km) - 1;
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            const ulonglong2 px = *reinterpret_cast<const ulonglong2*>(&sx[d][j]);
+            const unsigned long long da = sub2_rn(px.x, P[d]);
+            const unsigned long long db = sub2_rn(px.y, P[d]);
+            const unsigned long long qa = mul2_rn(da, da);
+            const unsigned long long qb = mul2_rn(db, db);
+            s0 = (d == 0) ? lo2(qa) : __fadd_rn(s0, lo2(qa));
+            s1 = (d == 0) ? hi2(qa) : __fadd_rn(s1, hi2(qa));
+            s2 = (d == 0) ? lo2(qb) : __fadd_rn(s2, lo2(qb));
+            s3 = (d == 0) ? hi2(qb) : __fadd_rn(s3, hi2(qb));
+        }
+        hm |= ((s0 <= r2 ? 1u : 0u) | (s1 <= r2 ? 2u : 0u) | (s2 <= r2 ? 4u : 0u) | (s3 <= r2 ? 8u : 0u)) << j;
+    }
+    return hm & keep;
+}
+template <int D>
+__device__ __forceinline__ unsigned pairs_exact(const double (*sx)[32], unsigned keep, const double* q, double r2) {
+    unsigned hm = 0;
+    for (unsigned km = keep; km; km &= km - 1) {
+        const int j = __ffs(km) - 1;
+        double t[D], diff[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) t[d] = sx[d][j];
+        hm |= (dist2<double, D>(t, q, diff) <= r2 ? 1u : 0u) << j;
+    }
+    return hm;
+}
+
+// The same by FAST: sx[d] = t', sx[D] = |t'|^2 (PairConst::far for a target
+// outside `keep`); m2q = -2 q', off = |q'|^2 - r2.  *close: some |d| <= eps.
+template <int D>
+__device__ __forceinline__ unsigned pairs_fast(const float (*sx)[32], unsigned keep, const float* m2q, float off,
+                                               float eps, bool* close) {
+    unsigned hm = 0;
+    float u = PairConst<float>::far;
+    unsigned long long M[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) M[d] = pack2(m2q[d], m2q[d]);
+    const unsigned long long O = pack2(off, off);
+    const unsigned steps = keep | keep >> 1 | keep >> 2 | keep >> 3;
+#pragma unroll
+    for (int j = 28; j >= 0; j -= 4) {
+        if (steps >> j & 1u) {
+            const ulonglong2 tt = *reinterpret_cast<const ulonglong2*>(&sx[D][j]);
+            unsigned long long a = add2_rn(tt.x, O), b = add2_rn(tt.y, O);
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                const ulonglong2 px = *reinterpret_cast<const ulonglong2*>(&sx[d][j]);
+                a = fma2_rn(px.x, M[d], a);
+                b = fma2_rn(px.y, M[d], b);
+            }
+            u = min3_abs(lo2(a), hi2(a), u);
+            u = min3_abs(lo2(b), hi2(b), u);
+            hm = __funnelshift_l((unsigned)(b >> 32), hm, 1);
+            hm = __funnelshift_l((unsigned)b, hm, 1);
+            hm = __funnelshift_l((unsigned)(a >> 32), hm, 1);
+            hm = __funnelshift_l((unsigned)a, hm, 1);
+        } else {
+            hm <<= 4;
+        }
+    }
+    *close = u <= eps;
+    return hm;
+}
+template <int D>
+__device__ __forceinline__ unsigned pairs_fast(const double (*sx)[32], unsigned keep, const double* m2q, double off,
+                                               double eps, bool* close) {
+    unsigned hm = 0, u = 0x7fffffffu;  // u: smallest high word of |d|
+    for (unsigned km = (keep | keep >> 1) & 0x55555555u; km; km &= km - 1) {
+        const int j = __ffs(km) - 1;
+        const double2 tt = *reinterpret_cast<const double2*>(&sx[D][j]);
+        double a = __dadd_rn(tt.x, off), b = __dadd_rn(tt.y, off);
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            const double2 px = *reinterpret_cast<const double2*>(&sx[d][j]);
+            a = __fma_rn(px.x, m2q[d], a);
+            b = __fma_rn(px.y, m2q[d], b);
+        }
+        const unsigned ha = (unsigned)__double2hiint(a), hb = (unsigned)__double2hiint(b);
+        u = min(u, min(ha & 0x7fffffffu, hb & 0x7fffffffu));
+        hm |= ((ha >> 31) | (hb >> 31) << 1) << j;
+    }
+    *close = u <= (unsigned)__double2hiint(eps);
+    return hm;
+}
+
+// Bound by instruction issue and the latency of a warp's dependent steps (63%
+// of issue slots at 38% of the warp slots on a 343,000-point lattice, where
+// k_edges over the tree with an exact test per pair executed 100 M warp
+// instructions, this one 64 M).  Count, before and after: 1M lattice points
+// 313 -> 258 us, 2M uniform points at 14 neighbors 792 -> 663, 1M clustered 2D
+// points at 151 neighbors 373 -> 298, 200,003 Float64 points 152 -> 138, 250,007
+// queries against 1M points 329 -> 255.  Not faster: loading the next chunk's
+// points while this one is tested (72 registers), spans of 256 or 1024
+// positions, two or eight warps per block, two chunks of queries per warp.
+//
 // ocount: in the record pass, ocount[0] counts the groups whose records
 // overflowed (those groups are walked again by the fill pass) and ocount[1]
 // is the largest record count of a query; in the fill pass, ocount[0] is
 // the bounds-guard word.  recs[qpos * rec_cap + r] = record r of the query at
-// sorted position qpos, rcount[qpos] = its record count, gflag[g] = 1 when a
-// query of group g had more than rec_cap records.
+// visiting position qpos, rcount[qpos] = its record count, gflag[g] = 1 when a
+// query of group g had more than rec_cap records.  qpos_of[i] = the visiting
+// position of query point i (when given), which the fill reads.
 template <class T, int D, int PASS>
-__global__ void __launch_bounds__(kEdgeThreads) k_edges(
-    const SPt<T, D>* __restrict__ qpts, const int2* __restrict__ qgroups, int64_t n_groups,
-    const TNode<T, D>* __restrict__ tnode, int32_t start_node,
-    const SPt<T, D>* __restrict__ tpts, int64_t n_tnodes, T r2, T inv_r, int exclude_self,
-    int32_t* __restrict__ counts, const int64_t* __restrict__ offsets, int32_t* __restrict__ senders,
-    int32_t* __restrict__ receivers, T* __restrict__ rdisp, T* __restrict__ rdist, int* __restrict__ ocount,
-    int2* __restrict__ recs, int64_t rec_cap, uint16_t* __restrict__ rcount, uint8_t* __restrict__ gflag, Batch bt,
-    unsigned long long* __restrict__ stats, int max_seg, int multi_pop, int nbox, int prefetch,
-    const int32_t* __restrict__ gstart) {
+__global__ void __launch_bounds__(kEdgeThreads, kEdgeBlocks<T>) k_edges(
+    const SPt<T, D>* __restrict__ qpts, const TNode<float, D>* __restrict__ qchunks, int64_t n_groups,
+    const __grid_constant__ Bvh<D> bv, const SPt<T, D>* __restrict__ tpts, int64_t n_targets, T r2, T inv_r, int exclude_self,
+    int32_t* __restrict__ counts, int32_t* __restrict__ qpos_of, const int64_t* __restrict__ offsets,
+    int32_t* __restrict__ senders, int32_t* __restrict__ receivers, T* __restrict__ rdisp, T* __restrict__ rdist,
+    int* __restrict__ ocount, int2* __restrict__ recs, int64_t rec_cap, uint16_t* __restrict__ rcount,
+    uint8_t* __restrict__ gflag, Batch bt, unsigned long long* __restrict__ stats) {
     pdl_wait();
     pdl_trigger();
     constexpr bool STAGE = PASS == EP_FILL;
     constexpr bool STATS = PASS == EP_STATS;
+    constexpr unsigned FULL = 0xffffffffu;
     long long st_t0 = 0, st_leaf = 0, st_pairs = 0;
     unsigned long long st_exp = 0, st_children = 0, st_chunks = 0, st_targets = 0, st_steps = 0;
     if constexpr (STATS) st_t0 = clock64();
-    // The usual DFS bound, plus the room the multi-node expansions may take.
-    constexpr int SD = stack_depth<D>() + kMultiLimit + 8;
-    // Stack entries are the pushed node's (a, b) record; bit 31 of a marks
-    // ascending-order subtrees (see below).
-    __shared__ int2 stack[kEdgeWarps][SD];
-    // The internal nodes expanded together: their stack entries and the
-    // first lane of each one's children.
-    __shared__ int2 snode[kEdgeWarps][kMultiPop];
-    __shared__ int soff[kEdgeWarps][kMultiPop + 1];
-    // The current leaf chunk, structure of arrays so pairs load as 8 bytes,
-    // its leaf segments (first position, first slot; entry nseg holds the
-    // point count), and per query lane the chunk slot of its own point
-    // ((chunk number << 5) | slot).
-    __shared__ __align__(16) T sx[kEdgeWarps][D][32];
-    __shared__ int2 sseg[kEdgeWarps][kMaxSeg + 1];
-    __shared__ int sself[kEdgeWarps][32];
-    // The boxes of the group's nbox runs of 32 / nbox consecutive queries
-    // (lo then hi per box): a target is tested only if it is within r of one.
-    __shared__ T sbox[kEdgeWarps][4][2 * D];
-    // Fill pass: each lane stages the sorted positions of its next hits; a
-    // flush writes them as runs of consecutive edges of one query.
+    // The current target chunk, structure of arrays so that four targets load
+    // as 16 bytes per axis (row D: |t'|^2).
+    __shared__ __align__(16) T sx[kEdgeWarps][D + 1][32];
+    // Upper levels of the walk: the child boxes still to visit, their first index.
+    __shared__ uint2 swalk[kEdgeWarps][kBvhLevels];
+    // Fill pass: each lane stages the positions of its next hits; a flush
+    // writes them as runs of consecutive edges of one query.
     __shared__ int32_t obuf[STAGE ? kEdgeWarps : 1][32][STAGE ? kStage + 1 : 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t g = (int64_t)blockIdx.x * kEdgeWarps + w;
     if (g >= n_groups) return;  // warp-uniform
     if (PASS == EP_FILL && recs != nullptr && gflag[g] == 0) return;  // expanded from its records
-    const int2 grp = qgroups[g];
-    const bool valid = lane < grp.y;
-    const int64_t qpos = grp.x + (valid ? lane : 0);  // sorted position of this lane's query
+    TNode<float, D> gc = qchunks[g];
+    const bool valid = lane < gc.b;
+    const int64_t qpos = gc.a + (valid ? lane : 0);  // position of this lane's query
     const SPt<T, D> q = qpts[qpos];
-    // A batch searches each cloud in its own tree with its own radius and
+    // A batch searches each cloud in its own positions with its own radius and
     // reports cloud-local indices.
     int32_t base = 0;
-    cloud_params<T>(bt, grp.x, r2, inv_r, start_node, base);
-    // The group's box.  Plain min/max suffice here (the coordinates are finite,
-    // and which zero a tie keeps does not move the box), unlike the build's
-    // bounds, which follow Julia's min/max.
-    T qlo[D], qhi[D];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-        T lo = q.x[d], hi = q.x[d];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-            hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-        }
-        qlo[d] = lo;
-        qhi[d] = hi;
+    int32_t plo = 0, phi = (int32_t)n_targets;
+    if (bt.n_clouds) {
+        const int c = cloud_of_position(bt, gc.a);
+        const double* cp = bt.cparam + (size_t)c * kCloudParams;
+        r2 = (T)cp[4];
+        inv_r = (T)cp[5];
+        base = plo = (int32_t)bt.coff[c];
+        phi = (int32_t)bt.coff[c + 1];
     }
-    if (nbox > 1) {
-        // sub-boxes over runs of 16 (nbox 2) or 8 (nbox 4) lanes; a lane
-        // past the group's end holds the group's first point, inside the box
-        const int width = 32 / nbox;
+    // The fast pair test's constants (see pairs_fast).
+    using PC = PairConst<T>;
+    const float lim = float_above(r2 * (T(1) + PC::slack)) + 1e-44f;
+    T ctr[D], m2q[D], off, eps;
+    bool fast;
+    {
+        const T r = sqrt_near(r2) * (T(1) + PC::slack);
+        T qq = T(0), tt = T(0), qn = T(0);
 #pragma unroll
         for (int d = 0; d < D; ++d) {
-            T lo = q.x[d], hi = q.x[d];
-            for (int o = width >> 1; o > 0; o >>= 1) {
-                lo = jl_min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-                hi = jl_max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-            }
-            if ((lane & (width - 1)) == 0) {
-                sbox[w][lane / width][d] = lo;
-                sbox[w][lane / width][D + d] = hi;
-            }
+            const T half = T(0.5) * ((T)gc.hi[d] - (T)gc.lo[d]);
+            ctr[d] = (T)gc.lo[d] + half;
+            const T h = half * (T(1) + PC::slack) + fabs(ctr[d]) * PC::slack;
+            qq += h * h;
+            tt += (h + r) * (h + r);
+            const T x = q.x[d] - ctr[d];
+            m2q[d] = T(-2) * x;
+            qn += x * x;
         }
-        __syncwarp();
+        const T S = T(2) * (qq + tt) + r2;
+        eps = PC::eps * S;
+        off = valid ? qn - r2 : PC::far;  // a lane without a query hits nothing
+        fast = eps <= PC::shell * r2 && r2 >= PC::tiny && S <= PC::huge;  // false for a NaN
     }
-    int64_t cnt = 0;
+    if constexpr (!std::is_same<T, float>::value) {
+        // room for the rounding of a Float64 target's coordinates to float
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            const float pad = (fmaxf(fabsf(gc.lo[d]), fabsf(gc.hi[d])) + sqrt_near(lim)) * 0x1p-22f;
+            gc.lo[d] -= pad;
+            gc.hi[d] += pad;
+        }
+    }
+    int32_t cnt = 0;
     int64_t cur = 0, cur_end = 0;
     if (PASS == EP_FILL && valid) {
         cur = offsets[q.idx];
         cur_end = offsets[q.idx + 1];
     }
-    const bool self_pair = exclude_self != 0;
     int ocnt = 0;
     int nrec = 0;
-    int chunk = 0;  // leaf chunks processed by this warp (warp-uniform)
-    sself[w][lane] = -1;
     const int cap = (int)rec_cap;
     int2* myrec = PASS == EP_RECORD ? recs + qpos * rec_cap : nullptr;  // this query's records
 
@@ -219,17 +373,17 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edges(
     // passing `need` are flushed, so each query leaves in long runs.
     auto flush = [&](bool need) {
         __syncwarp();
-        unsigned busy = __ballot_sync(0xffffffffu, need && ocnt > 0);
+        unsigned busy = __ballot_sync(FULL, need && ocnt > 0);
         while (busy) {
             const int ql = __ffs(busy) - 1;
             busy &= busy - 1;
-            const int nql = __shfl_sync(0xffffffffu, ocnt, ql);
-            const long long cq = __shfl_sync(0xffffffffu, (long long)cur, ql);
-            const long long ce = __shfl_sync(0xffffffffu, (long long)cur_end, ql);
-            const int32_t qi = __shfl_sync(0xffffffffu, q.idx, ql);
+            const int nql = __shfl_sync(FULL, ocnt, ql);
+            const long long cq = __shfl_sync(FULL, (long long)cur, ql);
+            const long long ce = __shfl_sync(FULL, (long long)cur_end, ql);
+            const int32_t qi = __shfl_sync(FULL, q.idx, ql);
             T px[D];
 #pragma unroll
-            for (int d = 0; d < D; ++d) px[d] = __shfl_sync(0xffffffffu, q.x[d], ql);
+            for (int d = 0; d < D; ++d) px[d] = __shfl_sync(FULL, q.x[d], ql);
             if (lane < nql) {
                 const int64_t k = cq + lane;
                 if (k < ce)
@@ -246,253 +400,161 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edges(
         __syncwarp();
     };
 
-    int sp = 0;
-    const int32_t gs = gstart ? gstart[g] : -1;
-    if (gs >= 0) {
-        // the group's own start node (k_groups): its subtree holds every
-        // neighbor, and the group lies inside it
-        const TNode<T, D> sn = tnode[gs & 0x3fffffff];
-        if (lane == 0) stack[w][0] = make_int2(sn.a | ((gs >> 30) & 1 ? (int32_t)0x80000000 : 0), sn.b);
-        sp = 1;
-    } else if (n_tnodes > 0) {
-        const TNode<T, D> root = tnode[start_node];
-        if (box_gap2<T, D>(qlo, qhi, root.lo, root.hi) <= r2) {
-            if (lane == 0) stack[w][0] = make_int2(root.a, root.b);
-            sp = 1;
+    // One target chunk: positions [first, first + num); t = this lane's point
+    // of it (lane < num).
+    auto visit = [&](int32_t first, int num, const SPt<T, D>& t) {
+        long long st_c0 = 0;
+        if constexpr (STATS) st_c0 = clock64();
+        // A target farther than r from the group's box can be no query's
+        // neighbor: the pair loop skips the steps whose targets all are.
+        float xf[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) xf[d] = (float)t.x[d];
+        const bool near = lane < num && boxes_near<D>(gc.lo, gc.hi, xf, xf, lim);
+        const unsigned keep = __ballot_sync(FULL, near);
+        if (keep == 0) return;
+        long long st_p0 = 0;
+        if constexpr (STATS) {
+            st_p0 = clock64();
+            ++st_chunks;
+            st_targets += num;
+            st_steps += __popc((keep | keep >> 1 | keep >> 2 | keep >> 3) & 0x11111111u);
         }
-    }
-    __syncwarp();
-    while (sp > 0) {
-        const int2 ent = stack[w][--sp];
-        const int32_t na = ent.x & 0x7fffffff;
-        const int32_t nb = ent.y;
-        if (nb > 0) {
-            // Leaves: every (query, point) pair, points in ascending position
-            // within a leaf, hits as a bit mask.  Leaves popped one after
-            // another (the next stack entries, so the DFS order is kept)
-            // share one chunk of at most kStage points as consecutive
-            // segments; a leaf of more than kStage points is cut into chunks.
-            for (int32_t c0 = 0; c0 < nb; c0 += kStage) {
-                long long st_c0 = 0;
-                if constexpr (STATS) st_c0 = clock64();
-                __syncwarp();  // every lane is done with the previous chunk's segment table
-                int total = min(kStage, nb - c0);
-                int nseg = 1;
-                if (lane == 0) sseg[w][0] = make_int2(na + c0, 0);
-                if (nb <= kStage) {
-                    while (sp > 0 && nseg < max_seg) {
-                        const int2 nx = stack[w][sp - 1];
-                        if (nx.y <= 0 || total + nx.y > kStage) break;
-                        --sp;
-                        if (lane == 0) sseg[w][nseg] = make_int2(nx.x & 0x7fffffff, total);
-                        total += nx.y;
-                        ++nseg;
-                    }
-                }
-                if (lane == 0) sseg[w][nseg] = make_int2(0, total);
-                const int mp = (total + 3) & ~3;  // padded to whole pairs of pairs with +inf points
-                ++chunk;
+        unsigned hm = 0;
+        bool exact = !fast;
+        if (fast) {
+            T x[D], tt = T(0);
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                x[d] = near ? t.x[d] - ctr[d] : T(0);
+                tt = d == 0 ? x[d] * x[d] : fma_rn(x[d], x[d], tt);
+            }
+            if (!near) tt = PC::far;
+            __syncwarp();  // every lane is done with the previous chunk
+#pragma unroll
+            for (int d = 0; d < D; ++d) sx[w][d][lane] = x[d];
+            sx[w][D][lane] = tt;
+            __syncwarp();
+            bool close;
+            hm = pairs_fast<D>(sx[w], keep, m2q, off, eps, &close);
+            exact = __any_sync(FULL, close);
+        }
+        if (exact) {
+            __syncwarp();
+#pragma unroll
+            for (int d = 0; d < D; ++d) sx[w][d][lane] = near ? t.x[d] : T(INFINITY);
+            __syncwarp();
+            hm = valid ? pairs_exact<D>(sx[w], keep, q.x, r2) : 0u;
+        }
+        if constexpr (STATS) st_pairs += clock64() - st_p0;
+        if (exclude_self && first == gc.a) hm &= ~(1u << lane);  // the group's own chunk (same tree)
+        const int nh = __popc(hm);
+        cnt += nh;
+        if (PASS == EP_RECORD) {
+            if (hm != 0) {
+                if (nrec < cap) myrec[nrec] = make_int2(first, (int32_t)hm);
+                ++nrec;
+            }
+        } else if (STAGE) {
+            if (__any_sync(FULL, ocnt + nh > kStage)) flush(ocnt + nh > kStage);
+            while (hm) {
+                const int j = __ffs(hm) - 1;
+                hm &= hm - 1;
+                obuf[w][lane][ocnt++] = first + j;
+            }
+        }
+        if constexpr (STATS) st_leaf += clock64() - st_c0;
+    };
+
+    // The walk: level `l` nodes from `b0` on, `m` those of the current round
+    // still to descend into; the levels above wait in swalk.  It starts at the
+    // lowest level with at most 64 nodes over the positions searched.
+    int top = 0;
+    while (top < bv.top && ((phi - 1) >> (kSpanShift + 5 * top)) - (plo >> (kSpanShift + 5 * top)) >= 64) ++top;
+    const int32_t i1 = ((phi - 1) >> (kSpanShift + 5 * top)) + 1;
+    int32_t na = 0, nb = 0;  // the last level-0 round's nodes, one per lane: first chunk, chunks
+    auto test = [&](int l, int32_t b0, int32_t end) {
+        const int32_t i = b0 + lane;
+        bool pass = false;
+        if (i < end) {
+            const TNode<float, D> nd = bv.lev[l][i];
+            pass = boxes_near<D>(gc.lo, gc.hi, nd.lo, nd.hi, lim);
+            if (l == 0) {
+                na = nd.a;
+                nb = nd.b;
+            }
+        }
+        if constexpr (STATS) {
+            ++st_exp;
+            st_children += min(32, end - b0);
+        }
+        return __ballot_sync(FULL, pass);
+    };
+    int l = top;
+    int32_t b0 = plo >> (kSpanShift + 5 * top);
+    unsigned m = test(l, b0, i1);
+    while (true) {
+        if (m == 0) {
+            if (l == top) {
+                b0 += 32;
+                if (b0 >= i1) break;
+                m = test(l, b0, i1);
+            } else {
+                ++l;
                 __syncwarp();
-                // A target farther than r from the group's box can be no
-                // query's neighbor (box_gap2 never exceeds a point distance):
-                // the pair loop skips the steps whose targets all are.
-                bool near = false;
-                if (lane < total) {
-                    int k = 0;
-                    while (sseg[w][k + 1].y <= lane) ++k;
-                    const int32_t pos = sseg[w][k].x + (lane - sseg[w][k].y);
-                    const SPt<T, D> t = tpts[pos];
-#pragma unroll
-                    for (int d = 0; d < D; ++d) sx[w][d][lane] = t.x[d];
-                    if (nbox == 1) {
-                        near = box_gap2<T, D>(qlo, qhi, t.x, t.x) <= r2;
-                    } else {
-                        for (int b = 0; b < nbox && !near; ++b)
-                            near = box_gap2<T, D>(&sbox[w][b][0], &sbox[w][b][D], t.x, t.x) <= r2;
-                    }
-                    if (self_pair) {  // query and target are the same tree: the group's own points
-                        const int64_t sl = pos - grp.x;
-                        if (sl >= 0 && sl < grp.y) sself[w][sl] = (chunk << 5) | lane;
-                    }
-                } else if (lane < mp) {
-#pragma unroll
-                    for (int d = 0; d < D; ++d) sx[w][d][lane] = T(INFINITY);
-                }
-                const unsigned keep = __ballot_sync(0xffffffffu, near);
-                __syncwarp();
-                if (prefetch && c0 + kStage >= nb) {
-                    // The next chunk's points (the leaves now at the stack top)
-                    // start their way into L1 while this chunk's pairs are tested.
-                    int acc = 0, ppos = -1;
-                    for (int j = sp - 1; j >= 0 && acc < 32; --j) {
-                        const int2 nx = stack[w][j];
-                        if (nx.y <= 0) break;
-                        if (lane >= acc && lane < acc + nx.y) ppos = (nx.x & 0x7fffffff) + (lane - acc);
-                        acc += nx.y;
-                    }
-                    if (ppos >= 0) prefetch_l1(tpts + ppos);
-                }
-                unsigned hm = 0;
-                long long st_p0 = 0;
-                if constexpr (STATS) {
-                    st_p0 = clock64();
-                    ++st_chunks;
-                    st_targets += total;
-                    st_steps += std::is_same<T, float>::value
-                                    ? __popc((keep | keep >> 1 | keep >> 2 | keep >> 3) & 0x11111111u)
-                                    : __popc(keep);
-                }
-                if constexpr (std::is_same<T, float>::value) {
-                    unsigned long long P[D];
-#pragma unroll
-                    for (int d = 0; d < D; ++d) P[d] = pack2(q.x[d], q.x[d]);
-                    // one bit per step of four targets with a target kept
-                    const unsigned steps = (keep | keep >> 1 | keep >> 2 | keep >> 3) & 0x11111111u;
-                    for (unsigned km = steps; km; km &= km - 1) {
-                        const int j = __ffs(km) - 1;
-                        // Four targets per step, two per packed operation:
-                        // packed differences and squares, scalar sums
-                        // ((dx*dx + dy*dy) + dz*dz) per element.  The sums stay
-                        // scalar: packed add.rn.f32x2 sums after the packed
-                        // squares changed results (8 of 1,547,624,876 edges of
-                        // the 4M-point 2D set), as a fused multiply-add would.
-                        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-#pragma unroll
-                        for (int d = 0; d < D; ++d) {
-                            const unsigned long long* px = reinterpret_cast<const unsigned long long*>(&sx[w][d][j]);
-                            const unsigned long long da = sub2_rn(px[0], P[d]);
-                            const unsigned long long db = sub2_rn(px[1], P[d]);
-                            const unsigned long long qa = mul2_rn(da, da);
-                            const unsigned long long qb = mul2_rn(db, db);
-                            s0 = (d == 0) ? lo2(qa) : __fadd_rn(s0, lo2(qa));
-                            s1 = (d == 0) ? hi2(qa) : __fadd_rn(s1, hi2(qa));
-                            s2 = (d == 0) ? lo2(qb) : __fadd_rn(s2, lo2(qb));
-                            s3 = (d == 0) ? hi2(qb) : __fadd_rn(s3, hi2(qb));
-                        }
-                        hm |= ((s0 <= r2 ? 1u : 0u) | (s1 <= r2 ? 2u : 0u) | (s2 <= r2 ? 4u : 0u) |
-                               (s3 <= r2 ? 8u : 0u)) << j;
-                    }
-                } else {
-                    for (unsigned km = keep; km; km &= km - 1) {
-                        const int j = __ffs(km) - 1;
-                        T t[D], diff[D];
-#pragma unroll
-                        for (int d = 0; d < D; ++d) t[d] = sx[w][d][j];
-                        hm |= (dist2<T, D>(t, q.x, diff) <= r2 ? 1u : 0u) << j;
-                    }
-                }
-                if constexpr (STATS) st_pairs += clock64() - st_p0;
-                if (!valid) hm = 0;
-                if (self_pair) {
-                    const int v = sself[w][lane];
-                    if ((v >> 5) == chunk) hm &= ~(1u << (v & 31));
-                }
-                const int nh = __popc(hm);
-                cnt += nh;
-                if (PASS == EP_RECORD) {
-                    // One record per leaf segment with hits, in pop order.
-                    if (__any_sync(0xffffffffu, hm != 0)) {
-                        for (int k = 0; k < nseg; ++k) {
-                            const int2 sg = sseg[w][k];
-                            const int len = sseg[w][k + 1].y - sg.y;
-                            const unsigned sub = (hm >> sg.y) & (0xffffffffu >> (32 - len));
-                            if (sub != 0u && nrec < cap) myrec[nrec] = make_int2(sg.x, (int32_t)sub);
-                            nrec += sub != 0u;
-                        }
-                    }
-                } else if (STAGE) {
-                    if (__any_sync(0xffffffffu, ocnt + nh > kStage)) flush(ocnt + nh > kStage);
-                    for (int k = 0; k < nseg; ++k) {
-                        const int2 sg = sseg[w][k];
-                        const int len = sseg[w][k + 1].y - sg.y;
-                        unsigned sub = (hm >> sg.y) & (len >= 32 ? 0xffffffffu : ((1u << len) - 1u));
-                        while (sub) {
-                            const int j = __ffs(sub) - 1;
-                            sub &= sub - 1;
-                            obuf[w][lane][ocnt++] = sg.x + j;
-                        }
-                    }
-                }
-                if constexpr (STATS) st_leaf += clock64() - st_c0;
+                const uint2 up = swalk[w][l];
+                m = up.x;
+                b0 = (int32_t)up.y;
             }
-        } else {
-            // Internal nodes.  The popped node and up to kMultiPop - 1 further
-            // internal entries at the stack top (the nodes the DFS expands
-            // next) have their children box-tested together, one lane per
-            // child; each node's passing children are pushed as a block, the
-            // first node's on top, so the visiting order is unchanged.  Only
-            // while the stack stays at most kMultiLimit deep: beyond it the
-            // usual single expansions bound the depth.
-            // The reference scans an internal node whose first child slot is
-            // empty as one leaf, in ascending position order
-            // (src/cpu/iterator_cpu.jl:87-101).  Below such a node the
-            // children are therefore visited in ascending slot order.
-            int nnodes = 1, totc = __popc((unsigned)(-nb));
-            if (lane == 0) {
-                snode[w][0] = ent;
-                soff[w][0] = 0;
+            continue;
+        }
+        const int i = __ffs(m) - 1;
+        m &= m - 1;
+        if (l > 0) {
+            __syncwarp();
+            if (lane == 0) swalk[w][l] = make_uint2(m, (unsigned)b0);
+            b0 = (b0 + i) * 32;
+            --l;
+            m = test(l, b0, min(b0 + 32, bv.cnt[l]));
+            continue;
+        }
+        const int32_t c0 = __shfl_sync(FULL, na, i);
+        const int nc = __shfl_sync(FULL, nb, i);
+        for (int cb = 0; cb < nc; cb += 32) {
+            int32_t first = 0, num = 0;
+            bool pass = false;
+            if (cb + lane < nc) {
+                const TNode<float, D> nd = bv.chunk[c0 + cb + lane];
+                pass = boxes_near<D>(gc.lo, gc.hi, nd.lo, nd.hi, lim) && nd.a >= plo && nd.a < phi;
+                first = nd.a;
+                num = nd.b;
             }
-            while (nnodes < multi_pop && sp > 0) {
-                const int2 nx = stack[w][sp - 1];
-                if (nx.y > 0) break;
-                const int c = __popc((unsigned)(-nx.y));
-                if (totc + c > 32 || sp - 1 + totc + c > kMultiLimit) break;
-                --sp;
-                if (lane == 0) {
-                    snode[w][nnodes] = nx;
-                    soff[w][nnodes] = totc;
-                }
-                totc += c;
-                ++nnodes;
-            }
-            if (lane == 0) soff[w][nnodes] = totc;
             if constexpr (STATS) {
                 ++st_exp;
-                st_children += totc;
+                st_children += min(32, nc - cb);
             }
-            __syncwarp();
-            int j = 0;
-            if (lane < totc)
-                while (soff[w][j + 1] <= lane) ++j;
-            const int2 nd = snode[w][j];
-            const unsigned slots = (unsigned)(-nd.y);
-            const bool casc = nd.x < 0 || !(slots & 1u);
-            const int o = soff[w][j], o2 = soff[w][j + 1];
-            bool pass = false;
-            int2 rec = make_int2(0, 0);
-            if (lane < totc) {
-                const TNode<T, D> c = tnode[(nd.x & 0x7fffffff) + (lane - o)];
-                pass = box_gap2<T, D>(qlo, qhi, c.lo, c.hi) <= r2;
-                rec = make_int2(c.a | (casc ? (int32_t)0x80000000 : 0), c.b);
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, pass);
-            if (pass) {
-                const unsigned upto = o2 >= 32 ? 0xffffffffu : ((1u << o2) - 1u);  // lanes of nodes <= j
-                const unsigned mine = m & upto & ~((1u << o) - 1u);
-                const int deeper = __popc(m & ~upto);  // passing children of the later nodes, below
-                const int np = __popc(mine);
-                const int rk = __popc(mine & lanemask_lt());
-                stack[w][sp + deeper + (casc ? np - 1 - rk : rk)] = rec;
-            }
-            sp += __popc(m);
-            __syncwarp();
-            if (prefetch && sp > 0) {
-                // what the next pop reads: an internal node's children, or a leaf's points
-                const int2 nx = stack[w][sp - 1];
-                const int32_t a = nx.x & 0x7fffffff;
-                if (nx.y <= 0) {
-                    if (lane < __popc((unsigned)(-nx.y))) prefetch_l1(tnode + a + lane);
-                } else if (lane < nx.y) {
-                    prefetch_l1(tpts + a + lane);
-                }
+            unsigned cm = __ballot_sync(FULL, pass);
+            while (cm) {
+                const int j = __ffs(cm) - 1;
+                cm &= cm - 1;
+                const int32_t f = __shfl_sync(FULL, first, j);
+                const int k = __shfl_sync(FULL, num, j);
+                SPt<T, D> t;
+                if (lane < k) t = tpts[f + lane];
+                visit(f, k, t);
             }
         }
     }
     if (STAGE) flush(true);
-    if (PASS != EP_FILL && valid) counts[q.idx] = (int32_t)cnt;
+    if (PASS != EP_FILL && valid) {
+        counts[q.idx] = cnt;
+        if (PASS == EP_RECORD || PASS == EP_COUNT) {
+            if (qpos_of) qpos_of[q.idx] = (int32_t)qpos;
+        }
+    }
     if constexpr (STATS) {
         const unsigned long long hits = warp_sum((unsigned long long)cnt);
-        const int nv = __popc(__ballot_sync(0xffffffffu, valid));
+        const int nv = __popc(__ballot_sync(FULL, valid));
         if (lane == 0) {
             const unsigned long long v[TS_NUM] = {1ull, (unsigned long long)nv, st_exp, st_children, st_chunks,
                                                   st_targets, st_steps, 4ull * st_steps * (unsigned long long)nv, hits,
@@ -503,11 +565,9 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edges(
         }
     }
     if (PASS == EP_RECORD) {
-        const bool over = __any_sync(0xffffffffu, nrec > cap);
+        const bool over = __any_sync(FULL, nrec > cap);
         if (valid) rcount[qpos] = over ? kOverflowMark : (uint16_t)nrec;
-        int mx = nrec;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const int mx = __reduce_max_sync(FULL, nrec);
         if (lane == 0) {
             gflag[g] = over ? 1 : 0;
             if (over) atomicAdd(ocount, 1);
@@ -546,7 +606,7 @@ __device__ __forceinline__ int kth_set_bit(unsigned m, int k) {
 //     window set one bit each at their first record in the window (the one
 //     running into the window at bit 0), so the query of record l is the
 //     (popc of the bits up to l)-th of them (ballot, reduce-or, popc; no search);
-//   * an edge's target is its record's leaf position plus the bit from the
+//   * an edge's target is its record's chunk position plus the bit from the
 //     table; its query's coordinates, index and radius come from the query's
 //     lane by shuffles.
 // Edge f of the flat list goes to COO slot kb[q] + f of its query q (slots
@@ -556,7 +616,7 @@ constexpr int kDirectWarps = 4;
 
 template <class T, int D>
 __global__ void __launch_bounds__(kDirectWarps * 32, sizeof(T) == 4 ? 10 : 1) k_expand_direct(
-    int64_t nq, const int32_t* __restrict__ iperm, const SPt<T, D>* __restrict__ qpts,
+    int64_t nq, const int32_t* __restrict__ qpos_of, const SPt<T, D>* __restrict__ qpts,
     const SPt<T, D>* __restrict__ tpts, const int64_t* __restrict__ offsets, const int2* __restrict__ recs,
     int64_t rec_cap, const uint16_t* __restrict__ rcount, T inv_r, int32_t* __restrict__ senders,
     int32_t* __restrict__ receivers, T* __restrict__ rdisp, T* __restrict__ rdist, Batch bt) {
@@ -572,7 +632,7 @@ __global__ void __launch_bounds__(kDirectWarps * 32, sizeof(T) == 4 ? 10 : 1) k_
     const int64_t i = i0 + lane;
     const bool valid = i < nq;
     const int64_t K0 = offsets[i0];  // the warp's first COO slot
-    const int32_t qp = valid ? iperm[i] : 0;
+    const int32_t qp = valid ? qpos_of[i] : 0;
     int nr = valid ? rcount[qp] : 0;
     int ne = 0;
     long long krel = 0;
@@ -585,8 +645,8 @@ __global__ void __launch_bounds__(kDirectWarps * 32, sizeof(T) == 4 ? 10 : 1) k_
     }
     const SPt<T, D> q = qpts[qp];
     T r2 = T(0), ir = inv_r;
-    int32_t start_node = 0, base = 0;
-    cloud_params<T>(bt, qp, r2, ir, start_node, base);
+    int32_t base = 0;
+    cloud_params<T>(bt, qp, r2, ir, base);
     const int32_t qi = q.idx - base + 1;
     const bool feat = rdisp != nullptr;  // false: neighbor lists (CSR values) only
     const unsigned le = full >> (31 - lane);  // lanes up to this one
@@ -741,7 +801,7 @@ __host__ __device__ constexpr size_t fill_ring_bytes(int ring) {
 
 template <class T, int D, bool FEAT, int CHUNK, int NCH>
 __global__ void __launch_bounds__(kFillWarps * 32) k_expand(
-    int64_t nq, const int32_t* __restrict__ iperm, const SPt<T, D>* __restrict__ qpts,
+    int64_t nq, const int32_t* __restrict__ qpos_of, const SPt<T, D>* __restrict__ qpts,
     const SPt<T, D>* __restrict__ tpts, const int64_t* __restrict__ offsets, const int2* __restrict__ recs,
     int64_t rec_cap, const uint16_t* __restrict__ rcount, T inv_r, int32_t* __restrict__ senders,
     int32_t* __restrict__ receivers, T* __restrict__ rdisp, T* __restrict__ rdist, Batch bt, int bulk_ok) {
@@ -765,7 +825,7 @@ __global__ void __launch_bounds__(kFillWarps * 32) k_expand(
     const int64_t i = i0 + lane;
     const bool valid = i < nq;
     const int nval = nq - i0 < 32 ? (int)(nq - i0) : 32;
-    const int32_t qp = valid ? iperm[i] : 0;
+    const int32_t qp = valid ? qpos_of[i] : 0;
     int nr = valid ? rcount[qp] : 0;
     const bool over = valid && nr == kOverflowMark;
     const long long k0 = valid ? offsets[i] : 0;
@@ -777,8 +837,8 @@ __global__ void __launch_bounds__(kFillWarps * 32) k_expand(
     }
     const SPt<T, D> q = qpts[qp];
     T r2 = T(0), ir = inv_r;
-    int32_t start_node = 0, base = 0;
-    cloud_params<T>(bt, qp, r2, ir, start_node, base);
+    int32_t base = 0;
+    cloud_params<T>(bt, qp, r2, ir, base);
     const int32_t qi = q.idx - base + 1;
     // record and hit prefixes over the queries
     int rincl = nr, eincl = ne;
@@ -1033,7 +1093,7 @@ int count_typed(Ctx& ctx, const Tree& q, const Tree& t, bool exclude_self, int64
     cudaStream_t s = ctx.stream;
     const int64_t nq = q.n;
     if ((err = ensure(ctx.counts, (size_t)std::max<int64_t>(nq, 1) * 4)) ||
-        (err = ensure(ctx.offsets, (size_t)(nq + 1) * 8)) ||
+        (err = ensure(ctx.qpos, (size_t)std::max<int64_t>(nq, 1) * 4)) || (err = ensure(ctx.offsets, (size_t)(nq + 1) * 8)) ||
         (err = ensure(ctx.scan_tmp, (size_t)scan_tmp_elems(nq) * 8)) || (err = ensure(ctx.total, 16)) ||
         (err = ensure(ctx.dstatus, 8)))
         return cuda_status(ctx, err, "allocating edge scratch");
@@ -1061,19 +1121,12 @@ int count_typed(Ctx& ctx, const Tree& q, const Tree& t, bool exclude_self, int64
         }
         PhaseTimer pt_(ctx, PH_COUNT);
         const int64_t ng = q.n_groups;
-        if (ctx.rec_cap)
-            launch_pdl(k_edges<T, D, EP_RECORD>, div_up(ng, kEdgeWarps), kEdgeThreads, 0, s, q.spts.as<SPt<T, D>>(),
-                q.groups.as<int2>(), ng, t.tnode.as<TNode<T, D>>(), t.dfs_start, t.spts.as<SPt<T, D>>(), t.n_nodes, r2,
-                T(0), exclude_self ? 1 : 0, ctx.counts.as<int32_t>(), nullptr, nullptr, nullptr, nullptr, nullptr,
-                (int*)(ctx.total.as<int64_t>() + 1), ctx.recs.as<int2>(), ctx.rec_cap, ctx.rcount.as<uint16_t>(),
-                ctx.gflag.as<uint8_t>(), t.batch(), nullptr, tn.max_seg, tn.multi_pop, tn.sub_boxes, tn.prefetch,
-                own_start(q, t));
-        else
-            launch_pdl(k_edges<T, D, EP_COUNT>, div_up(ng, kEdgeWarps), kEdgeThreads, 0, s, q.spts.as<SPt<T, D>>(),
-                q.groups.as<int2>(), ng, t.tnode.as<TNode<T, D>>(), t.dfs_start, t.spts.as<SPt<T, D>>(), t.n_nodes, r2,
-                T(0), exclude_self ? 1 : 0, ctx.counts.as<int32_t>(), nullptr, nullptr, nullptr, nullptr, nullptr,
-                nullptr, nullptr, 0, nullptr, nullptr, t.batch(), nullptr, tn.max_seg, tn.multi_pop, tn.sub_boxes,
-                tn.prefetch, own_start(q, t));
+        const auto kern = ctx.rec_cap ? k_edges<T, D, EP_RECORD> : k_edges<T, D, EP_COUNT>;
+        launch_pdl(kern, div_up(ng, kEdgeWarps), kEdgeThreads, 0, s, q.dpts.as<SPt<T, D>>(),
+            q.chunk.as<TNode<float, D>>(), ng, t.search_layout<D>(), t.dpts.as<SPt<T, D>>(), t.n, r2, T(0),
+            exclude_self ? 1 : 0, ctx.counts.as<int32_t>(), ctx.qpos.as<int32_t>(), nullptr, nullptr, nullptr, nullptr,
+            nullptr, (int*)(ctx.total.as<int64_t>() + 1), ctx.rec_cap ? ctx.recs.as<int2>() : nullptr, ctx.rec_cap,
+            ctx.rcount.as<uint16_t>(), ctx.gflag.as<uint8_t>(), t.batch(), nullptr);
         ctx.kernel_launches += 1;
     }
     {
@@ -1115,7 +1168,7 @@ cudaError_t launch_expand_shape(Ctx& ctx, const Tree& q, const Tree& t, T inv_r,
         }
     }
     kern<<<div_up(q.n, 32 * kFillWarps), kFillWarps * 32, smem, ctx.stream>>>(
-        q.n, q.iperm.as<int32_t>(), q.spts.as<SPt<T, D>>(), t.spts.as<SPt<T, D>>(), ctx.offsets.as<int64_t>(),
+        q.n, ctx.qpos.as<int32_t>(), q.dpts.as<SPt<T, D>>(), t.dpts.as<SPt<T, D>>(), ctx.offsets.as<int64_t>(),
         ctx.recs.as<int2>(), ctx.rec_cap, ctx.rcount.as<uint16_t>(), inv_r, senders, receivers, (T*)rel_disp,
         (T*)rel_dist, t.batch(), bulk_ok);
     return cudaGetLastError();
@@ -1138,7 +1191,7 @@ cudaError_t launch_expand(Ctx& ctx, const Tree& q, const Tree& t, T inv_r, int32
                                                         bulk_ok);
         default:  // direct stores
             launch_pdl(k_expand_direct<T, D>, div_up(q.n, 32 * kDirectWarps), kDirectWarps * 32, 0, ctx.stream, q.n,
-                q.iperm.as<int32_t>(), q.spts.as<SPt<T, D>>(), t.spts.as<SPt<T, D>>(), ctx.offsets.as<int64_t>(),
+                ctx.qpos.as<int32_t>(), q.dpts.as<SPt<T, D>>(), t.dpts.as<SPt<T, D>>(), ctx.offsets.as<int64_t>(),
                 ctx.recs.as<int2>(), ctx.rec_cap, ctx.rcount.as<uint16_t>(), inv_r, senders, receivers, (T*)rel_disp,
                 (T*)rel_dist, t.batch());
             return cudaGetLastError();
@@ -1152,12 +1205,9 @@ int fill_typed(Ctx& ctx, const Tree& q, const Tree& t, bool exclude_self, int32_
     const T r2 = r * r;
     const T inv_r = T(1) / r;  // inv(r), src/cpu/edges_cpu.jl:185
     cudaStream_t s = ctx.stream;
-    const Tuning& tn = ctx.plan_tuning;  // the shapes of the count this fill follows
     PhaseTimer pt_(ctx, PH_FILL);
     const int64_t ng = q.n_groups;
     if (ctx.rec_cap) {
-        const int st = ensure_iperm(ctx, q);  // the fill visits the queries in original index order
-        if (st != OK) return st;
         const bool feat = rel_disp != nullptr;
         auto aligned = [](const void* p) { return ((uintptr_t)p & 15u) == 0; };
         const int bulk_ok = aligned(senders) && (!feat || (aligned(receivers) && aligned(rel_disp) && aligned(rel_dist)));
@@ -1171,11 +1221,10 @@ int fill_typed(Ctx& ctx, const Tree& q, const Tree& t, bool exclude_self, int32_
     if (!ctx.rec_cap || ctx.rec_overflow) {
         // Groups without complete records walk the tree again.
         k_edges<T, D, EP_FILL><<<div_up(ng, kEdgeWarps), kEdgeThreads, 0, s>>>(
-            q.spts.as<SPt<T, D>>(), q.groups.as<int2>(), ng, t.tnode.as<TNode<T, D>>(), t.dfs_start,
-            t.spts.as<SPt<T, D>>(), t.n_nodes, r2, inv_r, exclude_self ? 1 : 0, nullptr, ctx.offsets.as<int64_t>(),
-            senders, receivers, (T*)rel_disp, (T*)rel_dist, ctx.dstatus.as<int>(),
-            ctx.rec_cap ? ctx.recs.as<int2>() : nullptr, ctx.rec_cap, nullptr, ctx.gflag.as<uint8_t>(), t.batch(),
-            nullptr, tn.max_seg, tn.multi_pop, tn.sub_boxes, tn.prefetch, own_start(q, t));
+            q.dpts.as<SPt<T, D>>(), q.chunk.as<TNode<float, D>>(), ng, t.search_layout<D>(), t.dpts.as<SPt<T, D>>(),
+            t.n, r2, inv_r, exclude_self ? 1 : 0, nullptr, nullptr, ctx.offsets.as<int64_t>(), senders, receivers,
+            (T*)rel_disp, (T*)rel_dist, ctx.dstatus.as<int>(), ctx.rec_cap ? ctx.recs.as<int2>() : nullptr,
+            ctx.rec_cap, nullptr, ctx.gflag.as<uint8_t>(), t.batch(), nullptr);
         ctx.kernel_launches += 1;
     }
     return cuda_status(ctx, cudaGetLastError(), "edge fill launch");
@@ -1198,9 +1247,9 @@ cudaError_t count_into_typed(const Tree& q, const Tree& t, bool exclude_self, in
     const T r = (T)t.radius;
     const T r2 = r * r;
     k_edges<T, D, EP_COUNT><<<div_up(q.n_groups, kEdgeWarps), kEdgeThreads, 0, s>>>(
-        q.spts.as<SPt<T, D>>(), q.groups.as<int2>(), q.n_groups, t.tnode.as<TNode<T, D>>(), t.dfs_start,
-        t.spts.as<SPt<T, D>>(), t.n_nodes, r2, T(0), exclude_self ? 1 : 0, counts, nullptr, nullptr, nullptr,
-        nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, t.batch(), nullptr, kMaxSeg, kMultiPop, 1, 0, nullptr);
+        q.dpts.as<SPt<T, D>>(), q.chunk.as<TNode<float, D>>(), q.n_groups, t.search_layout<D>(),
+        t.dpts.as<SPt<T, D>>(), t.n, r2, T(0), exclude_self ? 1 : 0, counts, nullptr, nullptr, nullptr, nullptr,
+        nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, t.batch(), nullptr);
     return cudaGetLastError();
 }
 
@@ -1208,12 +1257,10 @@ template <class T, int D>
 int stats_typed(Ctx& ctx, const Tree& q, const Tree& t, bool exclude_self, unsigned long long* stats_dev) {
     const T r = (T)t.radius;
     const T r2 = r * r;
-    const Tuning tn = ctx.tuning_for(t.ndims, t.dtype, q.n, q.nbrs_hint);
     k_edges<T, D, EP_STATS><<<div_up(q.n_groups, kEdgeWarps), kEdgeThreads, 0, ctx.stream>>>(
-        q.spts.as<SPt<T, D>>(), q.groups.as<int2>(), q.n_groups, t.tnode.as<TNode<T, D>>(), t.dfs_start,
-        t.spts.as<SPt<T, D>>(), t.n_nodes, r2, T(0), exclude_self ? 1 : 0, ctx.counts.as<int32_t>(), nullptr, nullptr,
-        nullptr, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, t.batch(), stats_dev, tn.max_seg,
-        tn.multi_pop, tn.sub_boxes, tn.prefetch, own_start(q, t));
+        q.dpts.as<SPt<T, D>>(), q.chunk.as<TNode<float, D>>(), q.n_groups, t.search_layout<D>(),
+        t.dpts.as<SPt<T, D>>(), t.n, r2, T(0), exclude_self ? 1 : 0, ctx.counts.as<int32_t>(), nullptr, nullptr,
+        nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, t.batch(), stats_dev);
     ctx.kernel_launches += 1;
     return cuda_status(ctx, cudaGetLastError(), "traversal statistics launch");
 }

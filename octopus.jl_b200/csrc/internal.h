@@ -109,7 +109,7 @@ struct Tree {
     const void* skeys_dev = nullptr;    // sorted keys of the last build (key_bytes wide)
     DevBuf tnode;                // TNode<T,D>[capacity]
     DevBuf nrange;               // int2 {first,last} 0-based per node
-    DevBuf parent;               // int32 per node (-1 for the root)
+    DevBuf link;                 // NodeLink per node: parent, children, for climbing
     DevBuf fchild;               // int32 per node: first child id from the id pass
     DevBuf arrive;               // int32 per node, refit arrival counters
     DevBuf lohi;                 // uint16 per position: first | last level starting here
@@ -119,11 +119,15 @@ struct Tree {
     DevBuf partials;             // double per-block bounds partials
     DevBuf hdr;                  // OctHeader
     DevBuf morton;               // uint64 per original point (refit mode), filled with the views
-    DevBuf groups;               // int2 {first position, count <= 32}: query groups
-    DevBuf gstart;               // int32 per group: traversal start node (| 1 << 30: ascending flag), -1 = root
-    int64_t n_groups = 0;
-    int32_t dfs_start = 0;
-    DevBuf chain;                // int32[64]: full-range chain node ids and flags
+    // Search layout (Bvh): what build_edges reads.
+    DevBuf dpts;                 // SPt<T,D>[n] in the search's visiting order
+    DevBuf dstart;               // uint8 per visiting position: point count of the chunk starting there, else 0
+    DevBuf dnode, rbox;          // a run's first leaf (int32, at its start) and its box (TNode<float,D> at that leaf)
+    DevBuf chunk;                // TNode<float,D> per chunk: box, first position, count <= group_cap
+    DevBuf bvh;                  // TNode<float,D>: the box hierarchy's levels, one after another
+    DevBuf bvh_arrive;           // int32 per node above the lowest level: children done
+    int64_t n_groups = 0;        // chunks
+    int32_t asc_key = 0;         // OctHeader::asc_key of the last topology
 
     // Refit mode across time steps: the previous build's sorted keys and
     // permutation (keys[sorted_buf], vals[sorted_buf]) seed the next build.
@@ -146,7 +150,6 @@ struct Tree {
     mutable double nbrs_hint = -1.0;
     DevBuf b_coff;               // int64 [n_clouds + 1]
     DevBuf b_cparam;             // double [n_clouds * kCloudParams]
-    DevBuf b_croot, b_cstart;    // int32 [n_clouds]
     DevBuf b_cbounds;            // double [n_clouds * 8] per-cloud reduce
     DevBuf b_eoff;               // int64 [n_clouds + 1] per-cloud edge offsets
     Batch batch() const {
@@ -155,11 +158,31 @@ struct Tree {
         b.kbits = kbits;
         b.coff = b_coff.as<int64_t>();
         b.cparam = b_cparam.as<double>();
-        b.croot = b_croot.as<int32_t>();
-        b.cstart = b_cstart.as<int32_t>();
         return b;
     }
-    int64_t group_capacity = 0;
+    // The box hierarchy's shape for n points: level sizes, and their sum.
+    static int32_t bvh_levels(int64_t n, int32_t* cnt, int64_t* total) {
+        int32_t top = 0;
+        cnt[0] = (int32_t)((n + kSpan - 1) / kSpan);
+        *total = cnt[0];
+        while (cnt[top] > 64 && top + 1 < kBvhLevels) {
+            cnt[top + 1] = (cnt[top] + 31) / 32;
+            *total += cnt[++top];
+        }
+        return top;
+    }
+    template <int D> Bvh<D> search_layout() const {
+        Bvh<D> b;
+        int64_t total = 0;
+        b.top = bvh_levels(n, b.cnt, &total);
+        b.chunk = chunk.as<TNode<float, D>>();
+        TNode<float, D>* p = bvh.as<TNode<float, D>>();
+        for (int l = 0; l <= b.top; ++l) {
+            b.lev[l] = p;
+            p += b.cnt[l];
+        }
+        return b;
+    }
     OctHeader* hdr_host = nullptr;  // pinned
 
     // Lazily materialized reference-layout views (DeviceView contract,
@@ -174,6 +197,7 @@ struct Ctx {
     std::string last_error;
     // Edge-count state carried from oct_edges_count to oct_edges_fill.
     DevBuf counts;       // int32 per query point
+    DevBuf qpos;         // int32 per query point: its position in the query tree's visiting order
     DevBuf offsets;      // int64 per query point + 1
     DevBuf scan_tmp;     // int64 tile sums
     DevBuf total;        // int64 device total, then the count of overflowed record groups
