@@ -820,7 +820,8 @@ class BatchedSearch:
         if len(sizes) != len(radii) or len(sizes) == 0:
             raise DimensionMismatch("sizes and radii need one entry per cloud")
         # radii in the element type, like set_search_radius! (src/api.jl:26)
-        radii = np.asarray([float(torch.tensor(float(r), dtype=self.T).item()) for r in radii], np.float64)
+        with np.errstate(over="ignore"):
+            radii = radii.astype(np.float32 if self.T == torch.float32 else np.float64).astype(np.float64)
         coff = np.zeros(len(sizes) + 1, np.int64)
         coff[1:] = np.cumsum(sizes)
         self.coords = colmajor(coords)

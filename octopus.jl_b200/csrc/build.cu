@@ -1666,7 +1666,7 @@ int build_typed(Ctx& ctx, Tree& t, const T* coords, int64_t n, double radius_d) 
     const T radius = (T)radius_d;
     if ((err = ensure(t.hdr, sizeof(OctHeader)))) return cuda_status(ctx, err, "allocating header");
     if (!t.hdr_host) {
-        if ((err = cudaMallocHost((void**)&t.hdr_host, sizeof(OctHeader)))) return cuda_status(ctx, err, "pinned header");
+        if ((err = header_alloc(&t.hdr_host))) return cuda_status(ctx, err, "pinned header");
     }
     OctHeader* hdr = t.hdr.as<OctHeader>();
     if ((err = cudaMemsetAsync(hdr, 0, sizeof(OctHeader), s))) return cuda_status(ctx, err, "header reset");
@@ -1743,7 +1743,7 @@ int build_batch_typed(Ctx& ctx, Tree& t, const T* coords, int64_t n, const int64
         (err = ensure(t.b_eoff, (size_t)(nc + 1) * 8)))
         return cuda_status(ctx, err, "allocating batch arrays");
     if (!t.hdr_host) {
-        if ((err = cudaMallocHost((void**)&t.hdr_host, sizeof(OctHeader)))) return cuda_status(ctx, err, "pinned header");
+        if ((err = header_alloc(&t.hdr_host))) return cuda_status(ctx, err, "pinned header");
     }
     if ((err = cudaMemsetAsync(t.hdr.p, 0, sizeof(OctHeader), s)) ||
         (err = cudaMemcpyAsync(t.b_coff.p, coff_host, (size_t)(nc + 1) * 8, cudaMemcpyHostToDevice, s)))

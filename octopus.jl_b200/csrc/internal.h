@@ -19,7 +19,13 @@ struct DevBuf {
 };
 
 cudaError_t ensure(DevBuf& b, size_t bytes);
-void release(DevBuf& b);
+void release(DevBuf& b, bool idle);  // idle: the device was synchronized since its last use
+bool device_idle();
+// A tree's pinned header block, and the number of contexts on the current
+// device (the device's pool is emptied with the last).
+cudaError_t header_alloc(OctHeader** h);
+void header_free(OctHeader* h);
+void pool_context(int delta);
 
 struct Ctx;
 
