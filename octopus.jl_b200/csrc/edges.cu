@@ -577,6 +577,35 @@ __global__ void __launch_bounds__(kEdgeThreads, kEdgeBlocks<T>) k_edges(
     }
 }
 
+// The D values of rel_displacement column k (T-aligned D-tuples).  PAIRS: the
+// array is aligned to two values, so two of them leave as one word: in 3D the
+// first two of an even column and the last two of an odd one, which halves the
+// columns' strided stores in the same two instructions for every lane.
+template <class T> struct Pair;
+template <> struct Pair<float> { using type = float2; };
+template <> struct Pair<double> { using type = double2; };
+template <class T, int D>
+__device__ __forceinline__ void store_column(T* __restrict__ rdisp, int64_t k, const T* v, bool pairs) {
+    using P = typename Pair<T>::type;
+    T* p = rdisp + (int64_t)D * k;
+    if (!pairs) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) p[d] = v[d];
+    } else if constexpr (D == 2) {
+        P w;
+        w.x = v[0];
+        w.y = v[1];
+        *reinterpret_cast<P*>(p) = w;
+    } else {
+        const bool odd = k & 1;
+        P w;
+        w.x = odd ? v[1] : v[0];
+        w.y = odd ? v[2] : v[1];
+        *reinterpret_cast<P*>(p + (odd ? 1 : 0)) = w;
+        p[odd ? 0 : 2] = odd ? v[0] : v[2];
+    }
+}
+
 // Position (0..31) of the k-th set bit (k from 0) of m; k < popc(m).
 __device__ __forceinline__ int kth_set_bit(unsigned m, int k) {
     int pos = 0;
@@ -594,39 +623,65 @@ __device__ __forceinline__ int kth_set_bit(unsigned m, int k) {
 }
 
 // Fill pass from the records with direct stores, in original index order
-// (the default fill; k_expand below writes through bulk copies instead, a
-// tuned alternative).  Warp v owns queries 32v .. 32v+31, one per lane; their
-// records, query after query, form one flat list, and so do their edges, in
-// the same order (a record's hits are consecutive edges of its query).  The
-// warp loads the records 32 at a time (one per lane), scans their hit counts,
-// lists each edge's (record lane, bit) in a per-warp shared-memory table (each
-// record lane writes its hits at its edges' slots), and writes the batch's
-// edges 32 at a time, one per lane:
+// (the default fill; k_expand below writes through bulk copies instead: a
+// tuned alternative, and the fill of more than 2^27 targets).  Warp v owns
+// queries 32v .. 32v+31, one per lane; their records, query after query, form
+// one flat list, and so do their edges, in the same order (a record's hits are
+// consecutive edges of its query).  The warp loads the records 32 at a time
+// (one per lane), scans their hit counts and appends each hit (query lane <<
+// 27 | target position) to a list in shared memory; whenever the list holds a
+// round of 64 edges it writes them, one per lane and window of 32:
 //   * a record's query: the queries whose records reach into the 32-record
 //     window set one bit each at their first record in the window (the one
 //     running into the window at bit 0), so the query of record l is the
 //     (popc of the bits up to l)-th of them (ballot, reduce-or, popc; no search);
-//   * an edge's target is its record's chunk position plus the bit from the
-//     table; its query's coordinates, index and radius come from the query's
-//     lane by shuffles.
-// Edge f of the flat list goes to COO slot kb[q] + f of its query q (slots
-// relative to the warp's first slot).  Queries of an
-// overflowed group (record count kOverflowMark) are left to the walking fill.
+//   * windows start at multiples of 32 COO slots, so a window's index and
+//     distance stores are one 128-byte line each (4-byte elements), and are
+//     full except at the two ends of the warp's range;
+//   * consecutive lanes take consecutive edges: their targets share chunks
+//     and their queries' data (one 16-byte load of shared memory) is mostly
+//     the same.
+// Edge f of the flat list goes to COO slot kb[q] + f of its query q.  Queries
+// of an overflowed group (record count kOverflowMark) are left to the walking
+// fill.
+//
+// Bound by L1 (72% on a 343,000-point lattice: the gathered targets and the
+// strided columns) and instruction issue (68%), at 3.5 to 3.8 TB/s of COO.
+// Against windows that start and end with each batch of 32 records, with the
+// query's data by shuffles and one store per value: 1M lattice points 225 ->
+// 193 us, 1M clustered 2D points (151 M edges) 985 -> 800, 2M uniform points
+// 299 -> 288, 100,000 points 35 -> 32.  Rounds of one or three windows, lists
+// of 256 or 960 further hits, 7 to 12 blocks per SM were equal or slower; four
+// consecutive edges per lane with 16-byte stores was 5 to 25% slower (its
+// gathers touch four times as many lines per instruction).
 constexpr int kDirectWarps = 4;
+constexpr int64_t kDirectTargets = 1LL << 27;
 
 template <class T, int D>
-__global__ void __launch_bounds__(kDirectWarps * 32, sizeof(T) == 4 ? 10 : 1) k_expand_direct(
+struct ExpandSmem {
+    static constexpr int kRound = 64;
+    static constexpr int kList = kRound + 512;  // an incomplete round, and the hits of the records taken next
+    uint32_t edge[kList];
+    SPt<T, D> q[32];  // the queries (idx: 1-based, cloud-local)
+    long long kb[32];
+    T ir[32];
+    int32_t base[32];
+};
+
+template <class T, int D>
+__global__ void __launch_bounds__(kDirectWarps * 32, sizeof(T) == 4 ? 10 : 4) k_expand_direct(
     int64_t nq, const int32_t* __restrict__ qpos_of, const SPt<T, D>* __restrict__ qpts,
     const SPt<T, D>* __restrict__ tpts, const int64_t* __restrict__ offsets, const int2* __restrict__ recs,
     int64_t rec_cap, const uint16_t* __restrict__ rcount, T inv_r, int32_t* __restrict__ senders,
     int32_t* __restrict__ receivers, T* __restrict__ rdisp, T* __restrict__ rdist, Batch bt) {
     pdl_wait();
     pdl_trigger();
-    const unsigned full = 0xffffffffu;
+    constexpr unsigned full = 0xffffffffu;
+    using Smem = ExpandSmem<T, D>;
+    constexpr int ROUND = Smem::kRound, U = ROUND / 32;
+    __shared__ __align__(16) Smem smem[kDirectWarps];
+    Smem& sm = smem[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    // per warp: (record lane << 5 | bit) of each edge of the current record batch
-    __shared__ uint16_t sedge[kDirectWarps][32 * 32];
-    uint16_t* se = sedge[threadIdx.x >> 5];
     const int64_t i0 = ((int64_t)blockIdx.x * kDirectWarps + (threadIdx.x >> 5)) * 32;
     if (i0 >= nq) return;  // warp-uniform
     const int64_t i = i0 + lane;
@@ -635,20 +690,17 @@ __global__ void __launch_bounds__(kDirectWarps * 32, sizeof(T) == 4 ? 10 : 1) k_
     const int32_t qp = valid ? qpos_of[i] : 0;
     int nr = valid ? rcount[qp] : 0;
     int ne = 0;
-    long long krel = 0;
-    if (valid && nr != kOverflowMark) {
-        const int64_t c0 = offsets[i];
-        ne = (int)(offsets[i + 1] - c0);
-        krel = c0 - K0;
+    long long k0 = 0;
+    const bool over = nr == kOverflowMark;
+    if (valid && !over) {
+        k0 = offsets[i];
+        ne = (int)(offsets[i + 1] - k0);
     } else {
         nr = 0;
     }
-    const SPt<T, D> q = qpts[qp];
-    T r2 = T(0), ir = inv_r;
-    int32_t base = 0;
-    cloud_params<T>(bt, qp, r2, ir, base);
-    const int32_t qi = q.idx - base + 1;
     const bool feat = rdisp != nullptr;  // false: neighbor lists (CSR values) only
+    const bool pairs = ((uintptr_t)rdisp & (2 * sizeof(T) - 1)) == 0;
+    const bool gaps = __any_sync(full, over);  // some query's slots are left out
     const unsigned le = full >> (31 - lane);  // lanes up to this one
     // flat record and edge ranges of the queries
     int rinc = nr, einc = ne;
@@ -662,14 +714,59 @@ __global__ void __launch_bounds__(kDirectWarps * 32, sizeof(T) == 4 ? 10 : 1) k_
         }
     }
     const int rexc = rinc - nr;
-    const long long kb = krel - (einc - ne);  // slot of flat edge f of this query: kb + f
-    const int R = __shfl_sync(full, rinc, 31);
-    int32_t* snd_w = senders + K0;
-    int32_t* rcv_w = receivers + K0;
-    T* dist_w = rdist + K0;
-    T* disp_w = feat ? rdisp + D * K0 : nullptr;
-    int fdone = 0;  // flat edges of the earlier record batches
-    for (int rb = 0; rb < R; rb += 32) {
+    {
+        SPt<T, D> q = qpts[qp];
+        T r2 = T(0), ir = inv_r;
+        int32_t base = 0;
+        cloud_params<T>(bt, qp, r2, ir, base);
+        q.idx = q.idx - base + 1;
+        sm.q[lane] = q;
+        sm.ir[lane] = ir;
+        sm.base[lane] = base;
+        sm.kb[lane] = k0 - (einc - ne);  // slot of flat edge f of this query: kb + f
+    }
+    const int R = __shfl_sync(full, rinc, 31), E = __shfl_sync(full, einc, 31);
+    // List entry b holds flat edge f0 + b.
+    const int head = (int)(K0 & 31);
+    int f0 = -head, cnt = head;
+    // The round at list index `at`: U windows, all target loads before any store.
+    auto write = [&](int at) {
+        SPt<T, D> t[U];
+        int ql[U];
+        bool ok[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int b = at + 32 * u + lane, f = f0 + b;
+            ok[u] = b < cnt && f >= 0 && f < E;  // the last always holds when records and counts agree
+            const uint32_t e = ok[u] ? sm.edge[b] : 0u;
+            ql[u] = (int)(e >> 27);
+            if (ok[u]) t[u] = tpts[e & 0x07ffffffu];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (!ok[u]) continue;
+            const int f = f0 + at + 32 * u + lane;
+            const int64_t k = (gaps ? sm.kb[ql[u]] : K0) + f;
+            int32_t base = 0;
+            T ir = inv_r;
+            if (bt.n_clouds) {
+                base = sm.base[ql[u]];
+                ir = sm.ir[ql[u]];
+            }
+            senders[k] = t[u].idx - base + 1;
+            if (feat) {
+                const SPt<T, D> q = sm.q[ql[u]];
+                T diff[D], disp[D];
+                const T d2 = dist2<T, D>(t[u].x, q.x, diff);
+                receivers[k] = q.idx;
+                rdist[k] = mul_rn(sqrt_rn(d2), ir);
+#pragma unroll
+                for (int d = 0; d < D; ++d) disp[d] = mul_rn(-diff[d], ir);
+                store_column<T, D>(rdisp, k, disp, pairs);
+            }
+        }
+    };
+    for (int rb = 0, take; rb < R; rb += take) {
         // record rho = rb + lane and its query
         // (queries without records set no bit, so the k-th bit belongs to the
         // k-th query lane that reaches into the window)
@@ -689,68 +786,35 @@ __global__ void __launch_bounds__(kDirectWarps * 32, sizeof(T) == 4 ? 10 : 1) k_
             const int a = __shfl_up_sync(full, incl, o);
             if (lane >= o) incl += a;
         }
-        const int excl = incl - c;
-        const int tot = __shfl_sync(full, incl, 31);
-        // each record lane lists its hits at its edges' slots
-        __syncwarp();  // the previous batch's table has been read
-        {
-            unsigned mb = (unsigned)rec.y;
-            for (int k = excl; mb; ++k) {
-                se[k] = (uint16_t)((lane << 5) | (__ffs(mb) - 1));
-                mb &= mb - 1;
-            }
-        }
+        // the records whose hits fit the list (one always does)
+        const bool fits = cnt + incl <= Smem::kList;
+        take = __popc(__ballot_sync(full, fits));
+        // each record lane lists its hits at its edges' places
+        int k = cnt + incl - c;
+        const uint32_t first = (uint32_t)rq << 27 | (uint32_t)rec.x;
+        for (unsigned mb = fits ? (unsigned)rec.y : 0u; mb; mb &= mb - 1, ++k)
+            sm.edge[k] = first + (uint32_t)(__ffs(mb) - 1);
+        cnt += __shfl_sync(full, incl, take - 1);
         __syncwarp();
-        // two windows per round, both gathers in flight before either is written
-        for (int w0 = 0; w0 < tot; w0 += 64) {
-            int32_t tpos[2];
-            long long slot[2];
-            int eqw[2];
-            bool ok[2];
+        int at = 0;
+        for (; cnt - at >= ROUND; at += ROUND) write(at);
+        if (at) {
+            // the incomplete round moves to the front
+            uint32_t e[U];
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int wu = w0 + 32 * u;
-                const int e = wu + lane;
-                const int sv = e < tot ? se[e] : 0;
-                const int ri = sv >> 5;  // this lane's record
-                const int rx = __shfl_sync(full, rec.x, ri);
-                const int eq = __shfl_sync(full, rq, ri);  // this lane's query
-                slot[u] = __shfl_sync(full, kb, eq) + (fdone + wu + lane);
-                const int qend = __shfl_sync(full, einc, eq);  // flat end of the query's edges
-                ok[u] = e < tot && fdone + e < qend;  // the second always holds when records and counts agree
-                tpos[u] = ok[u] ? rx + (sv & 31) : 0;
-                eqw[u] = eq;
+            for (int u = 0; u < U; ++u) {
+                const int b = at + 32 * u + lane;
+                e[u] = b < cnt ? sm.edge[b] : 0u;
             }
-            SPt<T, D> t[2];
+            __syncwarp();
 #pragma unroll
-            for (int u = 0; u < 2; ++u)
-                if (ok[u]) t[u] = tpts[tpos[u]];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int eq = eqw[u];
-                const int32_t bq = __shfl_sync(full, base, eq);
-                if (feat) {
-                    const int32_t qiq = __shfl_sync(full, qi, eq);
-                    const T iv = __shfl_sync(full, ir, eq);
-                    T px[D];
-#pragma unroll
-                    for (int d = 0; d < D; ++d) px[d] = __shfl_sync(full, q.x[d], eq);
-                    if (ok[u]) {
-                        T diff[D];
-                        const T d2 = dist2<T, D>(t[u].x, px, diff);
-                        snd_w[slot[u]] = t[u].idx - bq + 1;
-                        rcv_w[slot[u]] = qiq;
-                        dist_w[slot[u]] = mul_rn(sqrt_rn(d2), iv);
-#pragma unroll
-                        for (int d = 0; d < D; ++d) disp_w[(long long)D * slot[u] + d] = mul_rn(-diff[d], iv);
-                    }
-                } else if (ok[u]) {
-                    snd_w[slot[u]] = t[u].idx - bq + 1;
-                }
-            }
+            for (int u = 0; u < U; ++u) sm.edge[32 * u + lane] = e[u];
+            cnt -= at;
+            f0 += at;
+            __syncwarp();
         }
-        fdone += tot;
     }
+    if (cnt) write(0);
 }
 
 // Fill pass from the records, in original index order.  Warp v writes the
@@ -1179,7 +1243,9 @@ cudaError_t launch_expand_shape(Ctx& ctx, const Tree& q, const Tree& t, T inv_r,
 template <class T, int D, bool FEAT>
 cudaError_t launch_expand(Ctx& ctx, const Tree& q, const Tree& t, T inv_r, int32_t* senders, int32_t* receivers,
                           void* rel_disp, void* rel_dist, int bulk_ok) {
-    switch (ctx.plan_tuning.fill_chunk) {
+    int chunk = ctx.plan_tuning.fill_chunk;
+    if (chunk == 0 && t.n > kDirectTargets) chunk = 64;  // positions too wide for the direct fill's list entries
+    switch (chunk) {
         case 32:
             return launch_expand_shape<T, D, FEAT, 32>(ctx, q, t, inv_r, senders, receivers, rel_disp, rel_dist,
                                                        bulk_ok);
