@@ -141,6 +141,55 @@ struct alignas(4 * sizeof(T)) Term4 {
     T v[4];
 };
 
+// Status bits of the adjoint's checks (word 1 of the status buffer).
+constexpr int kAdjMissingTwin = 1;  // an edge without its mirror: not a self-pair COO
+constexpr int kAdjUngrouped = 2;    // receivers not in ascending order
+constexpr int kAdjBadIndex = 4;     // a sender or receiver outside 1..n
+constexpr int kAdjBadOrder = 8;     // an entry of the processing order outside 1..n
+
+// Each point's segment seg[i] = {first, end} of the edges, written where its
+// run of receivers starts and ends (points without edges keep the zeros the
+// caller put there), and the check that the receivers are in 1..n and
+// ascending.  Four receivers per thread.  Bound by DRAM: 4 bytes per edge in, 8
+// per point out (28.6 M edges of 2M points: 24 us; one binary search of the
+// receivers per point took 69, and 10 to pair the starts).
+constexpr int kSegRun = 4;
+__global__ void __launch_bounds__(256) k_segments(const int32_t* __restrict__ rcv, int64_t m, int64_t n,
+                                                  int2* __restrict__ seg, int* __restrict__ status) {
+    pdl_wait();
+    pdl_trigger();
+    const int64_t k0 = kSegRun * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    if (k0 >= m) return;
+    int32_t v[kSegRun + 2];  // receivers k0 - 1 .. k0 + kSegRun, 0 outside the array
+    if (((uintptr_t)rcv & 15) == 0 && k0 + kSegRun <= m) {
+        const int4 q = *reinterpret_cast<const int4*>(rcv + k0);
+        v[1] = q.x;
+        v[2] = q.y;
+        v[3] = q.z;
+        v[4] = q.w;
+    } else {
+#pragma unroll
+        for (int u = 0; u < kSegRun; ++u) v[u + 1] = k0 + u < m ? rcv[k0 + u] : 0;
+    }
+    v[0] = k0 ? rcv[k0 - 1] : 0;
+    v[kSegRun + 1] = k0 + kSegRun < m ? rcv[k0 + kSegRun] : 0;
+    int bad = 0;
+#pragma unroll
+    for (int u = 0; u < kSegRun; ++u) {
+        const int64_t k = k0 + u;
+        if (k >= m) break;
+        const int32_t i = v[u + 1];
+        if (i < 1 || i > n) {
+            bad |= kAdjBadIndex;
+            continue;
+        }
+        if (i < v[u]) bad |= kAdjUngrouped;
+        if (k == 0 || i != v[u]) seg[i - 1].x = (int32_t)k;
+        if (k + 1 == m || i != v[u + 2]) seg[i - 1].y = (int32_t)(k + 1);
+    }
+    if (bad) atomicOr(status, bad);
+}
+
 // term[e] for every edge (one coalesced pass over the edge arrays, 16 B per
 // edge for float), pass 1 of the searching adjoint.
 template <class T, int D, bool RECOMPUTE>
@@ -158,7 +207,7 @@ __global__ void k_edge_terms(int64_t m, int64_t n, const int32_t* __restrict__ s
     for (int d = 0; d < 4; ++d) o.v[d] = T(0);
     if (RECOMPUTE) {
         const int32_t i = rcv[k] - 1, j = snd[k] - 1;
-        if (i < 0 || i >= n || j < 0 || j >= n) {  // flagged by k_adjoint_twins
+        if (i < 0 || i >= n || j < 0 || j >= n) {  // flagged by k_segments or k_adjoint_twins
             term[k] = o;
             return;
         }
@@ -191,12 +240,6 @@ __global__ void k_seg_pairs(const int64_t* __restrict__ off, int64_t n, int2* __
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) seg[i] = make_int2((int32_t)off[i], (int32_t)off[i + 1]);
 }
-
-// Status bits of the adjoint's checks (word 1 of the status buffer).
-constexpr int kAdjMissingTwin = 1;  // an edge without its mirror: not a self-pair COO
-constexpr int kAdjUngrouped = 2;    // receivers not in ascending order
-constexpr int kAdjBadIndex = 4;     // a sender or receiver outside 1..n
-constexpr int kAdjBadOrder = 8;     // an entry of the processing order outside 1..n
 
 // Checks a COO: receivers (1..n_rcv) ascending, senders in 1..n_snd.
 __global__ void k_check_coo(const int32_t* __restrict__ snd, const int32_t* __restrict__ rcv, int64_t m,
@@ -261,8 +304,7 @@ __device__ __forceinline__ double group_sum(double v) {
 // Index of the entry equal to `key` in snd[lo, hi) (one thread's scan of a
 // segment, in aligned blocks of four entries: one 16-byte load per block when
 // `vec`, the sender array being 16-byte aligned), -1 when absent.  Entries
-// outside [lo, hi) in the first and last block are masked off.  (The adjoint
-// kernel keeps its own form of the scan: measured faster there, slower here.)
+// outside [lo, hi) in the first and last block are masked off.
 __device__ __forceinline__ int32_t find_mirror(const int32_t* __restrict__ snd, int32_t m, bool vec, int32_t lo,
                                                int32_t hi, int32_t key) {
     // unsigned: indices below 2^31, so qa + 4 cannot wrap
@@ -288,58 +330,81 @@ __device__ __forceinline__ int32_t find_mirror(const int32_t* __restrict__ snd, 
     return -1;
 }
 
+// Eight consecutive words in one 32-byte load (p is a multiple of 32).
+__device__ __forceinline__ void load8(const int32_t* p, int32_t* c) {
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]), "=r"(c[7])
+        : "l"(p));
+}
+
+// Index of the entry equal to `key` in the segment [lo, hi) of snd (one
+// thread's scan), -1 when absent: blocks of eight entries from a multiple of
+// eight on, one load each when the array is 32-byte aligned (VEC) and the
+// block lies inside it.  Entries outside the segment are masked off.
+template <bool VEC>
+__device__ __forceinline__ int32_t scan_segment(const int32_t* __restrict__ snd, uint32_t m, uint32_t lo, uint32_t hi,
+                                                int32_t key) {
+    for (uint32_t q = lo & ~7u; q < hi; q += 8) {
+        unsigned eq = 0;
+        if (VEC && q + 8 <= m) {
+            int32_t c[8];
+            load8(snd + q, c);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) eq |= c[u] == key ? 1u << u : 0u;
+        } else {
+#pragma unroll
+            for (uint32_t u = 0; u < 8; ++u)
+                if (q + u < m && snd[q + u] == key) eq |= 1u << u;
+        }
+        if (q < lo) eq &= 0xffu << (lo - q);
+        if (q + 8 > hi) eq &= 0xffu >> (q + 8 - hi);
+        if (eq) return (int32_t)(q + __ffs(eq) - 1);
+    }
+    return -1;
+}
+
 // Pass 2 of the searching adjoint: each edge's mirror found by scanning its
 // sender's segment, term(k) - term(mirror) summed per point.  The term
 // records stream in one coalesced pass (k_edge_terms) before this pass reads
-// them.  `vec`: the sender array is 16-byte aligned, so the scan reads four
-// entries per load.
-template <class T>
+// them; nothing is read through a segment when k_segments found the COO
+// ungrouped or out of range.  Bound by L1 (70%: the scans' blocks, the segments
+// and the mirrors' terms are a line per lane): 28.6 M edges of 2M points in
+// 745 us, 762 with 64-bit index arithmetic, blocks of four entries and the
+// receivers read again.
+template <class T, bool VEC>
 __global__ void __launch_bounds__(kTwinWarps * 32) k_adjoint_twins(
     int64_t n, int64_t m, const int32_t* __restrict__ order, const int2* __restrict__ seg,
-    const int32_t* __restrict__ snd, const int32_t* __restrict__ rcv, const Term4<T>* __restrict__ term, int ndims,
-    bool vec, T* __restrict__ grad, int* __restrict__ status) {
+    const int32_t* __restrict__ snd, const Term4<T>* __restrict__ term, int ndims, T* __restrict__ grad,
+    int* __restrict__ status) {
     pdl_wait();
     pdl_trigger();
     const int lane = threadIdx.x & 31, sub = lane & (kTwinLanes - 1);
     const int64_t w0 = ((int64_t)blockIdx.x * kTwinWarps + (threadIdx.x >> 5)) * kTwinGroups;
-    if (w0 >= n) return;  // warp-uniform
-    int bad = 0, p, k0, ne;
-    twin_point(n, m, order, seg, w0 + lane / kTwinLanes, p, k0, ne, bad);
+    if (w0 >= n || (__ldcg(status) & (kAdjUngrouped | kAdjBadIndex))) return;  // warp-uniform
+    int bad = 0, p = -1;
+    int2 sg = make_int2(0, 0);
+    {
+        const int64_t sl = w0 + lane / kTwinLanes;
+        if (sl < n) {
+            const int64_t pp = order ? (int64_t)order[sl] - 1 : sl;
+            if (pp < 0 || pp >= n) {
+                bad |= kAdjBadOrder;
+            } else {
+                p = (int)pp;
+                sg = seg[p];
+            }
+        }
+    }
     double acc[3] = {0.0, 0.0, 0.0};
-    for (int e = sub; e < ne; e += kTwinLanes) {
-        const int32_t k = k0 + e;
-        const int32_t i1 = p + 1;
+    for (int k = sg.x + sub; k < sg.y; k += kTwinLanes) {
         const int32_t j1 = snd[k];
-        if (rcv[k] != i1) bad |= kAdjUngrouped;
-        const Term4<T> tk = term[k];
-        if (j1 < 1 || j1 > n) {
+        if (j1 < 1 || j1 > (int32_t)n) {
             bad |= kAdjBadIndex;
             continue;
         }
         const int2 sj = seg[j1 - 1];
-        int32_t tw = -1;
-        if (vec) {
-            // aligned blocks of four entries; the last block of the array is
-            // read entry by entry
-            for (int32_t qa = sj.x & ~3; qa < sj.y && tw < 0; qa += 4) {
-                int32_t c[4];
-                if ((int64_t)qa + 3 < m) {
-                    const int4 v = *reinterpret_cast<const int4*>(snd + qa);
-                    c[0] = v.x;
-                    c[1] = v.y;
-                    c[2] = v.z;
-                    c[3] = v.w;
-                } else {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) c[u] = (int64_t)qa + u < m ? snd[qa + u] : 0;
-                }
-#pragma unroll
-                for (int u = 3; u >= 0; --u)
-                    if (c[u] == i1 && (int64_t)qa + u >= sj.x && (int64_t)qa + u < sj.y) tw = qa + u;
-            }
-        } else {
-            tw = find_mirror(snd, (int32_t)m, false, sj.x, sj.y, i1);
-        }
+        const Term4<T> tk = term[k];
+        const int32_t tw = scan_segment<VEC>(snd, (uint32_t)m, (uint32_t)sj.x, (uint32_t)sj.y, p + 1);
         if (tw < 0) {
             bad |= kAdjMissingTwin;
             continue;
@@ -525,26 +590,27 @@ int twins_typed(Ctx& ctx, int64_t n, int64_t m, const int32_t* snd, const int32_
     cudaError_t err;
     const T r = (T)radius;
     const T inv_r = T(1) / r;
-    if ((err = ensure(ctx.droff, (n + 1) * 8)) || (err = ensure(ctx.dstatus, 8)) ||
-        (err = ensure(ctx.dseg, n * 8)) || (err = ensure(ctx.dterm, (size_t)m * sizeof(Term4<T>))))
+    if ((err = ensure(ctx.dstatus, 8)) || (err = ensure(ctx.dseg, n * 8)) ||
+        (err = ensure(ctx.dterm, (size_t)m * sizeof(Term4<T>))))
         return cuda_status(ctx, err, "allocating adjoint scratch");
     const int tb = 256;
     PhaseTimer pt_(ctx, PH_ADJOINT);
     int* status = adjoint_status(ctx);
-    if ((err = cudaMemsetAsync(status, 0, 4, s))) return cuda_status(ctx, err, "status reset");
-    launch_pdl(k_segment_starts, div_up(n + 1, tb), tb, 0, s, rcv, m, n, ctx.droff.as<int64_t>());
-    launch_pdl(k_seg_pairs, div_up(n, tb), tb, 0, s, ctx.droff.as<int64_t>(), n, ctx.dseg.as<int2>());
+    if ((err = cudaMemsetAsync(status, 0, 4, s)) || (err = cudaMemsetAsync(ctx.dseg.p, 0, (size_t)n * 8, s)))
+        return cuda_status(ctx, err, "status reset");
     Term4<T>* term = ctx.dterm.as<Term4<T>>();
+    int2* seg = ctx.dseg.as<int2>();
+    launch_pdl(k_segments, div_up(m, tb * kSegRun), tb, 0, s, rcv, m, n, seg, status);
     if (coords)
         launch_pdl(k_edge_terms<T, D, true>, div_up(m, tb), tb, 0, s, m, n, snd, rcv, nullptr, nullptr,
             (const T*)coords, (const T*)d_disp, (const T*)d_dist, r, inv_r, term);
     else
         launch_pdl(k_edge_terms<T, D, false>, div_up(m, tb), tb, 0, s, m, n, snd, rcv, (const T*)rel_disp,
             (const T*)rel_dist, nullptr, (const T*)d_disp, (const T*)d_dist, r, inv_r, term);
-    const bool vec = ((uintptr_t)snd & 15) == 0;
-    launch_pdl(k_adjoint_twins<T>, (unsigned)div_up(n, kTwinGroups * kTwinWarps), 32 * kTwinWarps, 0, s, n, m, order,
-        ctx.dseg.as<int2>(), snd, rcv, term, D, vec, (T*)grad, status);
-    ctx.kernel_launches += 4;
+    const auto twins = ((uintptr_t)snd & 31) == 0 ? k_adjoint_twins<T, true> : k_adjoint_twins<T, false>;
+    launch_pdl(twins, div_up(n, kTwinGroups * kTwinWarps), 32 * kTwinWarps, 0, s, n, m, order, seg, snd, term, D,
+        (T*)grad, status);
+    ctx.kernel_launches += 3;
     if ((err = cudaGetLastError())) return cuda_status(ctx, err, "adjoint launch");
     return read_status(ctx, flags);
 }
@@ -663,7 +729,6 @@ int mirror_typed(Ctx& ctx, int64_t n, int64_t m, const int32_t* snd, const int32
     launch_pdl(k_segment_starts, div_up(n + 1, tb), tb, 0, s, rcv, m, n, ctx.droff.as<int64_t>());
     launch_pdl(k_seg_pairs, div_up(n, tb), tb, 0, s, ctx.droff.as<int64_t>(), n, ctx.dseg.as<int2>());
     const unsigned blocks = (unsigned)div_up(n, kTwinGroups * kTwinWarps);
-    const bool vec = ((uintptr_t)snd & 15) == 0;
     if (coords)
         launch_pdl(k_adjoint_mirror<T, D, true>, blocks, 32 * kTwinWarps, 0, s, n, m, order, ctx.dseg.as<int2>(), snd,
             rcv, mirror, nullptr, nullptr, (const T*)coords, (const T*)d_disp, (const T*)d_dist, r, inv_r, (T*)grad,
