@@ -556,16 +556,38 @@ __global__ void __launch_bounds__(kThreads) k_emit_nodes(const K* __restrict__ s
 // starting at visiting position p (kPiece set for a piece), else 0; a run's
 // box and dstart index go to rbox at the run's first leaf's node, dnode[p].
 //
-// A team of eight lanes per internal node handles its leaf children one after
-// another, eight points per load; the unit, the runs and the box of a node
-// whose children are all leaves are found once per node.  Warps take nodes
-// ids in strides (ids are level-major, so the internal nodes are
-// clustered).  Bounded below by 32n bytes read and written; bound by the
-// latency of a node's dependent loads.
+// A warp collects the internal nodes among the ids it scans in a queue and
+// reads what it needs of up to 32 of them at once, one per lane: their unit,
+// set and children.  Four teams of eight lanes then take a node each: its leaf
+// children's points, eight per round and child, four children's loads in
+// flight, folded so that each lane ends with the box of one child, from which
+// the runs and the node's own box follow by shuffles.  Bounded below by 32n
+// bytes read and written; bound by the latency of a node's dependent loads at
+// 16 warps per SM (long scoreboard 60% of the stalls, issue 28%; the loads of
+// the points to L2 ahead of time gained nothing).  16M uniform points: 222 us,
+// where teams that picked their own nodes and took one child after another
+// took 279; 1M lattice points 17 (32), 5.2M points in 512 clouds 65 (87), 2M
+// uniform points 44 (50), 8000 points 10 (14).  Eight children at once spill
+// (Float32: 241 us at 16M); three blocks per SM, which spill too, 259.
 constexpr int kTeam = 8;
-// points per lane in flight (float: 32 per team, a whole leaf of at most 32)
+constexpr int kTeamChildren = 4;  // children folded at once
+constexpr int kTeamRounds = 4;    // rounds of eight points; more of a larger leaf follow alone
+// points per lane in flight in a larger leaf's rest
 template <class T> constexpr int kTeamPtsOf = sizeof(T) == 4 ? 4 : 2;
+constexpr int kLayoutBlocks = 2;  // blocks per SM
+// A warp takes up to kPickRounds x 32 ids at a time, in clusters of eight ids
+// (a 128-byte line of links) when it has several rounds to come: level-major
+// ids hold their internal nodes in runs, which smaller clusters spread.
+constexpr int kPickRounds = 4;
+constexpr int kClusterShift = 3;
+// One wave of warps, or more when each still gets kWarpNodes ids: with fewer
+// the teams stay half empty (2D points of 1M in a mixture: 44 us, 52 with two
+// waves), with more the device waits for the slowest warp (the 512 clouds: 65
+// us, 84 in one wave).
+constexpr int kLayoutWave = 148 * kLayoutBlocks;
+constexpr int kWarpNodes = 64;
 constexpr int kPiece = 0x80;
+constexpr int kAscending = 1 << 17;  // beside kLinkFull: the node's points are visited in ascending order
 
 // This warp's next internal node (or any node of `todo`) for each team, -1 when none is left.
 __device__ __forceinline__ int32_t team_pick(unsigned& todo, int32_t id) {
@@ -594,6 +616,34 @@ __device__ __forceinline__ void team_fold(unsigned mask, typename OrdKey<T>::I* 
     }
 }
 
+// Boxes of four children, every lane of a team holding its part of each: lane
+// `sub` ends with the box of child sub % 4.  After one butterfly step the lanes
+// exchange halves of what they still hold, so the four boxes take 7 shuffles
+// per value where a butterfly for each would take 12.
+template <class T>
+__device__ __forceinline__ void fold_children(typename OrdKey<T>::I (&lo)[kTeamChildren],
+                                              typename OrdKey<T>::I (&hi)[kTeamChildren]) {
+    constexpr unsigned FULL = 0xffffffffu;
+    using I = typename OrdKey<T>::I;
+    const int sub = threadIdx.x & (kTeam - 1);
+#pragma unroll
+    for (int c = 0; c < kTeamChildren; ++c) {
+        lo[c] = min(lo[c], __shfl_xor_sync(FULL, lo[c], kTeamChildren));
+        hi[c] = max(hi[c], __shfl_xor_sync(FULL, hi[c], kTeamChildren));
+    }
+#pragma unroll
+    for (int o = kTeamChildren / 2; o > 0; o >>= 1) {
+        const bool up = sub & o;
+#pragma unroll
+        for (int c = 0; c < o; ++c) {
+            const I gl = up ? lo[c] : lo[c + o], gh = up ? hi[c] : hi[c + o];
+            const I kl = up ? lo[c + o] : lo[c], kh = up ? hi[c + o] : hi[c];
+            lo[c] = min(kl, __shfl_xor_sync(FULL, gl, o));
+            hi[c] = max(kh, __shfl_xor_sync(FULL, gh, o));
+        }
+    }
+}
+
 template <class T, int D>
 __device__ __forceinline__ void store_bounds(TNode<T, D>* nd, const typename OrdKey<T>::I* lo,
                                              const typename OrdKey<T>::I* hi) {
@@ -605,7 +655,7 @@ __device__ __forceinline__ void store_bounds(TNode<T, D>* nd, const typename Ord
 }
 
 template <class T, int D>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1) k_layout(int64_t capacity, int64_t n, TNode<T, D>* __restrict__ tnode,
+__global__ void __launch_bounds__(kThreads, kLayoutBlocks) k_layout(int64_t capacity, int64_t n, TNode<T, D>* __restrict__ tnode,
                                                      const int2* __restrict__ nrange,
                                                      const NodeLink* __restrict__ link,
                                                      const SPt<T, D>* __restrict__ spts, SPt<T, D>* __restrict__ dpts,
@@ -619,28 +669,101 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1) k_layout(int
     using I = typename K::I;
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int kTeamPts = kTeamPtsOf<T>;
+    constexpr int NCH = Dims<D>::nch;
+    constexpr int G = kTeamChildren;
     const int64_t nn = hdr->n_nodes;
     // After a sort whose wait ran out the ranges mean nothing (the build fails).
     if (nn > capacity || (hdr->status & DF_TIMEOUT)) return;
     const int32_t asc_min = 0x7fffffff - hdr->asc_key;  // no node above (before) this id is scanned ascending
-    const int lane = threadIdx.x & 31, sub = lane & (kTeam - 1);
+    const int lane = threadIdx.x & 31, sub = lane & (kTeam - 1), w = threadIdx.x >> 5;
     const unsigned team = 0xffu << (lane & ~(kTeam - 1));
-    const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
-    const int64_t warp = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-    for (int64_t base = warp; base < nn; base += warps * 32) {
-        const int64_t id = base + warps * lane;
-        bool work = false;  // internal nodes, and roots that are leaves
-        if (id < nn) work = tnode[id].b <= 0 || (bt.n_clouds ? link[id].parent < 0 : id == 0);
-        unsigned todo = __ballot_sync(0xffffffffu, work);
-        while (todo) {
+    const int64_t warps = min((int64_t)gridDim.x * (kThreads / 32), max((int64_t)kLayoutWave * (kThreads / 32), nn / kWarpNodes));
+    // Nodes are taken in clusters of 2^csh ids, a warp's clusters `warps` apart.
+    const int csh = nn >= warps * (32 * kPickRounds) ? kClusterShift : 0;
+    int64_t next = (int64_t)blockIdx.x * (kThreads / 32) + w;
+    if (next >= warps) return;  // warp-uniform
+    __shared__ int32_t queue[kThreads / 32][32 * (kPickRounds + 1)];
+    int head = 0, queued = 0;
+    while (true) {
+        if (queued < 32 && (next << csh) < nn) {
+            __syncwarp();
+            const int32_t rest = queue[w][min(head + lane, 32 * kPickRounds + 31)];
+            __syncwarp();
+            if (lane < queued) queue[w][lane] = rest;
+            head = 0;
+            do {
+                bool work[kPickRounds];  // internal nodes, and roots that are leaves
+                int32_t ids[kPickRounds];
+#pragma unroll
+                for (int r = 0; r < kPickRounds; ++r) {
+                    const int64_t id = ((next + ((lane >> csh) + r * (int64_t)(32 >> csh)) * warps) << csh) +
+                                       (lane & ((1 << csh) - 1));
+                    work[r] = false;
+                    ids[r] = (int32_t)id;
+                    if (id < nn) {
+                        const NodeLink lk = link[id];
+                        work[r] = (lk.meta & 0xff) != 0 || lk.parent < 0;
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < kPickRounds; ++r) {
+                    const unsigned m = __ballot_sync(FULL, work[r]);
+                    if (work[r]) queue[w][queued + __popc(m & ((1u << lane) - 1))] = ids[r];
+                    queued += __popc(m);
+                }
+                next += (int64_t)(kPickRounds * 32 >> csh) * warps;
+            } while (queued < 32 && (next << csh) < nn);
+            __syncwarp();
+        }
+        if (queued == 0) break;
+        const int take = min(queued, 32);
+        // One node per lane: its first child (a leaf root is its own), its
+        // children (0: a leaf root), whether its bounds are the set's, its
+        // unit's direction and the shift to visiting positions.
+        int32_t node = -1, first = 0, meta = 0, to = 0;
+        if (lane < take) {
+            node = queue[w][head + lane];
+            const NodeLink lk = link[node];
+            const int2 range = nrange[node];
+            meta = lk.meta & (kLinkFull | 0xff);
+            first = meta & 0xff ? lk.first : node;
+            // the children on their way to L2
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(tnode + first));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(tnode + first + max((meta & 0xff) - 1, 0)));
+            int32_t c0 = 0, c1 = (int32_t)n;
+            if (bt.n_clouds) {
+                const int c = cloud_of_position(bt, range.x);
+                c0 = (int32_t)bt.coff[c];
+                c1 = (int32_t)bt.coff[c + 1];
+            }
+            to = (int32_t)((uint32_t)c0 + (uint32_t)c1);
+            if ((lk.meta & 0xff) > (lk.meta >> 8 & 0xff)) {  // (some child is a leaf)
+                NodeLink ul = lk;
+                for (int32_t u = node; u >= asc_min; u = ul.parent, ul = link[max(u, 0)]) {
+                    if (!((unsigned)(-tnode[u].b) & 1u)) {
+                        const int2 ur = nrange[u];
+                        to = c0 + (c1 - (ur.y + 1)) - ur.x;
+                        meta |= kAscending;
+                    }
+                }
+            }
+        }
+        head += take;
+        queued -= take;
+        for (int k = 0; k < take; k += 32 / kTeam) {
             // The warp's four teams run in step (every shuffle is warp-wide, a
             // team without a node idles): a team of its own mask would execute
             // alone.
-            const int32_t q = team_pick(todo, (int32_t)id);
-            const int32_t qa = q >= 0 ? tnode[q].a : 0, qb = q >= 0 ? tnode[q].b : 0;
-            const bool internal = qb < 0;
-            const int nc = q < 0 ? 0 : internal ? __popc((unsigned)(-qb)) : 1;
-            const int32_t ch0 = internal ? qa : q;  // first child's id (a leaf root is its own)
+            const int src = k + lane / kTeam;
+            const int ms = __shfl_sync(FULL, meta, src & 31);
+            const int32_t q = __shfl_sync(FULL, node, src & 31), ch0 = __shfl_sync(FULL, first, src & 31);
+            const int32_t shift = __shfl_sync(FULL, to, src & 31);
+            const bool internal = src < take && (ms & 0xff) != 0, asc = ms & kAscending;
+            const int nc = src >= take ? 0 : internal ? ms & 0xff : 1;
+            // the visiting position of the child's point at sorted position a is place(a, b) + its rank
+            auto place = [&](int32_t a, int32_t b) {
+                return asc ? a + shift : (int32_t)((uint32_t)shift - (uint32_t)a - (uint32_t)b);
+            };
             int32_t ca = 0, cb = 0;
             if (sub < nc) {
                 ca = tnode[ch0 + sub].a;
@@ -648,105 +771,143 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1) k_layout(int
             }
             const unsigned leaf_m = __ballot_sync(FULL, cb > 0), inner_m = __ballot_sync(FULL, sub < nc && cb <= 0);
             if (leaf_m == 0) continue;
-            const int2 rg = q >= 0 ? nrange[q] : make_int2(0, 0);
-            int32_t c0 = 0, c1 = (int32_t)n;
-            if (bt.n_clouds && q >= 0) {
-                const int c = cloud_of_position(bt, rg.x);
-                c0 = (int32_t)bt.coff[c];
-                c1 = (int32_t)bt.coff[c + 1];
+            // The children's points, copied and folded: the first kTeamRounds
+            // rounds take eight points of each of G children, all loads in
+            // flight; lane `sub` gets the box of child `sub`.
+            cb = max(cb, 0);  // 0: no leaf here
+            const int bw = __reduce_max_sync(FULL, cb);
+            I lo[D], hi[D];
+#pragma unroll
+            for (int h = 0; h < NCH; h += G) {
+                int32_t a[G], b[G];
+                I gl[D][G], gh[D][G];
+#pragma unroll
+                for (int c = 0; c < G; ++c) {
+                    a[c] = __shfl_sync(FULL, ca, h + c, kTeam);
+                    b[c] = __shfl_sync(FULL, cb, h + c, kTeam);
+#pragma unroll
+                    for (int d = 0; d < D; ++d) { gl[d][c] = K::kMaxKey; gh[d][c] = K::kMinKey; }
+                }
+                for (int32_t m = sub; m - sub < min(bw, kTeam * kTeamRounds); m += kTeam) {
+                    SPt<T, D> p[G];
+#pragma unroll
+                    for (int c = 0; c < G; ++c)
+                        if (m < b[c]) p[c] = spts[a[c] + m];
+#pragma unroll
+                    for (int c = 0; c < G; ++c) {
+                        if (m < b[c]) {
+                            dpts[place(a[c], b[c]) + m] = p[c];
+#pragma unroll
+                            for (int d = 0; d < D; ++d) {
+                                const I k = K::key(K::bits(p[c].x[d]));
+                                gl[d][c] = min(gl[d][c], k);
+                                gh[d][c] = max(gh[d][c], k);
+                            }
+                        }
+                    }
+                }
+                __syncwarp();
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    fold_children<T>(gl[d], gh[d]);
+                    if (h == 0 || sub >= h) { lo[d] = gl[d][0]; hi[d] = gh[d][0]; }
+                }
             }
-            bool asc = false;
-            int32_t up_shift = 0;  // the shift of an ascending unit
-            if (internal && (leaf_m & team)) {
-                for (int32_t u = q; u >= asc_min; u = link[u].parent) {
-                    if (!((unsigned)(-tnode[u].b) & 1u)) {
-                        const int2 ur = nrange[u];
-                        up_shift = c0 + (c1 - (ur.y + 1)) - ur.x;
-                        asc = true;
+            if (bw > kTeam * kTeamRounds) {  // the rest of larger leaves, one child after another
+                for (int j = 0; j < NCH; ++j) {
+                    const int32_t a = __shfl_sync(FULL, ca, j, kTeam), b = __shfl_sync(FULL, cb, j, kTeam);
+                    const int32_t at = place(a, b);
+                    I rl[D], rh[D];
+#pragma unroll
+                    for (int d = 0; d < D; ++d) { rl[d] = K::kMaxKey; rh[d] = K::kMinKey; }
+                    const int32_t bj = __reduce_max_sync(FULL, b);
+                    if (bj <= kTeam * kTeamRounds) continue;
+                    for (int32_t m = kTeam * kTeamRounds + sub; m - sub < bj; m += kTeamPts * kTeam) {
+                        SPt<T, D> p[kTeamPts];
+#pragma unroll
+                        for (int t = 0; t < kTeamPts; ++t)
+                            if (m + t * kTeam < b) p[t] = spts[a + m + t * kTeam];
+#pragma unroll
+                        for (int t = 0; t < kTeamPts; ++t) {
+                            if (m + t * kTeam < b) {
+                                dpts[at + m + t * kTeam] = p[t];
+#pragma unroll
+                                for (int d = 0; d < D; ++d) {
+                                    const I k = K::key(K::bits(p[t].x[d]));
+                                    rl[d] = min(rl[d], k);
+                                    rh[d] = max(rh[d], k);
+                                }
+                            }
+                        }
+                    }
+                    __syncwarp();
+                    team_fold<T, D>(FULL, rl, rh);
+                    if (sub == j) {
+#pragma unroll
+                        for (int d = 0; d < D; ++d) { lo[d] = min(lo[d], rl[d]); hi[d] = max(hi[d], rh[d]); }
                     }
                 }
             }
-            // (the children's points lie between the node's first and last: on their way to L2 at once)
-            if ((leaf_m & team) && rg.y - rg.x < 1024)
-                for (int32_t p = rg.x + 8 * sub; p <= rg.y; p += 8 * kTeam)
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(spts + p));
-            I nlo[D], nhi[D], rlo[D], rhi[D];  // boxes of the node and of the open run
-            auto clear = [](I* lo, I* hi) {
+            if (cb > 0) store_bounds<T, D>(tnode + ch0 + sub, lo, hi);
+            if (sub >= nc || cb == 0) {
 #pragma unroll
                 for (int d = 0; d < D; ++d) { lo[d] = K::kMaxKey; hi[d] = K::kMinKey; }
-            };
-            clear(nlo, nhi);
-            clear(rlo, rhi);
-            int32_t run_first = 0, run_count = 0, run_id = 0;
-            auto close = [&]() {
-                if (run_count && sub == 0) {
+            }
+            // Runs: bit j of `start`: child j opens one, of `cut`: child j opens one or is in none.
+            unsigned start = 0, cut = 0;
+            {
+                int count = 0;
+#pragma unroll
+                for (int j = 0; j < NCH; ++j) {
+                    const int32_t b = __shfl_sync(FULL, cb, j, kTeam);
+                    const bool in = b > 0 && b <= gmax;
+                    const bool opens = in && (count == 0 || count + b > gmax);
+                    count = !in ? 0 : opens ? b : count + b;
+                    start |= opens ? 1u << j : 0u;
+                    cut |= opens || !in ? 1u << j : 0u;
+                }
+                cut |= ~0u << NCH;
+            }
+            {
+                // the run's last child after `sub`, the run's box at its first child
+                const int len = __ffs(cut >> (sub + 1));  // children from here to the run's end
+                I rlo[D], rhi[D];
+#pragma unroll
+                for (int d = 0; d < D; ++d) { rlo[d] = lo[d]; rhi[d] = hi[d]; }
+#pragma unroll
+                for (int o = 1; o < NCH; o <<= 1) {
+#pragma unroll
+                    for (int d = 0; d < D; ++d) {
+                        const I vl = __shfl_down_sync(FULL, rlo[d], o, kTeam), vh = __shfl_down_sync(FULL, rhi[d], o, kTeam);
+                        if (o < len) { rlo[d] = min(rlo[d], vl); rhi[d] = max(rhi[d], vh); }
+                    }
+                }
+                const int32_t run_end = __shfl_sync(FULL, ca + cb, (sub + len - 1) & (kTeam - 1), kTeam);
+                if (start >> sub & 1u) {
                     // outside an ascending unit the run's last leaf is visited first
-                    const int32_t p = asc ? run_first + up_shift : c0 + (c1 - (run_first + run_count));
-                    dstart[p] = (uint8_t)run_count;
-                    dnode[p] = run_id;
+                    const int32_t pos = place(ca, run_end - ca);
+                    dstart[pos] = (uint8_t)(run_end - ca);
+                    dnode[pos] = ch0 + sub;
                     TNode<float, D> nd;
 #pragma unroll
                     for (int d = 0; d < D; ++d) {
                         nd.lo[d] = float_below(K::value(rlo[d]));
                         nd.hi[d] = float_above(K::value(rhi[d]));
                     }
-                    nd.a = p;
-                    nd.b = run_count;
-                    rbox[run_id] = nd;
+                    nd.a = pos;
+                    nd.b = run_end - ca;
+                    rbox[ch0 + sub] = nd;
                 }
-                run_count = 0;
-                clear(rlo, rhi);
-            };
-            __syncwarp();
-            const int ncw = __reduce_max_sync(FULL, nc);
-            for (int j = 0; j < ncw; ++j) {
-                const int32_t a = __shfl_sync(FULL, ca, j, kTeam);
-                const int32_t b = max(__shfl_sync(FULL, cb, j, kTeam), 0);  // 0: no leaf here
-                const int bw = __reduce_max_sync(FULL, b);
-                const int32_t shift = asc ? up_shift : c0 + (c1 - (a + b)) - a;
-                I lo[D], hi[D];
-                clear(lo, hi);
-                for (int32_t m = sub; m - sub < bw; m += kTeamPts * kTeam) {
-                    SPt<T, D> p[kTeamPts];
-#pragma unroll
-                    for (int t = 0; t < kTeamPts; ++t)
-                        if (m + t * kTeam < b) p[t] = spts[a + m + t * kTeam];
-#pragma unroll
-                    for (int t = 0; t < kTeamPts; ++t) {
-                        if (m + t * kTeam < b) {
-                            dpts[a + m + t * kTeam + shift] = p[t];
-#pragma unroll
-                            for (int d = 0; d < D; ++d) {
-                                const I k = K::key(K::bits(p[t].x[d]));
-                                lo[d] = min(lo[d], k);
-                                hi[d] = max(hi[d], k);
-                            }
-                        }
-                    }
-                }
-                __syncwarp();
-                team_fold<T, D>(FULL, lo, hi);
-                if (b > 0 && sub == 0) store_bounds<T, D>(tnode + ch0 + j, lo, hi);
-                if (b == 0 || b > gmax || run_count + b > gmax) close();  // (an internal child ends the run too)
-                if (b > gmax) {
-                    for (int32_t c = sub * gmax; c < b; c += kTeam * gmax)
-                        dstart[a + c + shift] = (uint8_t)(kPiece | min(gmax, b - c));
-                } else if (b > 0) {
-                    if (run_count == 0) {
-                        run_first = a;
-                        run_id = ch0 + j;
-                    }
-                    run_count += b;
-#pragma unroll
-                    for (int d = 0; d < D; ++d) { rlo[d] = min(rlo[d], lo[d]); rhi[d] = max(rhi[d], hi[d]); }
-                }
-#pragma unroll
-                for (int d = 0; d < D; ++d) { nlo[d] = min(nlo[d], lo[d]); nhi[d] = max(nhi[d], hi[d]); }
             }
-            close();
+            if (cb > gmax) {  // pieces of a larger leaf
+                const int32_t at = place(ca, cb);
+                for (int32_t c = 0; c < cb; c += gmax) dstart[at + c] = (uint8_t)(kPiece | min(gmax, cb - c));
+            }
+            __syncwarp();
+            team_fold<T, D>(FULL, lo, hi);
             // (a node covering its whole set already has that set's bounds)
-            if (internal && (inner_m & team) == 0 && sub == 0 && !(rg.x == c0 && rg.y == c1 - 1))
-                store_bounds<T, D>(tnode + q, nlo, nhi);
+            if (internal && (inner_m & team) == 0 && sub == 0 && !(ms & kLinkFull))
+                store_bounds<T, D>(tnode + q, lo, hi);
             __syncwarp();
         }
     }
@@ -1356,7 +1517,7 @@ void launch_layout(Ctx& ctx, Tree& t, int64_t n, int64_t node_cap, int64_t chunk
     {
         PhaseTimer pt_(ctx, PH_REFIT);
         // a grid that fills the device; warps take further nodes in turn
-        const int64_t blocks = std::min<int64_t>(div_up(nodes, kThreads), 148 * 8);
+        const int64_t blocks = std::min<int64_t>(div_up(nodes, kThreads), 2 * kLayoutWave);
         launch_pdl(k_layout<T, D>, blocks, kThreads, 0, ctx.stream, node_cap, n, t.tnode.as<TNode<T, D>>(),
             t.nrange.as<int2>(), t.link.as<NodeLink>(), t.spts.as<SPt<T, D>>(), t.dpts.as<SPt<T, D>>(),
             t.dstart.as<uint8_t>(), t.dnode.as<int32_t>(), t.rbox.as<TNode<float, D>>(), gmax, hdr, t.batch());
