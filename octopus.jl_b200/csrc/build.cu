@@ -1130,35 +1130,53 @@ __global__ void k_view_morton(const SPt<T, D>* __restrict__ spts, const K* __res
 }
 
 // --------------------------------------------------------- 9. batches ----
-// Per-cloud min/max (Julia order) and non-finite flag, one block per cloud:
-// out[c*8 + 0..2] = min, [3..5] = max, [6] = non-finite.
+// Per-cloud min/max (Julia order) and non-finite flag: out[c*8 + 0..2] = min,
+// [3..5] = max, [6] = non-finite.  One block per cloud, kCloudLoads points per
+// thread in flight, folded as order keys.  Bound by the latency of the largest
+// cloud's loads (5.2M points in 512 clouds of up to 20,000: 21 us; one point
+// per thread of 256 at a time, folded as floats, took 67).
+constexpr int kCloudThreads = 512;
+constexpr int kCloudLoads = 8;
 template <class T, int D>
-__global__ void __launch_bounds__(kThreads) k_cloud_bounds(const T* __restrict__ coords, const int64_t* __restrict__ coff,
-                                                           double* __restrict__ out) {
-    __shared__ T smin[kThreads / 32][D], smax[kThreads / 32][D];
+__global__ void __launch_bounds__(kCloudThreads) k_cloud_bounds(const T* __restrict__ coords,
+                                                                const int64_t* __restrict__ coff,
+                                                                double* __restrict__ out) {
+    using K = OrdKey<T>;
+    using I = typename K::I;
+    __shared__ I smin[kCloudThreads / 32][D], smax[kCloudThreads / 32][D];
     __shared__ int snan;
     const int c = blockIdx.x;
     const int64_t s0 = coff[c], s1 = coff[c + 1];
     if (threadIdx.x == 0) snan = 0;
     __syncthreads();
-    T lo[D], hi[D];
+    I lo[D], hi[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) { lo[d] = T(INFINITY); hi[d] = T(-INFINITY); }
-    int bad = 0;
-    for (int64_t i = s0 + threadIdx.x; i < s1; i += blockDim.x) {
+    for (int d = 0; d < D; ++d) { lo[d] = K::kMaxKey; hi[d] = K::kMinKey; }
+    bool bad = false;
+    for (int64_t i0 = s0 + threadIdx.x; i0 < s1; i0 += kCloudLoads * kCloudThreads) {
+        T x[kCloudLoads][D];
 #pragma unroll
-        for (int d = 0; d < D; ++d) {
-            const T x = coords[D * i + d];
-            if (!isfinite(x)) bad = 1;
-            lo[d] = jl_min(lo[d], x);
-            hi[d] = jl_max(hi[d], x);
+        for (int u = 0; u < kCloudLoads; ++u) {
+            const int64_t i = min(i0 + u * kCloudThreads, s1 - 1);  // (the last point again beyond the end)
+#pragma unroll
+            for (int d = 0; d < D; ++d) x[u][d] = coords[D * i + d];
+        }
+#pragma unroll
+        for (int u = 0; u < kCloudLoads; ++u) {
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                bad |= !isfinite(x[u][d]);
+                const I k = K::key(K::bits(x[u][d]));
+                lo[d] = min(lo[d], k);
+                hi[d] = max(hi[d], k);
+            }
         }
     }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-        lo[d] = warp_min(lo[d]);
-        hi[d] = warp_max(hi[d]);
+        lo[d] = ord_warp_min(lo[d]);
+        hi[d] = ord_warp_max(hi[d]);
     }
     if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&snan, 1);
     if (lane == 0) {
@@ -1166,15 +1184,17 @@ __global__ void __launch_bounds__(kThreads) k_cloud_bounds(const T* __restrict__
         for (int d = 0; d < D; ++d) { smin[w][d] = lo[d]; smax[w][d] = hi[d]; }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w2 = 1; w2 < kThreads / 32; ++w2)
-            for (int d = 0; d < D; ++d) {
-                smin[0][d] = jl_min(smin[0][d], smin[w2][d]);
-                smax[0][d] = jl_max(smax[0][d], smax[w2][d]);
-            }
+    if (threadIdx.x < D) {
+        const int d = threadIdx.x;
+        I l = smin[0][d], h = smax[0][d];
+        for (int v = 1; v < kCloudThreads / 32; ++v) {
+            l = min(l, smin[v][d]);
+            h = max(h, smax[v][d]);
+        }
         double* p = out + (size_t)c * 8;
-        for (int d = 0; d < D; ++d) { p[d] = (double)smin[0][d]; p[3 + d] = (double)smax[0][d]; }
-        p[6] = snan ? 1.0 : 0.0;
+        p[d] = (double)K::value(l);
+        p[3 + d] = (double)K::value(h);
+        if (d == 0) p[6] = snan ? 1.0 : 0.0;
     }
 }
 
@@ -1911,7 +1931,7 @@ int build_batch_typed(Ctx& ctx, Tree& t, const T* coords, int64_t n, const int64
         return cuda_status(ctx, err, "batch upload");
     {
         PhaseTimer pt_(ctx, PH_BOUNDS);
-        k_cloud_bounds<T, D><<<nc, kThreads, 0, s>>>(coords, t.b_coff.as<int64_t>(), t.b_cbounds.as<double>());
+        k_cloud_bounds<T, D><<<nc, kCloudThreads, 0, s>>>(coords, t.b_coff.as<int64_t>(), t.b_cbounds.as<double>());
         ctx.kernel_launches += 1;
     }
     std::vector<double> cb((size_t)nc * 8);

@@ -61,6 +61,31 @@ __device__ __forceinline__ uint32_t spread2_32(uint32_t x) {
 __device__ __forceinline__ int cell_i32(float v) { return max(__float2int_rd(v), 0); }
 __device__ __forceinline__ int cell_i32(double v) { return max(__double2int_rd(v), 0); }
 
+// Origin, inverse cell size and id of the cloud a thread's points are in
+// (without a batch: of the point set), looked up when a point lies outside the
+// one before.  A thread's points are in input order and a few hundred apart at
+// most, so a search per thread serves nearly all of them (5.2M points in 512
+// clouds: counts and first pass 87 us, 112 with a search per point).
+template <class T>
+struct CloudCursor {
+    T o[3];
+    T inv_cs;
+    int32_t begin = 0, end = 0;  // its positions; none before the first look-up
+    int32_t cloud = 0;
+    __device__ __forceinline__ explicit CloudCursor(const EncodeParams<T>& ep)
+        : o{ep.o[0], ep.o[1], ep.o[2]}, inv_cs(ep.inv_cs) {}
+    __device__ __forceinline__ void seek(const Batch& bt, int64_t i) {
+        if (i >= begin && i < end) return;
+        cloud = cloud_of_position(bt, i);
+        begin = (int32_t)bt.coff[cloud];
+        end = (int32_t)bt.coff[cloud + 1];
+        const double* cp = bt.cparam + (size_t)cloud * kCloudParams;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) o[d] = (T)cp[d];
+        inv_cs = (T)cp[3];
+    }
+};
+
 // Morton key of one point's cell (src/cpu/bin_cpu.jl:12-31,
 // src/morton.jl:13-60): floor((x - origin) * inv_cs) per axis, clamped to the
 // key's bits per axis, bit-interleaved with x in the lowest bit; in a batch,
@@ -68,19 +93,12 @@ __device__ __forceinline__ int cell_i32(double v) { return max(__double2int_rd(v
 // A 32-bit key K means that the host found every cell index below 2^10 (3D)
 // or 2^16 (2D), so the interleave runs on 32-bit words.
 template <class T, int D, class K>
-__device__ __forceinline__ K point_key(const T* x, int64_t i, const EncodeParams<T>& ep) {
+__device__ __forceinline__ K point_key(const T* x, int64_t i, const EncodeParams<T>& ep, CloudCursor<T>& cur) {
     constexpr int64_t cmax = (1LL << Dims<D>::bits) - 1;
-    T o[3] = {ep.o[0], ep.o[1], ep.o[2]};
-    T inv_cs = ep.inv_cs;
-    int cloud = 0;
-    if (ep.bt.n_clouds) {
-        cloud = cloud_of_position(ep.bt, i);
-        const double* cp = ep.bt.cparam + (size_t)cloud * kCloudParams;
-        o[0] = (T)cp[0];
-        o[1] = (T)cp[1];
-        o[2] = (T)cp[2];
-        inv_cs = (T)cp[3];
-    }
+    if (ep.bt.n_clouds) cur.seek(ep.bt, i);
+    const T* o = cur.o;
+    const T inv_cs = cur.inv_cs;
+    const int cloud = cur.cloud;
     if constexpr (sizeof(K) == 4) {
         uint32_t c[3] = {0, 0, 0};
 #pragma unroll
@@ -114,8 +132,9 @@ __global__ void __launch_bounds__(kSortThreads) k_point_counts(const T* __restri
     for (int p = 0; p < passes; ++p) c[p][threadIdx.x] = 0;
     __syncthreads();
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nthr = (int64_t)gridDim.x * blockDim.x;
+    CloudCursor<T> cur(ep);
     auto take = [&](const T* x, int64_t i) {
-        const K k = point_key<T, D, K>(x, i, ep);
+        const K k = point_key<T, D, K>(x, i, ep, cur);
         for (int p = 0; p < passes; ++p) atomicAdd(&c[p][(unsigned)(k >> (8 * p)) & 255u], 1u);
     };
     int64_t done = 0;  // points counted by the vector loop
@@ -216,6 +235,7 @@ __global__ void __launch_bounds__(kSortThreads) k_point_pass(
     }
     const int lbase = w * (32 * kSortItems);  // this warp's part of the tile
     K key[kSortItems];
+    CloudCursor<T> cur(ep);
     if (FIRST) {
         copy_async_wait();
         __syncthreads();
@@ -225,7 +245,7 @@ __global__ void __launch_bounds__(kSortThreads) k_point_pass(
         const int l = lbase + it * 32 + lane;
         key[it] = K(0);
         if (l < tcnt)
-            key[it] = FIRST ? point_key<T, D, K>(reinterpret_cast<const T*>(sm.pts) + D * l, tbase + l, ep)
+            key[it] = FIRST ? point_key<T, D, K>(reinterpret_cast<const T*>(sm.pts) + D * l, tbase + l, ep, cur)
                             : kin[tbase + l];
     }
     // Rank of each key among the tile's keys of its digit that come before it:
