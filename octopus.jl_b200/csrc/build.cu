@@ -67,129 +67,133 @@ __device__ __forceinline__ long long ord_warp_max(long long v) {
     return v;
 }
 
+// Minima, maxima (Julia order, as order keys) and largest magnitude of a
+// block's values, in every lane of its first warp; `sm` holds a warp's per row.
+template <class T, int D>
+__device__ __forceinline__ void block_bounds(typename OrdKey<T>::I* lo, typename OrdKey<T>::I* hi,
+                                             typename OrdKey<T>::I& mag,
+                                             typename OrdKey<T>::I (*sm)[2 * D + 1]) {
+    using K = OrdKey<T>;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+        lo[d] = ord_warp_min(lo[d]);
+        hi[d] = ord_warp_max(hi[d]);
+    }
+    mag = ord_warp_max(mag);
+    if (lane == 0) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            sm[w][2 * d] = lo[d];
+            sm[w][2 * d + 1] = hi[d];
+        }
+        sm[w][2 * D] = mag;
+    }
+    __syncthreads();
+    if (w == 0) {
+        const bool in = lane < kThreads / 32;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            lo[d] = ord_warp_min(in ? sm[lane][2 * d] : K::kMaxKey);
+            hi[d] = ord_warp_max(in ? sm[lane][2 * d + 1] : K::kMinKey);
+        }
+        mag = ord_warp_max(in ? sm[lane][2 * D] : 0);
+    }
+}
+
 // Per-axis min/max (Julia min/max order) and a non-finite flag.  The last
-// block to finish folds the per-block partials into the header.
+// block to finish folds the per-block partials (rows of eight order keys: D
+// minima, D maxima, the largest magnitude) into the header.  The fold runs on
+// order keys (OrdKey): integer min/max give Julia's min/max of finite values,
+// and a magnitude at or above the exponent mask marks a NaN or Inf (whose
+// bounds then do not matter: the build fails).  Bound by latency up to a
+// million points: the loads, then the two folds, in parallel through redux
+// (1000 points 7.5 us, 11.4 with one thread folding the warps' floats; 1M
+// lattice points 13, 17; 1M 2D points and 200,003 Float64 points, which read
+// one value per load before, 11.4 and 13.3, 17.5 and 19.3).
 template <class T, int D>
 __global__ void __launch_bounds__(kThreads) k_bounds(const T* __restrict__ coords, int64_t n,
-                                                     double* __restrict__ partials, OctHeader* hdr) {
+                                                     typename OrdKey<T>::I* __restrict__ partials, OctHeader* hdr) {
     pdl_wait();
     pdl_trigger();
-    __shared__ T smin[kThreads / 32][D], smax[kThreads / 32][D];
-    __shared__ int snan;
+    using K = OrdKey<T>;
+    using I = typename K::I;
+    __shared__ I sm[kThreads / 32][2 * D + 1];
     __shared__ bool is_last;
-    if (threadIdx.x == 0) snan = 0;
-    __syncthreads();
-    // The fold runs on order keys (OrdKey): integer min/max give Julia's
-    // min/max of finite values, and a magnitude at or above the exponent
-    // mask marks a NaN or Inf (whose bounds then do not matter: the build
-    // fails).
-    using I = typename OrdKey<T>::I;
-    I klo[D], khi[D], mag = 0;
+    I lo[D], hi[D], mag = 0;
 #pragma unroll
-    for (int d = 0; d < D; ++d) { klo[d] = OrdKey<T>::kMaxKey; khi[d] = OrdKey<T>::kMinKey; }
+    for (int d = 0; d < D; ++d) { lo[d] = K::kMaxKey; hi[d] = K::kMinKey; }
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nthr = (int64_t)gridDim.x * blockDim.x;
     auto take = [&](int d, T x) {
-        const I b = OrdKey<T>::bits(x);
-        const I k = OrdKey<T>::key(b);
-        klo[d] = min(klo[d], k);
-        khi[d] = max(khi[d], k);
-        mag = max(mag, b & OrdKey<T>::kMag);
+        const I b = K::bits(x);
+        const I k = K::key(b);
+        lo[d] = min(lo[d], k);
+        hi[d] = max(hi[d], k);
+        mag = max(mag, b & K::kMag);
     };
     int64_t done = 0;  // points folded by the vector loop
-    if constexpr (std::is_same<T, float>::value && D == 3) {
-        if (((uintptr_t)coords & 15) == 0) {
-            // Four points = 12 floats = three float4 (axes x y z x | y z x y | z x y z),
-            // two groups of four points in flight per thread.
-            const float4* v = reinterpret_cast<const float4*>(coords);
-            const int64_t groups = n / 4;
-            for (int64_t g = tid; g < groups; g += 2 * nthr) {
-                const int64_t g2 = g + nthr;
-                const float4 a = v[3 * g], b = v[3 * g + 1], c = v[3 * g + 2];
-                float4 a2 = a, b2 = b, c2 = c;
-                if (g2 < groups) {
-                    a2 = v[3 * g2];
-                    b2 = v[3 * g2 + 1];
-                    c2 = v[3 * g2 + 2];
-                }
-                take(0, a.x); take(1, a.y); take(2, a.z); take(0, a.w);
-                take(1, b.x); take(2, b.y); take(0, b.z); take(1, b.w);
-                take(2, c.x); take(0, c.y); take(1, c.z); take(2, c.w);
-                take(0, a2.x); take(1, a2.y); take(2, a2.z); take(0, a2.w);
-                take(1, b2.x); take(2, b2.y); take(0, b2.z); take(1, b2.w);
-                take(2, c2.x); take(0, c2.y); take(1, c2.z); take(2, c2.w);
+    if (((uintptr_t)coords & 15) == 0) {
+        // D words of 16 bytes = E points (their values in order, so an axis
+        // each), kGroups of them in flight per thread.
+        constexpr int E = 16 / (int)sizeof(T), kGroups = D == 3 ? 2 : 3;
+        const uint4* v = reinterpret_cast<const uint4*>(coords);
+        const int64_t groups = n / E;
+        for (int64_t g = tid; g < groups; g += kGroups * nthr) {
+            uint4 q[kGroups][D];
+#pragma unroll
+            for (int u = 0; u < kGroups; ++u) {
+                const int64_t gu = g + u * nthr < groups ? g + u * nthr : g;
+#pragma unroll
+                for (int c = 0; c < D; ++c) q[u][c] = v[D * gu + c];
             }
-            done = groups * 4;
+#pragma unroll
+            for (int u = 0; u < kGroups; ++u) {
+                T x[D * E];
+                memcpy(x, q[u], sizeof(x));
+#pragma unroll
+                for (int c = 0; c < D * E; ++c) take(c % D, x[c]);
+            }
         }
+        done = groups * E;
     }
     for (int64_t i = done + tid; i < n; i += nthr) {
 #pragma unroll
         for (int d = 0; d < D; ++d) take(d, coords[D * i + d]);
     }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    T lo[D], hi[D];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-        lo[d] = OrdKey<T>::value(ord_warp_min(klo[d]));
-        hi[d] = OrdKey<T>::value(ord_warp_max(khi[d]));
-    }
-    const int bad = mag >= OrdKey<T>::kExp;
-    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&snan, 1);
-    if (lane == 0) {
-#pragma unroll
-        for (int d = 0; d < D; ++d) { smin[w][d] = lo[d]; smax[w][d] = hi[d]; }
-    }
-    __syncthreads();
+    block_bounds<T, D>(lo, hi, mag, sm);
     if (threadIdx.x == 0) {
-        for (int w2 = 1; w2 < kThreads / 32; ++w2)
-            for (int d = 0; d < D; ++d) {
-                smin[0][d] = jl_min(smin[0][d], smin[w2][d]);
-                smax[0][d] = jl_max(smax[0][d], smax[w2][d]);
-            }
-        double* p = partials + (size_t)blockIdx.x * 8;
-        for (int d = 0; d < D; ++d) { p[d] = (double)smin[0][d]; p[3 + d] = (double)smax[0][d]; }
-        p[6] = snan ? 1.0 : 0.0;
-        __threadfence();
-        const int ticket = atomicAdd(&hdr->n_blocks_done, 1);
-        is_last = (ticket == (int)gridDim.x - 1);
+        I* p = partials + (size_t)blockIdx.x * 8;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            p[d] = lo[d];
+            p[3 + d] = hi[d];
+        }
+        p[6] = mag;
+        is_last = cuda::atomic_ref<int32_t, cuda::thread_scope_device>(hdr->n_blocks_done)
+                      .fetch_add(1, cuda::memory_order_acq_rel) == (int)gridDim.x - 1;
     }
     __syncthreads();
     if (!is_last) return;
-    // Last block: fold the per-block partials in parallel.
-    __threadfence();
-    T glo[D], ghi[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) { glo[d] = T(INFINITY); ghi[d] = T(-INFINITY); }
-    int anynan = 0;
-    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-        const double* p = partials + (size_t)b * 8;
+    for (int d = 0; d < D; ++d) { lo[d] = K::kMaxKey; hi[d] = K::kMinKey; }
+    mag = 0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += kThreads) {
+        const I* p = partials + (size_t)b * 8;
 #pragma unroll
         for (int d = 0; d < D; ++d) {
-            glo[d] = jl_min(glo[d], (T)__ldcg(p + d));
-            ghi[d] = jl_max(ghi[d], (T)__ldcg(p + 3 + d));
+            lo[d] = min(lo[d], __ldcg(p + d));
+            hi[d] = max(hi[d], __ldcg(p + 3 + d));
         }
-        if (__ldcg(p + 6) != 0.0) anynan = 1;
+        mag = max(mag, __ldcg(p + 6));
     }
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-        glo[d] = warp_min(glo[d]);
-        ghi[d] = warp_max(ghi[d]);
-    }
-    anynan = __any_sync(0xffffffffu, anynan);
-    __syncthreads();
-    if (lane == 0) {
-#pragma unroll
-        for (int d = 0; d < D; ++d) { smin[w][d] = glo[d]; smax[w][d] = ghi[d]; }
-        if (anynan) atomicOr(&snan, 2);
-    }
-    __syncthreads();
+    block_bounds<T, D>(lo, hi, mag, sm);
     if (threadIdx.x == 0) {
-        for (int w2 = 1; w2 < kThreads / 32; ++w2)
-            for (int d = 0; d < D; ++d) {
-                smin[0][d] = jl_min(smin[0][d], smin[w2][d]);
-                smax[0][d] = jl_max(smax[0][d], smax[w2][d]);
-            }
-        for (int d = 0; d < D; ++d) { hdr->gmin[d] = (double)smin[0][d]; hdr->gmax[d] = (double)smax[0][d]; }
-        hdr->nan_flag = (snan & 2) ? 1 : 0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            hdr->gmin[d] = (double)K::value(lo[d]);
+            hdr->gmax[d] = (double)K::value(hi[d]);
+        }
+        hdr->nan_flag = mag >= K::kExp ? 1 : 0;
         hdr->n_blocks_done = 0;
     }
 }
@@ -1857,7 +1861,7 @@ int build_typed(Ctx& ctx, Tree& t, const T* coords, int64_t n, double radius_d) 
     if ((err = ensure(t.partials, (size_t)nb * 8 * 8))) return cuda_status(ctx, err, "allocating partials");
     {
         PhaseTimer pt_(ctx, PH_BOUNDS);
-        launch_pdl(k_bounds<T, D>, nb, kThreads, 0, s, coords, n, t.partials.as<double>(), hdr);
+        launch_pdl(k_bounds<T, D>, nb, kThreads, 0, s, coords, n, t.partials.as<typename OrdKey<T>::I>(), hdr);
         ctx.kernel_launches += 1;
     }
     // Refit mode with a reusable previous order: re-encode in that order now,

@@ -154,14 +154,6 @@ __device__ __forceinline__ int cloud_of_position(const Batch& b, int64_t i) {
 }
 
 // --------------------------------------------------- Julia float semantics --
-// Base.min/max on IEEE floats for non-NaN operands: -0.0 orders below +0.0.
-template <class T> __host__ __device__ __forceinline__ T jl_min(T x, T y) {
-    return (y < x || (y == x && signbit(y) && !signbit(x))) ? y : x;
-}
-template <class T> __host__ __device__ __forceinline__ T jl_max(T x, T y) {
-    return (y > x || (y == x && !signbit(y) && signbit(x))) ? y : x;
-}
-
 // Correctly rounded arithmetic without contraction (Julia never fuses).
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
@@ -298,21 +290,6 @@ __device__ __forceinline__ unsigned lanemask_lt() {
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
     return m;
 }
-
-template <class T> __device__ __forceinline__ T warp_min(T v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = jl_min(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-template <class T> __device__ __forceinline__ T warp_max(T v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = jl_max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-// Integers: one redux.sync instead of a shuffle tree.
-__device__ __forceinline__ int warp_min(int v) { return __reduce_min_sync(0xffffffffu, v); }
-__device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(0xffffffffu, v); }
 
 template <class T> __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
