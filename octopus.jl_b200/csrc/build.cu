@@ -501,13 +501,26 @@ __global__ void __launch_bounds__(kThreads) k_emit_nodes(const K* __restrict__ s
         // pass, is their first position); each one's slot is its key's digit.
         const int shd = D * BITS - D * (L + 1);
         const int64_t lend = L + 2 <= BITS ? blockoff[(int64_t)(L + 2) * nblocks] : nn;  // first id past level L+1
+        // (all of them read at once: a loop that stopped at the first child
+        // past the range would wait for each in turn)
+        int32_t cs[NCH];
+#pragma unroll
+        for (int j = 0; j < NCH; ++j) cs[j] = first_child + j < lend ? nrange[first_child + j].x : INT32_MAX;
+        K ck[NCH];
+        int32_t cf[NCH];
+#pragma unroll
+        for (int j = 0; j < NCH; ++j) {
+            ck[j] = cs[j] < e ? skeys[cs[j]] : K(0);
+            cf[j] = cs[j] < e ? first_child_in[first_child + j] : -1;
+        }
         unsigned slots = 0u;
-        for (int64_t c = first_child; c < lend && c < (int64_t)first_child + NCH; ++c) {
-            const int64_t cs = nrange[c].x;
-            if (cs >= e) break;
-            slots |= 1u << slot_digit<D, K>(skeys[cs], shd, bt);
-            inner += first_child_in[c] >= 0;
-            link[c].parent = (int32_t)id;
+#pragma unroll
+        for (int j = 0; j < NCH; ++j) {
+            if (cs[j] < e) {
+                slots |= 1u << slot_digit<D, K>(ck[j], shd, bt);
+                inner += cf[j] >= 0;
+                link[first_child + j].parent = (int32_t)id;
+            }
         }
         nd.a = first_child;
         nd.b = -(int32_t)slots;
