@@ -606,29 +606,16 @@ constexpr int kWarpNodes = 64;
 constexpr int kPiece = 0x80;
 constexpr int kAscending = 1 << 17;  // beside kLinkFull: the node's points are visited in ascending order
 
-// This warp's next internal node (or any node of `todo`) for each team, -1 when none is left.
-__device__ __forceinline__ int32_t team_pick(unsigned& todo, int32_t id) {
-    const int team = (threadIdx.x & 31) / kTeam;
-    int pick = -1;
-#pragma unroll
-    for (int t = 0; t < 32 / kTeam; ++t) {
-        if (todo && t == team) pick = __ffs(todo) - 1;
-        todo &= todo - 1;
-    }
-    const int32_t q = __shfl_sync(0xffffffffu, id, pick & 31);
-    return pick < 0 ? -1 : q;
-}
-
 // Box of a team's lanes on order keys (integer min/max follow Julia's
 // min/max of finite values, -0.0 below +0.0), in every lane.
-template <class T, int D>
-__device__ __forceinline__ void team_fold(unsigned mask, typename OrdKey<T>::I* lo, typename OrdKey<T>::I* hi) {
+template <class T, int D, int W = kTeam>
+__device__ __forceinline__ void team_fold(typename OrdKey<T>::I* lo, typename OrdKey<T>::I* hi) {
 #pragma unroll
     for (int d = 0; d < D; ++d) {
 #pragma unroll
-        for (int o = kTeam / 2; o > 0; o >>= 1) {
-            lo[d] = min(lo[d], __shfl_xor_sync(mask, lo[d], o));
-            hi[d] = max(hi[d], __shfl_xor_sync(mask, hi[d], o));
+        for (int o = W / 2; o > 0; o >>= 1) {
+            lo[d] = min(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+            hi[d] = max(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
         }
     }
 }
@@ -858,7 +845,7 @@ __global__ void __launch_bounds__(kThreads, kLayoutBlocks) k_layout(int64_t capa
                         }
                     }
                     __syncwarp();
-                    team_fold<T, D>(FULL, rl, rh);
+                    team_fold<T, D>(rl, rh);
                     if (sub == j) {
 #pragma unroll
                         for (int d = 0; d < D; ++d) { lo[d] = min(lo[d], rl[d]); hi[d] = max(hi[d], rh[d]); }
@@ -921,7 +908,7 @@ __global__ void __launch_bounds__(kThreads, kLayoutBlocks) k_layout(int64_t capa
                 for (int32_t c = 0; c < cb; c += gmax) dstart[at + c] = (uint8_t)(kPiece | min(gmax, cb - c));
             }
             __syncwarp();
-            team_fold<T, D>(FULL, lo, hi);
+            team_fold<T, D>(lo, hi);
             // (a node covering its whole set already has that set's bounds)
             if (internal && (inner_m & team) == 0 && sub == 0 && !(ms & kLinkFull))
                 store_bounds<T, D>(tnode + q, lo, hi);
@@ -934,11 +921,10 @@ __global__ void __launch_bounds__(kThreads, kLayoutBlocks) k_layout(int64_t capa
 // One launch, two kinds of blocks that do not depend on each other (both need
 // only section 6).
 //
-// Node bounds: a team of eight lanes climbs from each internal node whose
-// children are all leaves; at a parent, the last internal child to arrive
-// folds the boxes of all its children, one per lane
-// (src/cpu/refit_cpu.jl:50-60).  No thread waits: a team that is not last
-// stops.  Only internal children count as arrivals, so the acquire-release
+// Node bounds: a lane climbs from each internal node whose children are all
+// leaves; at a parent, the boxes of all its children are folded for the last
+// internal child to arrive (src/cpu/refit_cpu.jl:50-60).  No thread waits: a
+// lane that is not last stops.  Only internal children count as arrivals, so the acquire-release
 // counters (whose acquire drops the SM's L1) are an eighth of the nodes.
 //
 // Chunks: one warp per span of kSpan visiting positions lists the chunks that
@@ -949,50 +935,69 @@ __global__ void __launch_bounds__(kThreads, kLayoutBlocks) k_layout(int64_t capa
 // next level, and so on up.
 constexpr int kSpansPerBlock = kThreads / 32;
 
-// A level costs three dependent round trips: the release of the team's box
-// with the counter, the sibling boxes, and in their shade the next link.
+// A level costs three dependent round trips: the release of the box with the
+// counter, the children's boxes, and in their shade the next link.  A warp
+// climbs from 32 nodes at once; those that arrive last at their parents are
+// folded by teams of one lane per child, as many at a time as the warp holds,
+// and every step is taken by the whole warp (teams with masks of their own
+// execute one after another).  The whole launch, with such teams of eight and
+// now: 16M uniform points 110 and 76 us, 500,009 2D points 25 and 17, 5.2M points
+// in 512 clouds 28 and 21, 100,000 points 12 and 12; one lane folding all the
+// children took 88, 17, 23 and 13, and 19 us instead of 15 for 200,003 Float64
+// points.
 template <class T, int D>
-__device__ __forceinline__ void fold_nodes(int64_t warp, int64_t warps, int64_t nn, TNode<T, D>* tnode,
+__device__ __forceinline__ void fold_nodes(int64_t first, int64_t stride, int64_t nn, TNode<T, D>* tnode,
                                            const NodeLink* __restrict__ link, int32_t* arrive) {
     using K = OrdKey<T>;
     using I = typename K::I;
-    const int lane = threadIdx.x & 31, sub = lane & (kTeam - 1);
-    const unsigned team = 0xffu << (lane & ~(kTeam - 1));
-    for (int64_t base = warp; base < nn; base += warps * 32) {
-        const int64_t id = base + warps * lane;
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int NCH = Dims<D>::nch;
+    const int lane = threadIdx.x & 31, sub = lane & (NCH - 1), team = lane / NCH;
+    for (int64_t base = first; base < nn; base += stride) {
         // nodes whose children are all leaves: their boxes are done (section 6)
-        const int meta0 = id < nn ? link[id].meta : 0;
-        unsigned todo = __ballot_sync(0xffffffffu, meta0 != 0 && (meta0 & (0xff00 | kLinkFull)) == 0);
-        while (todo) {
-            const int32_t q0 = team_pick(todo, (int32_t)id);
-            int32_t q = q0 >= 0 ? link[q0].parent : -1;
-            NodeLink lk;
+        int32_t q = -1;
+        NodeLink lk;
+        if (base + lane < nn) {
+            lk = link[base + lane];
+            if ((lk.meta & 0xff) != 0 && (lk.meta & (0xff00 | kLinkFull)) == 0) q = lk.parent;
             if (q >= 0) lk = link[q];
-            while (q >= 0 && !(lk.meta & kLinkFull)) {  // (a full node's bounds come from the set's reduce)
-                const int nc = lk.meta & 0xff, inner = lk.meta >> 8 & 0xff;
-                const int32_t up = lk.parent;
-                NodeLink next;
-                if (up >= 0) next = link[up];
-                int old = 0;
-                if (sub == 0)
-                    old = cuda::atomic_ref<int32_t, cuda::thread_scope_device>(arrive[q]).fetch_add(
-                        1, cuda::memory_order_acq_rel);
-                old = __shfl_sync(team, old, 0, kTeam);
-                if (old != inner - 1) break;
-                __syncwarp(team);  // lane 0's acquire covers the team's reads
-                const TNode<T, D>* ch = tnode + lk.first + sub;
+        }
+        while (true) {
+            if (q >= 0 && (lk.meta & kLinkFull)) q = -1;  // (a full node's bounds come from the set's reduce)
+            if (!__any_sync(FULL, q >= 0)) break;
+            NodeLink next;
+            if (q >= 0) {
+                if (lk.parent >= 0) next = link[lk.parent];
+                if (cuda::atomic_ref<int32_t, cuda::thread_scope_device>(arrive[q]).fetch_add(
+                        1, cuda::memory_order_acq_rel) != (lk.meta >> 8 & 0xff) - 1)
+                    q = -1;
+            }
+            __syncwarp();  // a lane's acquire covers its team's reads
+            for (unsigned won = __ballot_sync(FULL, q >= 0); won;) {
+                int src = -1;
+#pragma unroll
+                for (int t = 0; t < 32 / NCH; ++t) {
+                    if (won && t == team) src = __ffs(won) - 1;
+                    won &= won - 1;
+                }
+                const int32_t node = __shfl_sync(FULL, q, src & 31);
+                const int32_t ch0 = __shfl_sync(FULL, lk.first, src & 31);
+                const int nc = __shfl_sync(FULL, lk.meta, src & 31) & 0xff;
+                const bool in = src >= 0 && sub < nc;
                 I lo[D], hi[D];
 #pragma unroll
                 for (int d = 0; d < D; ++d) {
-                    lo[d] = sub < nc ? K::key(K::bits(__ldcg(&ch->lo[d]))) : K::kMaxKey;
-                    hi[d] = sub < nc ? K::key(K::bits(__ldcg(&ch->hi[d]))) : K::kMinKey;
+                    lo[d] = in ? K::key(K::bits(__ldcg(&tnode[ch0 + sub].lo[d]))) : K::kMaxKey;
+                    hi[d] = in ? K::key(K::bits(__ldcg(&tnode[ch0 + sub].hi[d]))) : K::kMinKey;
                 }
-                team_fold<T, D>(team, lo, hi);
-                if (sub == 0) store_bounds<T, D>(tnode + q, lo, hi);
-                q = up;
+                team_fold<T, D, NCH>(lo, hi);
+                if (src >= 0 && sub == 0) store_bounds<T, D>(tnode + node, lo, hi);
+            }
+            __syncwarp();  // the boxes' stores, before the lanes' next releases
+            if (q >= 0) {
+                q = lk.parent;
                 lk = next;
             }
-            __syncwarp();
         }
     }
 }
@@ -1013,8 +1018,8 @@ __global__ void __launch_bounds__(kThreads) k_fold_chunks(int span_blocks, int64
     if (nn > capacity || (hdr->status & DF_TIMEOUT)) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if ((int)blockIdx.x >= span_blocks) {
-        fold_nodes<T, D>((int64_t)(blockIdx.x - span_blocks) * (kThreads / 32) + w,
-                         (int64_t)(gridDim.x - span_blocks) * (kThreads / 32), nn, tnode, link, arrive);
+        fold_nodes<T, D>(((int64_t)(blockIdx.x - span_blocks) * kSpansPerBlock + w) * 32,
+                         (int64_t)(gridDim.x - span_blocks) * kThreads, nn, tnode, link, arrive);
         return;
     }
     int32_t node = blockIdx.x * kSpansPerBlock + w;
