@@ -339,16 +339,16 @@ OCT_API int oct_edges_count_noalloc(oct_ctx* ctx, const oct_tree* query, const o
  *                          the waits after it run out (-1 = off, default)
  * Kernel shapes (no result depends on them; 0 = the tuning table's choice,
  * or the default when no table is loaded, see oct_ctx_load_tuning):
- *   OCT_OPT_MAX_SEG        leaves sharing one staged chunk of the traversal, 1..16 (16)
- *   OCT_OPT_MULTI_POP      internal nodes the traversal expands together, 1..4 (4)
+ *   OCT_OPT_MAX_SEG        1..16 (16): accepted and reported, without effect (the
+ *                          count walks boxes over the visiting order, not the tree)
+ *   OCT_OPT_MULTI_POP      1..4 (4): likewise without effect
  *   OCT_OPT_FILL_CHUNK     the fill's stores: 1 direct (default), or 32, 64 or 128 for
  *                          bulk copies of that many edges per chunk (a table row says 0
  *                          for direct)
- *   OCT_OPT_GROUP_CAP      query points per traversal group, 8..32 (32), set at the build
- *   OCT_OPT_SUB_BOXES      boxes a group's queries are split into (runs of 32/k lanes)
- *                          for the test that skips distant target points: 1, 2 or 4 (1)
- *   OCT_OPT_PREFETCH       the traversal prefetches into L1 what it reads next (the next
- *                          leaf chunk's points, the next node's children): 1 off, 2 on (off)
+ *   OCT_OPT_GROUP_CAP      points per chunk of the search layout (queries of a warp,
+ *                          targets of a step), 8..32 (32), set at the build
+ *   OCT_OPT_SUB_BOXES      1, 2 or 4 (1): accepted and reported, without effect
+ *   OCT_OPT_PREFETCH       1 or 2 (1): accepted and reported, without effect
  * Read-only (oct_ctx_get_option):
  *   OCT_STAT_TUNING_ROW       tuning-table row the last count or build used (-1 = defaults)
  *   OCT_STAT_BUILD_ATTEMPTS   topology attempts of the last build (1 = none retried)

@@ -33,12 +33,13 @@ struct Ctx;
 // No result depends on them: they change how the work is cut, not what is
 // computed.
 struct Tuning {
-    int max_seg = 16;     // leaves sharing one staged chunk of the traversal (1..16)
-    int multi_pop = 4;    // internal nodes expanded together by the traversal (1..4)
     int fill_chunk = 0;   // the fill's stores: 0 direct, else bulk copies of chunks of 32, 64 or 128 edges
-    int group_cap = 32;   // query points per traversal group, set at the build (8..32)
-    int sub_boxes = 1;    // boxes a group's queries are split into for the target test (1, 2 or 4)
-    int prefetch = 0;     // 1: the traversal prefetches the next chunk's points / children into L1
+    int group_cap = 32;   // points per chunk of the search layout, set at the build (8..32)
+    // Shapes of a walk of the tree itself: accepted, kept and reported, without effect.
+    int max_seg = 16;     // 1..16
+    int multi_pop = 4;    // 1..4
+    int sub_boxes = 1;    // 1, 2 or 4
+    int prefetch = 0;     // 0 or 1
 };
 
 // One row of a tuning table: the shapes measured best for point sets of

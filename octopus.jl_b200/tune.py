@@ -1,7 +1,7 @@
-"""Autotuner of the kernel shapes (leaf chunks per traversal step, internal
-nodes expanded together, fill staging depth, query points per traversal
-group, sub-boxes of a group for the target test, L1 prefetch in the
-traversal).
+"""Autotuner of the kernel shapes: points per chunk of the search layout
+(group_cap) and the fill's stores (fill_chunk).  The table's other columns
+(max_seg, multi_pop, sub_boxes, prefetch) belonged to an earlier walk of the
+tree; they are written with their defaults and change nothing.
 
     python octopus.jl_b200/tune.py [--out PATH] [--steps K] [--rounds R]
 
@@ -32,11 +32,7 @@ DEFAULT_TABLE = os.path.join(HERE, "tuning.tsv")
 # option id and candidate values of each shape, in the order they are tuned
 SHAPES = [
     ("group_cap", 9, (16, 24, 32)),
-    ("max_seg", 6, (1, 4, 8, 16)),
-    ("multi_pop", 7, (1, 2, 4)),
     ("fill_chunk", 8, (0, 32, 64, 128)),
-    ("sub_boxes", 10, (1, 2, 4)),
-    ("prefetch", 11, (0, 1)),
 ]
 DEFAULTS = {"group_cap": 32, "max_seg": 16, "multi_pop": 4, "fill_chunk": 0, "sub_boxes": 1, "prefetch": 0}
 
@@ -90,12 +86,10 @@ class Runner:
     def force(self, shapes):
         for name, opt, _ in SHAPES:
             v = shapes.get(name)
-            # 0 hands a shape back to the table; prefetch is forced as 1 (off) /
-            # 2 (on), direct fill stores (fill_chunk 0) as 1
+            # 0 hands a shape back to the table; direct fill stores
+            # (fill_chunk 0) are forced as 1
             if v is None:
                 v = 0
-            elif name == "prefetch":
-                v = v + 1
             elif name == "fill_chunk" and v == 0:
                 v = 1
             self.ctx.check(self.ctx.lib.oct_ctx_set_option(self.ctx.handle, opt, int(v)), name)
