@@ -658,13 +658,30 @@ __device__ __forceinline__ void store_bounds(TNode<T, D>* nd, const typename Ord
     }
 }
 
+// Box units of a single set from this build's bounds, with the host's
+// arithmetic (the origin as in k_resort_mark; Tree::box_units).
+template <class T, int D>
+__device__ __forceinline__ BoxUnits set_units(const OctHeader* hdr, T inv_r) {
+    BoxUnits u;
+    double cells = 0.0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+        const T o = sub_rn((T)hdr->gmin[d], T(1e-6));
+        u.o[d] = (double)o;
+        cells = fmax(cells, (double)mul_rn(sub_rn((T)hdr->gmax[d], o), inv_r));
+    }
+    u.mul = box_mul(cells);
+    u.s = (double)inv_r * u.mul;
+    return u;
+}
+
 template <class T, int D>
 __global__ void __launch_bounds__(kThreads, kLayoutBlocks) k_layout(int64_t capacity, int64_t n, TNode<T, D>* __restrict__ tnode,
                                                      const int2* __restrict__ nrange,
                                                      const NodeLink* __restrict__ link,
                                                      const SPt<T, D>* __restrict__ spts, SPt<T, D>* __restrict__ dpts,
                                                      uint8_t* __restrict__ dstart, int32_t* __restrict__ dnode,
-                                                     TNode<float, D>* __restrict__ rbox, int gmax,
+                                                     BoxNode<T, D>* __restrict__ rbox, int gmax, T inv_r,
                                                      const OctHeader* hdr,
                                                      Batch bt) {
     pdl_wait();
@@ -685,6 +702,11 @@ __global__ void __launch_bounds__(kThreads, kLayoutBlocks) k_layout(int64_t capa
     // Nodes are taken in clusters of 2^csh ids, a warp's clusters `warps` apart.
     const int csh = nn >= warps * (32 * kPickRounds) ? kClusterShift : 0;
     int64_t next = (int64_t)blockIdx.x * (kThreads / 32) + w;
+    __shared__ BoxUnits units;
+    if constexpr (sizeof(T) == 8) {
+        if (threadIdx.x == 0 && !bt.n_clouds) units = set_units<T, D>(hdr, inv_r);
+        __syncthreads();
+    }
     if (next >= warps) return;  // warp-uniform
     __shared__ int32_t queue[kThreads / 32][32 * (kPickRounds + 1)];
     int head = 0, queued = 0;
@@ -724,7 +746,7 @@ __global__ void __launch_bounds__(kThreads, kLayoutBlocks) k_layout(int64_t capa
         // One node per lane: its first child (a leaf root is its own), its
         // children (0: a leaf root), whether its bounds are the set's, its
         // unit's direction and the shift to visiting positions.
-        int32_t node = -1, first = 0, meta = 0, to = 0;
+        int32_t node = -1, first = 0, meta = 0, to = 0, cloud = 0;
         if (lane < take) {
             node = queue[w][head + lane];
             const NodeLink lk = link[node];
@@ -736,9 +758,9 @@ __global__ void __launch_bounds__(kThreads, kLayoutBlocks) k_layout(int64_t capa
             asm volatile("prefetch.global.L2 [%0];" ::"l"(tnode + first + max((meta & 0xff) - 1, 0)));
             int32_t c0 = 0, c1 = (int32_t)n;
             if (bt.n_clouds) {
-                const int c = cloud_of_position(bt, range.x);
-                c0 = (int32_t)bt.coff[c];
-                c1 = (int32_t)bt.coff[c + 1];
+                cloud = cloud_of_position(bt, range.x);
+                c0 = (int32_t)bt.coff[cloud];
+                c1 = (int32_t)bt.coff[cloud + 1];
             }
             to = (int32_t)((uint32_t)c0 + (uint32_t)c1);
             if ((lk.meta & 0xff) > (lk.meta >> 8 & 0xff)) {  // (some child is a leaf)
@@ -762,6 +784,7 @@ __global__ void __launch_bounds__(kThreads, kLayoutBlocks) k_layout(int64_t capa
             const int ms = __shfl_sync(FULL, meta, src & 31);
             const int32_t q = __shfl_sync(FULL, node, src & 31), ch0 = __shfl_sync(FULL, first, src & 31);
             const int32_t shift = __shfl_sync(FULL, to, src & 31);
+            const int32_t cl = sizeof(T) == 8 ? __shfl_sync(FULL, cloud, src & 31) : 0;
             const bool internal = src < take && (ms & 0xff) != 0, asc = ms & kAscending;
             const int nc = src >= take ? 0 : internal ? ms & 0xff : 1;
             // the visiting position of the child's point at sorted position a is place(a, b) + its rank
@@ -892,11 +915,13 @@ __global__ void __launch_bounds__(kThreads, kLayoutBlocks) k_layout(int64_t capa
                     const int32_t pos = place(ca, run_end - ca);
                     dstart[pos] = (uint8_t)(run_end - ca);
                     dnode[pos] = ch0 + sub;
-                    TNode<float, D> nd;
+                    BoxNode<T, D> nd;
+                    BoxUnits u;
+                    if constexpr (sizeof(T) == 8) u = bt.n_clouds ? cloud_units(bt, cl) : units;
 #pragma unroll
                     for (int d = 0; d < D; ++d) {
-                        nd.lo[d] = float_below(K::value(rlo[d]));
-                        nd.hi[d] = float_above(K::value(rhi[d]));
+                        nd.lo[d] = box_coord(K::value(rlo[d]), d, u);
+                        nd.hi[d] = box_coord(K::value(rhi[d]), d, u);
                     }
                     nd.a = pos;
                     nd.b = run_end - ca;
@@ -1008,9 +1033,10 @@ __global__ void __launch_bounds__(kThreads) k_fold_chunks(int span_blocks, int64
                                                           int32_t* arrive, const SPt<T, D>* __restrict__ dpts,
                                                           const uint8_t* __restrict__ dstart,
                                                           const int32_t* __restrict__ dnode,
-                                                          const TNode<float, D>* __restrict__ rbox, int64_t chunk_cap,
-                                                          const __grid_constant__ Bvh<D> bv,
-                                                          int32_t* __restrict__ bvh_arrive, OctHeader* hdr) {
+                                                          const BoxNode<T, D>* __restrict__ rbox, int64_t chunk_cap,
+                                                          const __grid_constant__ Bvh<T, D> bv,
+                                                          int32_t* __restrict__ bvh_arrive, T inv_r, OctHeader* hdr,
+                                                          Batch bt) {
     pdl_wait();
     pdl_trigger();
     __shared__ uint32_t list_sm[kSpansPerBlock][kSpan];  // (offset in the span << 8) | dstart
@@ -1050,29 +1076,40 @@ __global__ void __launch_bounds__(kThreads) k_fold_chunks(int span_blocks, int64
     if (lane == 0) cbase = (int32_t)atomicAdd((unsigned long long*)&hdr->n_groups, (unsigned long long)total);
     cbase = __shfl_sync(0xffffffffu, cbase, 0);
     __syncwarp();
-    float slo[D], shi[D];
+    using B = typename BoxCoord<T>::type;
+    constexpr B kHigh = sizeof(T) == 8 ? B(1 << 30) : B(INFINITY), kLow = -kHigh;  // beyond every box
+    B slo[D], shi[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) { slo[d] = INFINITY; shi[d] = -INFINITY; }
+    for (int d = 0; d < D; ++d) { slo[d] = kHigh; shi[d] = kLow; }
     for (int k = 0; k < total; k += 32) {
         const uint32_t v = k + lane < total ? list[k + lane] : 0;
         const int32_t first = (int32_t)(s0 + (v >> 8));
         const int cnt = (int)(v & (kPiece - 1));
-        TNode<float, D> nd;
+        BoxNode<T, D> nd;
 #pragma unroll
-        for (int d = 0; d < D; ++d) { nd.lo[d] = INFINITY; nd.hi[d] = -INFINITY; }
+        for (int d = 0; d < D; ++d) { nd.lo[d] = kHigh; nd.hi[d] = kLow; }
         nd.a = first;
         nd.b = cnt;
         if (v && !(v & kPiece)) nd = rbox[dnode[first]];
-        for (unsigned pm = __ballot_sync(0xffffffffu, (v & kPiece) != 0); pm; pm &= pm - 1) {
+        unsigned pm = __ballot_sync(0xffffffffu, (v & kPiece) != 0);
+        BoxUnits u;
+        if constexpr (sizeof(T) == 8) {
+            if (pm && !bt.n_clouds) u = set_units<T, D>(hdr, inv_r);
+        }
+        for (; pm; pm &= pm - 1) {
             const int j = __ffs(pm) - 1;
             const int32_t f = __shfl_sync(0xffffffffu, first, j);
             const int m = __shfl_sync(0xffffffffu, cnt, j);
             SPt<T, D> p;
             if (lane < m) p = dpts[f + lane];
+            if constexpr (sizeof(T) == 8) {
+                if (bt.n_clouds) u = cloud_units(bt, cloud_of_position(bt, f));
+            }
 #pragma unroll
             for (int d = 0; d < D; ++d) {
-                const float lo = box_min(lane < m ? float_below(p.x[d]) : INFINITY);
-                const float hi = box_max(lane < m ? float_above(p.x[d]) : -INFINITY);
+                const B x = lane < m ? box_coord(p.x[d], d, u) : kLow;
+                const B lo = box_min(lane < m ? x : kHigh);
+                const B hi = box_max(x);
                 if (lane == j) { nd.lo[d] = lo; nd.hi[d] = hi; }
             }
         }
@@ -1083,8 +1120,8 @@ __global__ void __launch_bounds__(kThreads) k_fold_chunks(int span_blocks, int64
             shi[d] = max(shi[d], box_max(nd.hi[d]));
         }
     }
-    auto store_box = [&](TNode<float, D>* out, int32_t a, int32_t b) {
-        TNode<float, D> nd;
+    auto store_box = [&](BoxNode<T, D>* out, int32_t a, int32_t b) {
+        BoxNode<T, D> nd;
 #pragma unroll
         for (int d = 0; d < D; ++d) { nd.lo[d] = slo[d]; nd.hi[d] = shi[d]; }
         nd.a = a;
@@ -1102,11 +1139,11 @@ __global__ void __launch_bounds__(kThreads) k_fold_chunks(int span_blocks, int64
         old = __shfl_sync(0xffffffffu, old, 0);
         if (old != need - 1) return;
         __syncwarp();
-        const TNode<float, D>* ch = bv.lev[l - 1] + 32 * up + lane;
+        const BoxNode<T, D>* ch = bv.lev[l - 1] + 32 * up + lane;
 #pragma unroll
         for (int d = 0; d < D; ++d) {
-            slo[d] = box_min(lane < need ? __ldcg(&ch->lo[d]) : INFINITY);
-            shi[d] = box_max(lane < need ? __ldcg(&ch->hi[d]) : -INFINITY);
+            slo[d] = box_min(lane < need ? __ldcg(&ch->lo[d]) : kHigh);
+            shi[d] = box_max(lane < need ? __ldcg(&ch->hi[d]) : kLow);
         }
         if (lane == 0) store_box(bv.lev[l] + up, 0, 0);
         bvh_arrive += bv.cnt[l];
@@ -1554,7 +1591,8 @@ void guard_check(Ctx& ctx, const DevBuf& b, size_t bytes, OctHeader* hdr) {
 // Bounds, visiting order, chunks and box hierarchy (sections 6 and 7) of the
 // tree whose topology was just launched; `nodes` bounds its node count.
 template <class T, int D>
-void launch_layout(Ctx& ctx, Tree& t, int64_t n, int64_t node_cap, int64_t chunk_cap, int64_t nodes, int gmax) {
+void launch_layout(Ctx& ctx, Tree& t, int64_t n, int64_t node_cap, int64_t chunk_cap, int64_t nodes, int gmax,
+                   T inv_r) {
     OctHeader* hdr = t.hdr.as<OctHeader>();
     {
         PhaseTimer pt_(ctx, PH_REFIT);
@@ -1562,15 +1600,14 @@ void launch_layout(Ctx& ctx, Tree& t, int64_t n, int64_t node_cap, int64_t chunk
         const int64_t blocks = std::min<int64_t>(div_up(nodes, kThreads), 2 * kLayoutWave);
         launch_pdl(k_layout<T, D>, blocks, kThreads, 0, ctx.stream, node_cap, n, t.tnode.as<TNode<T, D>>(),
             t.nrange.as<int2>(), t.link.as<NodeLink>(), t.spts.as<SPt<T, D>>(), t.dpts.as<SPt<T, D>>(),
-            t.dstart.as<uint8_t>(), t.dnode.as<int32_t>(), t.rbox.as<TNode<float, D>>(), gmax, hdr, t.batch());
+            t.dstart.as<uint8_t>(), t.dnode.as<int32_t>(), t.rbox.as<BoxNode<T, D>>(), gmax, inv_r, hdr, t.batch());
     }
     PhaseTimer pt_(ctx, PH_GROUPS);
     const int span_blocks = div_up(n, kSpan * kSpansPerBlock);
     const int64_t fold_blocks = std::min<int64_t>(div_up(nodes, kThreads), 148 * 16);
     launch_pdl(k_fold_chunks<T, D>, span_blocks + fold_blocks, kThreads, 0, ctx.stream, span_blocks, n, node_cap,
-        t.tnode.as<TNode<T, D>>(), t.link.as<NodeLink>(), t.arrive.as<int32_t>(), t.dpts.as<SPt<T, D>>(), t.dstart.as<uint8_t>(), t.dnode.as<int32_t>(), t.rbox.as<TNode<float, D>>(), chunk_cap,
-        t.search_layout<D>(),
-        t.bvh_arrive.as<int32_t>(), hdr);
+        t.tnode.as<TNode<T, D>>(), t.link.as<NodeLink>(), t.arrive.as<int32_t>(), t.dpts.as<SPt<T, D>>(), t.dstart.as<uint8_t>(), t.dnode.as<int32_t>(), t.rbox.as<BoxNode<T, D>>(), chunk_cap,
+        t.search_layout<T, D>(), t.bvh_arrive.as<int32_t>(), inv_r, hdr, t.batch());
     ctx.kernel_launches += 2;
 }
 
@@ -1593,7 +1630,7 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
     const int n_arrive = (int)(bvh_nodes - lev[0]);
     if ((err = ensure(t.dpts, (size_t)n * sizeof(SPt<T, D>))) || (err = ensure(t.dstart, (size_t)n)) ||
         (err = ensure(t.dnode, (size_t)n * 4)) ||
-        (err = ensure(t.bvh, (size_t)bvh_nodes * sizeof(TNode<float, D>))) ||
+        (err = ensure(t.bvh, (size_t)bvh_nodes * sizeof(BoxNode<T, D>))) ||
         (err = ensure(t.bvh_arrive, (size_t)n_arrive * 4)))
         return cuda_status(ctx, err, "allocating the search layout");
     OctHeader* hdr = t.hdr.as<OctHeader>();
@@ -1676,7 +1713,7 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
                 ctx.kernel_launches += 1;
             }
             // the chunk array's capacity is that of the build that made it
-            launch_layout<T, D>(ctx, t, n, t.capacity, t.n_groups, t.n_nodes, t.group_cap);
+            launch_layout<T, D>(ctx, t, n, t.capacity, t.n_groups, t.n_nodes, t.group_cap, inv_cs);
             if ((err = cudaGetLastError())) return cuda_status(ctx, err, "bounds refit");
             t.last_path = 2;
             t.sorted_buf = sorted;
@@ -1746,14 +1783,14 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
             (err = ensure_g(ctx, t.nrange, (size_t)cap * 8)) || (err = ensure_g(ctx, t.link, (size_t)cap * sizeof(NodeLink))) ||
             (err = ensure_g(ctx, t.arrive, (size_t)cap * 4)) || (err = ensure_g(ctx, t.fchild, (size_t)cap * 4)) ||
             (err = ensure(t.scan_tmp, (size_t)scan_tmp_elems(nbc) * 8)) ||
-            (err = ensure_g(ctx, t.rbox, (size_t)cap * sizeof(TNode<float, D>))) ||
-            (err = ensure_g(ctx, t.chunk, gcap * sizeof(TNode<float, D>))))
+            (err = ensure_g(ctx, t.rbox, (size_t)cap * sizeof(BoxNode<T, D>))) ||
+            (err = ensure_g(ctx, t.chunk, gcap * sizeof(BoxNode<T, D>))))
             return cuda_status(ctx, err, "allocating node arrays");
         if ((err = guard_fill(ctx, t.tnode, (size_t)cap * sizeof(TNode<T, D>))) ||
             (err = guard_fill(ctx, t.nrange, (size_t)cap * 8)) || (err = guard_fill(ctx, t.link, (size_t)cap * sizeof(NodeLink))) ||
             (err = guard_fill(ctx, t.arrive, (size_t)cap * 4)) || (err = guard_fill(ctx, t.fchild, (size_t)cap * 4)) ||
-            (err = guard_fill(ctx, t.rbox, (size_t)cap * sizeof(TNode<float, D>))) ||
-            (err = guard_fill(ctx, t.chunk, gcap * sizeof(TNode<float, D>))))
+            (err = guard_fill(ctx, t.rbox, (size_t)cap * sizeof(BoxNode<T, D>))) ||
+            (err = guard_fill(ctx, t.chunk, gcap * sizeof(BoxNode<T, D>))))
             return cuda_status(ctx, err, "node array guards");
         {
         PhaseTimer pt_(ctx, PH_TOPOLOGY);
@@ -1768,15 +1805,15 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
             t.blockoff.as<int64_t>(), nblocks, hdr, bt);
         ctx.kernel_launches += 3;
         }
-        launch_layout<T, D>(ctx, t, n, cap, (int64_t)gcap, cap, gmax);
+        launch_layout<T, D>(ctx, t, n, cap, (int64_t)gcap, cap, gmax, inv_cs);
         if (ctx.guard_check) {
             guard_check(ctx, t.tnode, (size_t)cap * sizeof(TNode<T, D>), hdr);
             guard_check(ctx, t.nrange, (size_t)cap * 8, hdr);
             guard_check(ctx, t.link, (size_t)cap * sizeof(NodeLink), hdr);
             guard_check(ctx, t.arrive, (size_t)cap * 4, hdr);
             guard_check(ctx, t.fchild, (size_t)cap * 4, hdr);
-            guard_check(ctx, t.rbox, (size_t)cap * sizeof(TNode<float, D>), hdr);
-            guard_check(ctx, t.chunk, gcap * sizeof(TNode<float, D>), hdr);
+            guard_check(ctx, t.rbox, (size_t)cap * sizeof(BoxNode<T, D>), hdr);
+            guard_check(ctx, t.chunk, gcap * sizeof(BoxNode<T, D>), hdr);
             if (moved == -1) {
                 for (int b = 0; b < 2; ++b) guard_check(ctx, t.keys[b], (size_t)n * sizeof(K), hdr);
                 guard_check(ctx, t.vals[0], (size_t)n * 4, hdr);
@@ -1842,10 +1879,12 @@ int host_key_width(Ctx& ctx, Tree& t, T radius) {
         return set_error(ctx, ERR_INEXACT, "InexactError: floor(Int32, NaN/Inf) in bin_point (non-finite coordinate)");
     const T inv_cs = T(1) / radius;
     int64_t cmax_all = 0;
+    double cells = 0.0;
     for (int d = 0; d < D; ++d) {
         const T o = (T)t.hdr_host->gmin[d] - T(1e-6);
         t.origin[d] = (double)o;
         const T v = ((T)t.hdr_host->gmax[d] - o) * inv_cs;
+        cells = std::max(cells, (double)v);
         const T f = std::floor(v);
         if (!(f >= T(-2147483648.0) && f < T(2147483648.0)))
             return set_error(ctx, ERR_INEXACT, "InexactError: floor(Int32, (p - origin) / radius) exceeds Int32");
@@ -1854,6 +1893,7 @@ int host_key_width(Ctx& ctx, Tree& t, T radius) {
         c = c < 0 ? 0 : (c > cm ? cm : c);
         cmax_all = std::max(cmax_all, c);
     }
+    t.mul = box_mul(cells);
     int nbits_axis = 0;
     while (nbits_axis < 63 && (cmax_all >> nbits_axis) != 0) ++nbits_axis;
     t.key_bits = D * nbits_axis;
@@ -1964,6 +2004,7 @@ int build_batch_typed(Ctx& ctx, Tree& t, const T* coords, int64_t n, const int64
     // (src/cpu/bin_cpu.jl:22,35,60; src/cpu/edges_cpu.jl:184-185).
     std::vector<double> cp((size_t)nc * kCloudParams, 0.0);
     int64_t cmax_all = 0;
+    double cells = 0.0;
     for (int c = 0; c < nc; ++c) {
         if (coff_host[c + 1] == coff_host[c]) continue;
         const double* b = cb.data() + (size_t)c * 8;
@@ -1975,7 +2016,9 @@ int build_batch_typed(Ctx& ctx, Tree& t, const T* coords, int64_t n, const int64
         for (int d = 0; d < D; ++d) {
             const T o = (T)b[d] - T(1e-6);
             p[d] = (double)o;
-            const T f = std::floor(((T)b[3 + d] - o) * inv_cs);
+            const T v = ((T)b[3 + d] - o) * inv_cs;
+            cells = std::max(cells, (double)v);
+            const T f = std::floor(v);
             if (!(f >= T(-2147483648.0) && f < T(2147483648.0)))
                 return set_error(ctx, ERR_INEXACT, "InexactError: floor(Int32, (p - origin) / radius) exceeds Int32");
             int64_t ci = (int64_t)f;
@@ -1991,6 +2034,7 @@ int build_batch_typed(Ctx& ctx, Tree& t, const T* coords, int64_t n, const int64
     }
     if ((err = cudaMemcpyAsync(t.b_cparam.p, cp.data(), cp.size() * 8, cudaMemcpyHostToDevice, s)))
         return cuda_status(ctx, err, "cloud parameters");
+    t.mul = box_mul(cells);
     int nbits_axis = 0;
     while (nbits_axis < 63 && (cmax_all >> nbits_axis) != 0) ++nbits_axis;
     int cbits = 0;

@@ -60,17 +60,47 @@ template <class T, int D> struct alignas(16) TNode {
 // Search layout of a built tree: the points in the order in which the
 // reference's depth-first search visits them, cut into chunks of at most 32
 // (runs of sibling leaves) with their boxes (TNode: a = first position, b =
-// count; in float for every element type, a Float64 box rounded outward: the
-// box tests only have to keep what may be near), under a hierarchy of boxes with fan-out 32 over fixed spans of
+// count), under a hierarchy of boxes with fan-out 32 over fixed spans of
 // positions.  lev[0] holds one node per kSpan positions (a = first chunk
 // starting in the span, b = number of such chunks); lev[l] one node per 32 of
 // lev[l - 1].
+//
+// A Float32 box is in coordinates.  A Float64 box is in 32-bit fixed point:
+// floor((x - o) s) of its corners, o the set's (or cloud's) origin and s =
+// mul / radius with mul = 2^14, or less when the set is wider than 2^15 radii
+// (BoxUnits), so that every value stays below 2^29.  The units follow the radius
+// and the set's own place, so the boxes reject as much at any offset and scale
+// (float boxes of coordinates reject nothing once a float step is a radius
+// wide: count and fill of 200,003 points shifted by 3e6, r = 0.03, took 57 ms
+// and take 0.25).  A node is half of one in doubles, whose loads and Float64
+// latency cost more (8M uniform points in the unit cube: 4.42 ms, 4.9 with
+// doubles, 4.26 with floats).
+template <class T> struct BoxCoord { using type = T; };
+template <> struct BoxCoord<double> { using type = int32_t; };
+template <class T, int D> using BoxNode = TNode<typename BoxCoord<T>::type, D>;
+
+struct BoxUnits {
+    double o[3];
+    double s;
+    double width;  // 1 / s (for the search)
+    double mul;    // units per radius, a power of two
+};
+// `mul` for a set `cells` radii wide, 2^-2 to 2^14: cells * mul < 2^29 for
+// cells below 2^31 (the host refuses more).
+__host__ __device__ inline double box_mul(double cells) {
+    union { double d; unsigned long long u; } v;
+    v.d = cells;
+    const int bits = (int)(v.u >> 52 & 0x7ff) - 1022;  // cells < 2^bits
+    const int k = 29 - bits > 14 ? 14 : 29 - bits < -2 ? -2 : 29 - bits;
+    v.u = (unsigned long long)(k + 1023) << 52;
+    return v.d;
+}
 constexpr int kSpanShift = 9;
 constexpr int kSpan = 1 << kSpanShift;
 constexpr int kBvhLevels = 4;
-template <int D> struct Bvh {
-    TNode<float, D>* chunk = nullptr;
-    TNode<float, D>* lev[kBvhLevels] = {};
+template <class T, int D> struct Bvh {
+    BoxNode<T, D>* chunk = nullptr;
+    BoxNode<T, D>* lev[kBvhLevels] = {};
     int32_t cnt[kBvhLevels] = {};
     int32_t top = 0;  // highest level built: the first with at most 64 nodes, or the last
 };
@@ -141,7 +171,20 @@ struct Batch {
     int32_t kbits = 0;
     const int64_t* coff = nullptr;   // [n_clouds + 1]
     const double* cparam = nullptr;  // [n_clouds * kCloudParams], values exact in the element type
+    double mul = 1.0;                // BoxUnits::mul of every cloud
 };
+
+// Box units of one cloud.
+__device__ __forceinline__ BoxUnits cloud_units(const Batch& b, int cloud) {
+    const double* cp = b.cparam + (size_t)cloud * kCloudParams;
+    BoxUnits u;
+    u.o[0] = cp[0];
+    u.o[1] = cp[1];
+    u.o[2] = cp[2];
+    u.s = cp[3] * b.mul;
+    u.mul = b.mul;
+    return u;
+}
 
 // Cloud containing input (== sorted) position i: binary search of coff.
 __device__ __forceinline__ int cloud_of_position(const Batch& b, int64_t i) {
@@ -210,11 +253,13 @@ __device__ __forceinline__ float box_max(float v) {
     asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(m) : "f"(v));
     return m;
 }
-// Values rounded down / up to float.
-__device__ __forceinline__ float float_below(float v) { return v; }
-__device__ __forceinline__ float float_above(float v) { return v; }
-__device__ __forceinline__ float float_below(double v) { return __double2float_rd(v); }
-__device__ __forceinline__ float float_above(double v) { return __double2float_ru(v); }
+__device__ __forceinline__ int32_t box_min(int32_t v) { return __reduce_min_sync(0xffffffffu, v); }
+__device__ __forceinline__ int32_t box_max(int32_t v) { return __reduce_max_sync(0xffffffffu, v); }
+// A coordinate as a box holds it (monotone, so boxes of coordinates map to boxes).
+__device__ __forceinline__ float box_coord(float x, int, const BoxUnits&) { return x; }
+__device__ __forceinline__ int32_t box_coord(double x, int d, const BoxUnits& u) {
+    return __double2int_rd(__dmul_rn(__dsub_rn(x, u.o[d]), u.s));
+}
 
 // Morton interleave, src/morton.jl:13-23 and :50-58.
 __host__ __device__ __forceinline__ uint64_t split_by_3(uint64_t x) {

@@ -12,13 +12,12 @@
 //     a run of sibling leaves).  It walks the box hierarchy over the target's
 //     layout, one lane per child box (fan-out 32), in ascending position,
 //     down to the target chunks.  The box tests are conservative
-//     (boxes_near), and the exact per-pair test
+//     (QueryBox), and the exact per-pair test
 //     d2 = ((dx*dx + dy*dy) + dz*dz) <= r*r decides membership.
 //   * Target points are staged in shared memory and broadcast to the 32 lanes.
 //   * counts -> int64 exclusive scan -> fill at the per-query cursor.
 
 #include <algorithm>
-#include <type_traits>
 
 #include "internal.h"
 #include "scan.cuh"
@@ -130,39 +129,83 @@ template <> struct PairConst<float> {
     static constexpr float eps = 1.0f / (1 << 19);  // 32 u
     static constexpr float shell = 1.0f / (1 << 11);
     static constexpr float slack = 1.0f / (1 << 20);
+    static constexpr float place = 1.0f / (1 << 20);  // rounding of a box's middle against its coordinates
     static constexpr float tiny = 1e-30f, huge = 1e36f, far = 1e38f;
 };
 template <> struct PairConst<double> {
     static constexpr double eps = 1.0 / (1ULL << 48);  // 32 u
     static constexpr double shell = 1.0 / (1 << 11);
-    static constexpr double slack = 1.0 / (1 << 20);
+    static constexpr double slack = 1.0 / (1 << 15);  // also the slack of QueryBox
+    static constexpr double place = 1.0 / (1ULL << 48);
     static constexpr double tiny = 1e-290, huge = 1e290, far = 1e300;
 };
 
-// Whether the boxes (or points: lo == hi) are near enough for pairs within r:
-// the per-axis gaps, squared and summed in float by fused multiply-adds,
-// against lim = r2 (1 + 2^-20) + tiny.  A pair of points inside with d2 <= r2
-// has per-axis gaps of at most its own differences, and the roundings of the
-// two sums (4 u each) are far inside the bound's slack, so no such pair is
-// lost.
-__device__ __forceinline__ float max3(float a, float b, float c) {
-    float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
 __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
-template <int D>
-__device__ __forceinline__ bool boxes_near(const float* qlo, const float* qhi, const float* lo, const float* hi,
-                                           float lim) {
-    float acc = 0.f;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-        const float g = max3(__fsub_rn(lo[d], qhi[d]), __fsub_rn(qlo[d], hi[d]), 0.f);
-        acc = d == 0 ? __fmul_rn(g, g) : __fmaf_rn(g, g, acc);
-    }
-    return acc <= lim;
+// max(a, b, 0)
+__device__ __forceinline__ float gap(float a, float b) {
+    float d;
+    asm("max.f32 %0, %1, %2, 0f00000000;" : "=f"(d) : "f"(a), "f"(b));
+    return d;
 }
+
+// The box of a warp's queries against the search's boxes and target points.
+// No pair within r is lost; how near the rest may be decides only the work.
+template <class T, int D> struct QueryBox;
+
+// Float32: per-axis gaps of the coordinates, squared and summed by fused
+// multiply-adds, against lim = r2 (1 + 2^-20) + 7 subnormals.  A pair of points
+// inside with d2 <= r2 has per-axis gaps of at most its own differences, and
+// the roundings of the two sums (4 u each, and less than a subnormal per
+// square) are far inside the bound's slack.
+template <int D> struct QueryBox<float, D> {
+    float lo[D], hi[D], lim;
+    __device__ __forceinline__ bool near(const float* blo, const float* bhi) const {
+        float acc = 0.f;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            const float g = gap(__fsub_rn(blo[d], hi[d]), __fsub_rn(lo[d], bhi[d]));
+            acc = d == 0 ? __fmul_rn(g, g) : __fmaf_rn(g, g, acc);
+        }
+        return acc <= lim;
+    }
+    __device__ __forceinline__ bool near(const BoxNode<float, D>& nd) const { return near(nd.lo, nd.hi); }
+    __device__ __forceinline__ bool near_point(const float* x, const float*) const { return near(x, x); }
+};
+
+// Float64: gaps of the fixed-point boxes (BoxUnits) in integers.  For a pair
+// within r, with u = (x - o) s rounded to 2^-21 at most, two floors differ by
+// less than |u_t - u_q| + 1 <= r s + 1 on an axis; lo and hi hold the queries'
+// extremes less and plus that 1, so the squared gaps sum to less than
+// (r s)^2 + 1 = lim (lim's extra 1 covers the 2^-21).  A gap is cut at 2^15,
+// above any r s, which keeps the sum below 2^32.
+//
+// A target point is tested by its offset from the box's middle, which the pair
+// test needs anyway, in radii and Float32 (`half` has room for its rounding).
+template <int D> struct QueryBox<double, D> {
+    int32_t lo[D], hi[D];
+    unsigned lim;
+    float half[D];
+    double per_r;  // 1 / r
+    __device__ __forceinline__ bool near(const BoxNode<double, D>& nd) const {
+        unsigned acc = 0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            const unsigned g = min(__vimax3_s32(nd.lo[d] - hi[d], lo[d] - nd.hi[d], 0), 1 << 15);
+            acc += g * g;
+        }
+        return acc <= lim;
+    }
+    __device__ __forceinline__ bool near_point(const double*, const double* x) const {
+        float acc = 0.f;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            const float g = fmaxf(__fsub_rn(fabsf((float)__dmul_rn(x[d], per_r)), half[d]), 0.f);
+            acc = d == 0 ? __fmul_rn(g, g) : __fmaf_rn(g, g, acc);
+        }
+        return acc <= 1.f + 0x1p-16f;
+    }
+};
 
 // Bits of the targets (those of `keep`) within the radius of query q; sx[d] =
 // the targets' coordinates.
@@ -282,8 +325,9 @@ __device__ __forceinline__ unsigned pairs_fast(const double (*sx)[32], unsigned 
 // position of query point i (when given), which the fill reads.
 template <class T, int D, int PASS>
 __global__ void __launch_bounds__(kEdgeThreads, kEdgeBlocks<T>) k_edges(
-    const SPt<T, D>* __restrict__ qpts, const TNode<float, D>* __restrict__ qchunks, int64_t n_groups,
-    const __grid_constant__ Bvh<D> bv, const SPt<T, D>* __restrict__ tpts, int64_t n_targets, T r2, T inv_r, int exclude_self,
+    const SPt<T, D>* __restrict__ qpts, const BoxNode<T, D>* __restrict__ qchunks, int64_t n_groups,
+    const __grid_constant__ Bvh<T, D> bv, const __grid_constant__ BoxUnits bu, const SPt<T, D>* __restrict__ tpts,
+    int64_t n_targets, T r2, T inv_r, int exclude_self,
     int32_t* __restrict__ counts, int32_t* __restrict__ qpos_of, const int64_t* __restrict__ offsets,
     int32_t* __restrict__ senders, int32_t* __restrict__ receivers, T* __restrict__ rdisp, T* __restrict__ rdist,
     int* __restrict__ ocount, int2* __restrict__ recs, int64_t rec_cap, uint16_t* __restrict__ rcount,
@@ -308,37 +352,74 @@ __global__ void __launch_bounds__(kEdgeThreads, kEdgeBlocks<T>) k_edges(
     const int64_t g = (int64_t)blockIdx.x * kEdgeWarps + w;
     if (g >= n_groups) return;  // warp-uniform
     if (PASS == EP_FILL && recs != nullptr && gflag[g] == 0) return;  // expanded from its records
-    TNode<float, D> gc = qchunks[g];
+    const BoxNode<T, D> gc = qchunks[g];
     const bool valid = lane < gc.b;
     const int64_t qpos = gc.a + (valid ? lane : 0);  // position of this lane's query
     const SPt<T, D> q = qpts[qpos];
     // A batch searches each cloud in its own positions with its own radius and
     // reports cloud-local indices.
-    int32_t base = 0;
+    int32_t base = 0, cloud = 0;
     int32_t plo = 0, phi = (int32_t)n_targets;
     if (bt.n_clouds) {
-        const int c = cloud_of_position(bt, gc.a);
-        const double* cp = bt.cparam + (size_t)c * kCloudParams;
+        cloud = cloud_of_position(bt, gc.a);
+        const double* cp = bt.cparam + (size_t)cloud * kCloudParams;
         r2 = (T)cp[4];
         inv_r = (T)cp[5];
-        base = plo = (int32_t)bt.coff[c];
-        phi = (int32_t)bt.coff[c + 1];
+        base = plo = (int32_t)bt.coff[cloud];
+        phi = (int32_t)bt.coff[cloud + 1];
     }
-    // The fast pair test's constants (see pairs_fast).
+    // The queries' box and the fast pair test's constants (see pairs_fast).
     using PC = PairConst<T>;
-    const float lim = float_above(r2 * (T(1) + PC::slack)) + 1e-44f;
-    T ctr[D], m2q[D], off, eps;
-    bool fast;
+    QueryBox<T, D> qb;
+    T ctr[D], m2q[D], off, eps;  // ctr: the middle of the queries' box
+    bool fast = r2 >= PC::tiny;
     {
         const T r = sqrt_near(r2) * (T(1) + PC::slack);
+        T h[D];  // |x - ctr| of a query is no more
+        if constexpr (sizeof(T) == 4) {
+            qb.lim = r2 * (T(1) + PC::slack) + 1e-44f;
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                qb.lo[d] = gc.lo[d];
+                qb.hi[d] = gc.hi[d];
+                const T half = T(0.5) * (gc.hi[d] - gc.lo[d]);
+                ctr[d] = gc.lo[d] + half;
+                h[d] = half * (T(1) + PC::slack) + fabs(ctr[d]) * PC::place;
+            }
+        } else {
+            BoxUnits un = bu;
+            if (bt.n_clouds) {
+                un = cloud_units(bt, cloud);
+                un.width = div_rn(1.0, un.s);
+            }
+            const T half_unit = T(0.5) * un.width, half_more = half_unit * (T(1) + PC::slack);
+            qb.lim = (un.mul > 1.0 ? (unsigned)(un.mul * un.mul) : 1u) + 1u;
+            qb.per_r = un.s / un.mul;
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                // The box in the target's units: another query set's from its
+                // points, cut at +-kFar (beyond that no target is near, and the
+                // fast test's bounds do not hold).
+                constexpr int32_t kFar = (1 << 30) - 1;
+                int32_t lo = gc.lo[d], hi = gc.hi[d];
+                if (qchunks != bv.chunk) {
+                    const int32_t u = min(max(box_coord(q.x[d], d, un), -kFar), kFar);
+                    lo = box_min(u);
+                    hi = box_max(u);
+                    fast = fast && lo > -kFar && hi < kFar;
+                }
+                qb.lo[d] = lo - 1;
+                qb.hi[d] = hi + 1;
+                ctr[d] = fma_rn((T)(lo + hi + 1), half_unit, un.o[d]);
+                h[d] = fma_rn((T)(hi - lo + 1), half_more, (fabs(ctr[d]) + fabs(un.o[d])) * PC::place);
+                qb.half[d] = __fmaf_rn(__double2float_ru(h[d] * qb.per_r), 1.f + 0x1p-20f, 0x1p-20f);
+            }
+        }
         T qq = T(0), tt = T(0), qn = T(0);
 #pragma unroll
         for (int d = 0; d < D; ++d) {
-            const T half = T(0.5) * ((T)gc.hi[d] - (T)gc.lo[d]);
-            ctr[d] = (T)gc.lo[d] + half;
-            const T h = half * (T(1) + PC::slack) + fabs(ctr[d]) * PC::slack;
-            qq += h * h;
-            tt += (h + r) * (h + r);
+            qq += h[d] * h[d];
+            tt += (h[d] + r) * (h[d] + r);
             const T x = q.x[d] - ctr[d];
             m2q[d] = T(-2) * x;
             qn += x * x;
@@ -346,16 +427,7 @@ __global__ void __launch_bounds__(kEdgeThreads, kEdgeBlocks<T>) k_edges(
         const T S = T(2) * (qq + tt) + r2;
         eps = PC::eps * S;
         off = valid ? qn - r2 : PC::far;  // a lane without a query hits nothing
-        fast = eps <= PC::shell * r2 && r2 >= PC::tiny && S <= PC::huge;  // false for a NaN
-    }
-    if constexpr (!std::is_same<T, float>::value) {
-        // room for the rounding of a Float64 target's coordinates to float
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-            const float pad = (fmaxf(fabsf(gc.lo[d]), fabsf(gc.hi[d])) + sqrt_near(lim)) * 0x1p-22f;
-            gc.lo[d] -= pad;
-            gc.hi[d] += pad;
-        }
+        fast = fast && eps <= PC::shell * r2 && S <= PC::huge;  // false for a NaN
     }
     int32_t cnt = 0;
     int64_t cur = 0, cur_end = 0;
@@ -407,10 +479,10 @@ __global__ void __launch_bounds__(kEdgeThreads, kEdgeBlocks<T>) k_edges(
         if constexpr (STATS) st_c0 = clock64();
         // A target farther than r from the group's box can be no query's
         // neighbor: the pair loop skips the steps whose targets all are.
-        float xf[D];
+        T x[D];
 #pragma unroll
-        for (int d = 0; d < D; ++d) xf[d] = (float)t.x[d];
-        const bool near = lane < num && boxes_near<D>(gc.lo, gc.hi, xf, xf, lim);
+        for (int d = 0; d < D; ++d) x[d] = t.x[d] - ctr[d];
+        const bool near = lane < num && qb.near_point(t.x, x);
         const unsigned keep = __ballot_sync(FULL, near);
         if (keep == 0) return;
         long long st_p0 = 0;
@@ -423,10 +495,10 @@ __global__ void __launch_bounds__(kEdgeThreads, kEdgeBlocks<T>) k_edges(
         unsigned hm = 0;
         bool exact = !fast;
         if (fast) {
-            T x[D], tt = T(0);
+            T tt = T(0);
 #pragma unroll
             for (int d = 0; d < D; ++d) {
-                x[d] = near ? t.x[d] - ctr[d] : T(0);
+                if (!near) x[d] = T(0);
                 tt = d == 0 ? x[d] * x[d] : fma_rn(x[d], x[d], tt);
             }
             if (!near) tt = PC::far;
@@ -477,8 +549,8 @@ __global__ void __launch_bounds__(kEdgeThreads, kEdgeBlocks<T>) k_edges(
         const int32_t i = b0 + lane;
         bool pass = false;
         if (i < end) {
-            const TNode<float, D> nd = bv.lev[l][i];
-            pass = boxes_near<D>(gc.lo, gc.hi, nd.lo, nd.hi, lim);
+            const BoxNode<T, D> nd = bv.lev[l][i];
+            pass = qb.near(nd);
             if (l == 0) {
                 na = nd.a;
                 nb = nd.b;
@@ -524,8 +596,8 @@ __global__ void __launch_bounds__(kEdgeThreads, kEdgeBlocks<T>) k_edges(
             int32_t first = 0, num = 0;
             bool pass = false;
             if (cb + lane < nc) {
-                const TNode<float, D> nd = bv.chunk[c0 + cb + lane];
-                pass = boxes_near<D>(gc.lo, gc.hi, nd.lo, nd.hi, lim) && nd.a >= plo && nd.a < phi;
+                const BoxNode<T, D> nd = bv.chunk[c0 + cb + lane];
+                pass = qb.near(nd) && nd.a >= plo && nd.a < phi;
                 first = nd.a;
                 num = nd.b;
             }
@@ -1187,7 +1259,7 @@ int count_typed(Ctx& ctx, const Tree& q, const Tree& t, bool exclude_self, int64
         const int64_t ng = q.n_groups;
         const auto kern = ctx.rec_cap ? k_edges<T, D, EP_RECORD> : k_edges<T, D, EP_COUNT>;
         launch_pdl(kern, div_up(ng, kEdgeWarps), kEdgeThreads, 0, s, q.dpts.as<SPt<T, D>>(),
-            q.chunk.as<TNode<float, D>>(), ng, t.search_layout<D>(), t.dpts.as<SPt<T, D>>(), t.n, r2, T(0),
+            q.chunk.as<BoxNode<T, D>>(), ng, t.search_layout<T, D>(), t.box_units(), t.dpts.as<SPt<T, D>>(), t.n, r2, T(0),
             exclude_self ? 1 : 0, ctx.counts.as<int32_t>(), ctx.qpos.as<int32_t>(), nullptr, nullptr, nullptr, nullptr,
             nullptr, (int*)(ctx.total.as<int64_t>() + 1), ctx.rec_cap ? ctx.recs.as<int2>() : nullptr, ctx.rec_cap,
             ctx.rcount.as<uint16_t>(), ctx.gflag.as<uint8_t>(), t.batch(), nullptr);
@@ -1287,7 +1359,7 @@ int fill_typed(Ctx& ctx, const Tree& q, const Tree& t, bool exclude_self, int32_
     if (!ctx.rec_cap || ctx.rec_overflow) {
         // Groups without complete records walk the tree again.
         k_edges<T, D, EP_FILL><<<div_up(ng, kEdgeWarps), kEdgeThreads, 0, s>>>(
-            q.dpts.as<SPt<T, D>>(), q.chunk.as<TNode<float, D>>(), ng, t.search_layout<D>(), t.dpts.as<SPt<T, D>>(),
+            q.dpts.as<SPt<T, D>>(), q.chunk.as<BoxNode<T, D>>(), ng, t.search_layout<T, D>(), t.box_units(), t.dpts.as<SPt<T, D>>(),
             t.n, r2, inv_r, exclude_self ? 1 : 0, nullptr, nullptr, ctx.offsets.as<int64_t>(), senders, receivers,
             (T*)rel_disp, (T*)rel_dist, ctx.dstatus.as<int>(), ctx.rec_cap ? ctx.recs.as<int2>() : nullptr,
             ctx.rec_cap, nullptr, ctx.gflag.as<uint8_t>(), t.batch(), nullptr);
@@ -1313,7 +1385,7 @@ cudaError_t count_into_typed(const Tree& q, const Tree& t, bool exclude_self, in
     const T r = (T)t.radius;
     const T r2 = r * r;
     k_edges<T, D, EP_COUNT><<<div_up(q.n_groups, kEdgeWarps), kEdgeThreads, 0, s>>>(
-        q.dpts.as<SPt<T, D>>(), q.chunk.as<TNode<float, D>>(), q.n_groups, t.search_layout<D>(),
+        q.dpts.as<SPt<T, D>>(), q.chunk.as<BoxNode<T, D>>(), q.n_groups, t.search_layout<T, D>(), t.box_units(),
         t.dpts.as<SPt<T, D>>(), t.n, r2, T(0), exclude_self ? 1 : 0, counts, nullptr, nullptr, nullptr, nullptr,
         nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, t.batch(), nullptr);
     return cudaGetLastError();
@@ -1324,7 +1396,7 @@ int stats_typed(Ctx& ctx, const Tree& q, const Tree& t, bool exclude_self, unsig
     const T r = (T)t.radius;
     const T r2 = r * r;
     k_edges<T, D, EP_STATS><<<div_up(q.n_groups, kEdgeWarps), kEdgeThreads, 0, ctx.stream>>>(
-        q.dpts.as<SPt<T, D>>(), q.chunk.as<TNode<float, D>>(), q.n_groups, t.search_layout<D>(),
+        q.dpts.as<SPt<T, D>>(), q.chunk.as<BoxNode<T, D>>(), q.n_groups, t.search_layout<T, D>(), t.box_units(),
         t.dpts.as<SPt<T, D>>(), t.n, r2, T(0), exclude_self ? 1 : 0, ctx.counts.as<int32_t>(), nullptr, nullptr,
         nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, t.batch(), stats_dev);
     ctx.kernel_launches += 1;

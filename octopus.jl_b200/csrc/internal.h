@@ -100,6 +100,7 @@ struct Tree {
     int64_t capacity = 0;    // node capacity of the node arrays
     int n_mark_blocks = 0;
     double origin[3] = {0, 0, 0};
+    double mul = 1.0;        // BoxUnits::mul (Float64 boxes)
 
     // Device storage.
     DevBuf keys[2], vals[2];     // radix-sort ping-pong
@@ -129,9 +130,9 @@ struct Tree {
     // Search layout (Bvh): what build_edges reads.
     DevBuf dpts;                 // SPt<T,D>[n] in the search's visiting order
     DevBuf dstart;               // uint8 per visiting position: point count of the chunk starting there, else 0
-    DevBuf dnode, rbox;          // a run's first leaf (int32, at its start) and its box (TNode<float,D> at that leaf)
-    DevBuf chunk;                // TNode<float,D> per chunk: box, first position, count <= group_cap
-    DevBuf bvh;                  // TNode<float,D>: the box hierarchy's levels, one after another
+    DevBuf dnode, rbox;          // a run's first leaf (int32, at its start) and its box (BoxNode<T,D> at that leaf)
+    DevBuf chunk;                // BoxNode<T,D> per chunk: box, first position, count <= group_cap
+    DevBuf bvh;                  // BoxNode<T,D>: the box hierarchy's levels, one after another
     DevBuf bvh_arrive;           // int32 per node above the lowest level: children done
     int64_t n_groups = 0;        // chunks
     int32_t asc_key = 0;         // OctHeader::asc_key of the last topology
@@ -165,7 +166,17 @@ struct Tree {
         b.kbits = kbits;
         b.coff = b_coff.as<int64_t>();
         b.cparam = b_cparam.as<double>();
+        b.mul = mul;
         return b;
+    }
+    // Box units of a single Float64 set, as the build's kernels derive them.
+    BoxUnits box_units() const {
+        BoxUnits u{};
+        for (int d = 0; d < ndims; ++d) u.o[d] = origin[d];
+        u.s = (1.0 / radius) * mul;
+        u.width = 1.0 / u.s;
+        u.mul = mul;
+        return u;
     }
     // The box hierarchy's shape for n points: level sizes, and their sum.
     static int32_t bvh_levels(int64_t n, int32_t* cnt, int64_t* total) {
@@ -178,12 +189,12 @@ struct Tree {
         }
         return top;
     }
-    template <int D> Bvh<D> search_layout() const {
-        Bvh<D> b;
+    template <class T, int D> Bvh<T, D> search_layout() const {
+        Bvh<T, D> b;
         int64_t total = 0;
         b.top = bvh_levels(n, b.cnt, &total);
-        b.chunk = chunk.as<TNode<float, D>>();
-        TNode<float, D>* p = bvh.as<TNode<float, D>>();
+        b.chunk = chunk.as<BoxNode<T, D>>();
+        BoxNode<T, D>* p = bvh.as<BoxNode<T, D>>();
         for (int l = 0; l <= b.top; ++l) {
             b.lev[l] = p;
             p += b.cnt[l];
