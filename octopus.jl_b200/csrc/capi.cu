@@ -21,10 +21,12 @@ namespace {
 // device, for the next allocation of about that size: a new tree takes some
 // thirty buffers, and allocating them afresh costs more than building and
 // searching it (100,000 points: 1.7 ms for a first pass, 0.3 ms with the
-// blocks of an earlier tree).  A block enters only after a device
-// synchronize, which cudaFree would make too, so whichever stream or thread
-// takes it next finds no work on it.  At most kPoolBytes are held per device;
-// the rest is freed, everything is when the device's last context is
+// blocks of an earlier tree).  A block enters only when the work that used it
+// is known to be done (all on one stream, which was waited for), so whichever
+// stream or thread takes it next finds no work on it; the others are freed,
+// which waits for their work.  Nothing here waits for the whole device: that
+// would invalidate any capture in progress.  At most kPoolBytes are held per
+// device; the rest is freed, everything is when the device's last context is
 // destroyed or an allocation fails.
 constexpr size_t kPoolBytes = 4ULL << 30;
 constexpr int kPoolDevices = 64;
@@ -81,7 +83,7 @@ cudaError_t block_alloc(size_t least, size_t want, DevBuf& b) {
     return e;
 }
 
-// `idle`: the device has been synchronized since the block's last use.
+// `idle`: the work that used the block is done.
 void block_free(DevBuf& b, bool idle) {
     if (!b.p) return;
     BlockPool* pool = idle ? pool_of_current_device() : nullptr;
@@ -104,9 +106,25 @@ void block_free(DevBuf& b, bool idle) {
 
 }  // namespace
 
-// Whether the device could be waited for (not while a stream is captured).
-bool device_idle() {
-    if (cudaDeviceSynchronize() == cudaSuccess) return true;
+void UsedStream::note(cudaStream_t s) {
+    unsigned long long now = kSeveral, none = kNone;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone ||
+        cudaStreamGetId(s, &now) != cudaSuccess) {
+        (void)cudaGetLastError();  // the call that follows reports what is wrong with the stream
+        now = kSeveral;
+    }
+    if (!id.compare_exchange_strong(none, now) && none != now) id.store(kSeveral);
+}
+
+bool UsedStream::wait(cudaStream_t s) const {
+    const unsigned long long was = id.load();
+    if (was == kNone || was == kSeveral) return was == kNone;
+    unsigned long long now = kSeveral;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamGetId(s, &now) == cudaSuccess && now == was && cudaStreamIsCapturing(s, &cs) == cudaSuccess &&
+        cs == cudaStreamCaptureStatusNone && cudaStreamSynchronize(s) == cudaSuccess)
+        return true;
     (void)cudaGetLastError();
     return false;
 }
@@ -115,9 +133,10 @@ cudaError_t ensure(DevBuf& b, size_t bytes) {
     if (bytes == 0) bytes = 16;
     if (b.bytes >= bytes) return cudaSuccess;
     if (b.p) {
-        const cudaError_t e = cudaDeviceSynchronize();
+        const cudaError_t e = cudaFree(b.p);
         if (e != cudaSuccess) return e;
-        block_free(b, true);
+        b.p = nullptr;
+        b.bytes = 0;
     }
     return block_alloc(bytes, bytes + bytes / 8, b);  // slack so slowly growing inputs do not reallocate every call
 }
@@ -153,9 +172,9 @@ cudaError_t header_alloc(OctHeader** h) {
     return cudaMallocHost((void**)h, kHeaderBytes);
 }
 
-void header_free(OctHeader* h) {
+void header_free(OctHeader* h, bool idle) {
     if (!h) return;
-    if (BlockPool* pool = pool_of_current_device()) {
+    if (BlockPool* pool = idle ? pool_of_current_device() : nullptr) {
         std::lock_guard<std::mutex> lock(pool->mu);
         if (pool->contexts > 0 && pool->headers.size() < kHeaders) {
             try {
@@ -302,17 +321,20 @@ struct DeviceGuard {
     }
 };
 
-void release_tree(oct::Tree& t) {
-    const bool idle = oct::device_idle();  // its buffers may go to another tree, on another stream
+void release_tree(oct::Tree& t, const oct::Ctx* owner) {
+    // its buffers may go to another tree, on another stream
+    const bool idle = owner && t.used.wait(owner->stream);
     using oct::release;
+    // the caller's own kernels may be reading the views, on any stream
+    for (auto* b : {&t.morton, &t.v_first, &t.v_last, &t.v_children, &t.v_bmin, &t.v_bmax, &t.v_perm})
+        release(*b, false);
     for (auto* b : {&t.b_coff, &t.b_cparam, &t.b_cbounds, &t.b_eoff})
         release(*b, idle);
     for (auto* b : {&t.keys[0], &t.keys[1], &t.vals[0], &t.vals[1], &t.hist, &t.sort_tmp, &t.look, &t.spts, &t.spts_tmp, &t.tnode, &t.nrange,
                     &t.link, &t.fchild, &t.arrive, &t.dpts, &t.dstart, &t.dnode, &t.rbox, &t.chunk, &t.bvh, &t.bvh_arrive, &t.lohi, &t.blockcnt, &t.blockoff, &t.scan_tmp, &t.partials, &t.hdr,
-                    &t.morton, &t.v_first, &t.v_last, &t.v_children, &t.v_bmin, &t.v_bmax, &t.v_perm, &t.iperm,
-                    &t.rflag, &t.rcnt, &t.roff, &t.mkeys, &t.mvals, &t.mkeys2, &t.mvals2})
+                    &t.iperm, &t.rflag, &t.rcnt, &t.roff, &t.mkeys, &t.mvals, &t.mkeys2, &t.mvals2})
         release(*b, idle);
-    oct::header_free(t.hdr_host);
+    oct::header_free(t.hdr_host, idle);
     t.hdr_host = nullptr;
 }
 
@@ -361,12 +383,12 @@ OCT_API int oct_ctx_create(int device, oct_ctx** out) {
 OCT_API int oct_ctx_destroy(oct_ctx* ctx) {
     if (!ctx) return OCT_OK;
     DeviceGuard g(ctx->c.device);
-    const bool idle = oct::device_idle();
+    cudaStreamSynchronize(ctx->c.stream);
     using oct::release;
     for (auto* b : {&ctx->c.counts, &ctx->c.qpos, &ctx->c.offsets, &ctx->c.scan_tmp, &ctx->c.total, &ctx->c.dkeys[0],
                     &ctx->c.dkeys[1], &ctx->c.dvals[0], &ctx->c.dvals[1], &ctx->c.dhist, &ctx->c.dsort_tmp, &ctx->c.droff,
                     &ctx->c.dsoff, &ctx->c.dstatus, &ctx->c.dredge, &ctx->c.dterm, &ctx->c.dseg, &ctx->c.tstats, &ctx->c.recs, &ctx->c.rcount, &ctx->c.gflag})
-        release(*b, idle);
+        release(*b, false);
     if (ctx->c.total_host) cudaFreeHost(ctx->c.total_host);
     for (auto& r : ctx->c.prof) {
         cudaEventDestroy(r.start);
@@ -417,7 +439,7 @@ OCT_API int oct_tree_destroy(oct_tree* tree) {
     if (!tree) return OCT_OK;
     {
         DeviceGuard g(tree->owner ? tree->owner->c.device : 0);
-        release_tree(tree->t);
+        release_tree(tree->t, tree->owner ? &tree->owner->c : nullptr);
     }
     delete tree;
     return OCT_OK;
@@ -433,6 +455,7 @@ OCT_API int oct_tree_build(oct_ctx* ctx, oct_tree* tree, const void* coords, int
     if (n > 0 && !coords) return oct::set_error(ctx->c, OCT_ERR_ARGUMENT, "coords is NULL");
     DeviceGuard g(ctx->c.device);
     tree->t.keep_morton = keep_morton != 0;
+    tree->t.used.note(ctx->c.stream);
     return oct::build_tree(ctx->c, tree->t, coords, n, radius);
 }
 
@@ -453,6 +476,7 @@ OCT_API int oct_tree_build_batch(oct_ctx* ctx, oct_tree* tree, const void* coord
     }
     if (n > 0 && !coords) return oct::set_error(ctx->c, OCT_ERR_ARGUMENT, "coords is NULL");
     DeviceGuard g(ctx->c.device);
+    tree->t.used.note(ctx->c.stream);
     return oct::build_tree_batch(ctx->c, tree->t, coords, n, cloud_offsets, radii, n_clouds);
 }
 
@@ -462,6 +486,7 @@ OCT_API int oct_batch_edge_offsets(oct_ctx* ctx, oct_tree* tree, int64_t* edge_o
     if (!tree->t.built || tree->t.n_clouds < 1)
         return oct::set_error(ctx->c, OCT_ERR_STATE, "batch edge offsets: the tree is not a built batch");
     DeviceGuard g(ctx->c.device);
+    tree->t.used.note(ctx->c.stream);
     return oct::batch_edge_offsets(ctx->c, tree->t, edge_offsets);
 }
 
@@ -488,6 +513,7 @@ OCT_API int oct_tree_view_get(oct_ctx* ctx, oct_tree* tree, oct_tree_view* out) 
     if (!t.built) return oct::set_error(ctx->c, OCT_ERR_STATE, "tree has not been built (call run! first)");
     if (t.n_clouds > 0) return oct::set_error(ctx->c, OCT_ERR_STATE, "a batched tree has no single-tree view");
     DeviceGuard g(ctx->c.device);
+    t.used.note(ctx->c.stream);
     const int st = oct::materialize_view(ctx->c, t);
     if (st != OCT_OK) return st;
     out->n_points = t.n;
@@ -500,6 +526,11 @@ OCT_API int oct_tree_view_get(oct_ctx* ctx, oct_tree* tree, oct_tree_view* out) 
     out->perm = t.v_perm.as<int32_t>();
     out->morton = (t.keep_morton && t.n > 0) ? t.morton.as<uint64_t>() : nullptr;
     return OCT_OK;
+}
+
+static void note_pair(const oct_ctx* ctx, const oct_tree* query, const oct_tree* target) {
+    query->t.used.note(ctx->c.stream);
+    if (target != query) target->t.used.note(ctx->c.stream);
 }
 
 static int check_pair(oct_ctx* ctx, const oct_tree* query, const oct_tree* target) {
@@ -533,6 +564,7 @@ OCT_API int oct_edges_count(oct_ctx* ctx, const oct_tree* query, const oct_tree*
     const int st = oct_check_count_pair(ctx, query, target, exclude_self);
     if (st != OCT_OK) return st;
     DeviceGuard g(ctx->c.device);
+    note_pair(ctx, query, target);
     return oct::edges_count(ctx->c, query->t, target->t, exclude_self != 0, n_edges);
 }
 
@@ -543,6 +575,7 @@ OCT_API int oct_edges_traversal_stats(oct_ctx* ctx, const oct_tree* query, const
     const int st = oct_check_count_pair(ctx, query, target, exclude_self);
     if (st != OCT_OK) return st;
     DeviceGuard g(ctx->c.device);
+    note_pair(ctx, query, target);
     return oct::traversal_stats(ctx->c, query->t, target->t, exclude_self != 0, stats, n_stats);
 }
 
@@ -556,6 +589,7 @@ OCT_API int oct_edges_fill(oct_ctx* ctx, const oct_tree* query, const oct_tree* 
     if (capacity > 0 && (!senders || !receivers || !rel_displacement || !rel_dist_norm))
         return oct::set_error(ctx->c, OCT_ERR_ARGUMENT, "edge output buffer is NULL");
     DeviceGuard g(ctx->c.device);
+    note_pair(ctx, query, target);
     return oct::edges_fill(ctx->c, query->t, target->t, exclude_self != 0, senders, receivers, rel_displacement,
                            rel_dist_norm, capacity);
 }
@@ -569,6 +603,7 @@ OCT_API int oct_edges_fill_diff(oct_ctx* ctx, const oct_tree* tree, int32_t* sen
     if (capacity > 0 && (!senders || !receivers || !rel_displacement || !rel_dist_norm || !mirror))
         return oct::set_error(ctx->c, OCT_ERR_ARGUMENT, "edge output buffer is NULL");
     DeviceGuard g(ctx->c.device);
+    note_pair(ctx, tree, tree);
     return oct::edges_fill_diff(ctx->c, tree->t, senders, receivers, rel_displacement, rel_dist_norm, mirror,
                                 capacity);
 }
@@ -582,6 +617,7 @@ OCT_API int oct_csr_fill(oct_ctx* ctx, const oct_tree* query, const oct_tree* ta
     if (!offsets || (capacity > 0 && !flat))
         return oct::set_error(ctx->c, OCT_ERR_ARGUMENT, "neighbor list output buffer is NULL");
     DeviceGuard g(ctx->c.device);
+    note_pair(ctx, query, target);
     return oct::csr_fill(ctx->c, query->t, target->t, exclude_self != 0, offsets, flat, capacity);
 }
 
@@ -590,6 +626,7 @@ OCT_API int oct_zsort_apply(oct_ctx* ctx, const oct_tree* tree, const void* in, 
     if (!ctx || !tree) return OCT_ERR_ARGUMENT;
     ctx->c.last_error.clear();
     DeviceGuard g(ctx->c.device);
+    tree->t.used.note(ctx->c.stream);
     return oct::zsort_apply(ctx->c, tree->t, in, out, n, row_bytes, direction);
 }
 
@@ -611,6 +648,7 @@ OCT_API int oct_neighbors(oct_ctx* ctx, const oct_tree* target, const void* quer
     if (!target->t.built) return oct::set_error(ctx->c, OCT_ERR_STATE, "target tree has not been built");
     if (target->t.n_clouds > 0) return oct::set_error(ctx->c, OCT_ERR_STATE, "neighbor queries need a single-set tree");
     DeviceGuard g(ctx->c.device);
+    target->t.used.note(ctx->c.stream);
     return oct::neighbors_of(ctx->c, target->t, query_coords, n_queries, out_counts, out_indices, cap_per_query);
 }
 

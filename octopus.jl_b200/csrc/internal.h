@@ -1,6 +1,7 @@
 // Library-internal objects shared by the build, edge and C-ABI translation units.
 #pragma once
 
+#include <atomic>
 #include <chrono>
 #include <cstdint>
 #include <string>
@@ -19,12 +20,11 @@ struct DevBuf {
 };
 
 cudaError_t ensure(DevBuf& b, size_t bytes);
-void release(DevBuf& b, bool idle);  // idle: the device was synchronized since its last use
-bool device_idle();
+void release(DevBuf& b, bool idle);  // idle: the work that used it is known to be done
 // A tree's pinned header block, and the number of contexts on the current
 // device (the device's pool is emptied with the last).
 cudaError_t header_alloc(OctHeader** h);
-void header_free(OctHeader* h);
+void header_free(OctHeader* h, bool idle);
 void pool_context(int delta);
 
 struct Ctx;
@@ -79,6 +79,18 @@ struct PhaseTimer {
     ~PhaseTimer();
 };
 
+// The stream whose work has used an object's buffers, by its id (an id is
+// never given twice, unlike a handle): none, one, or several.  A stream that
+// was being captured counts as several, since the graph may run on any.
+struct UsedStream {
+    static constexpr unsigned long long kNone = ~0ULL, kSeveral = ~0ULL - 1;
+    std::atomic<unsigned long long> id{kNone};
+    void note(cudaStream_t s);
+    // Waits for the work if it was all on `s`; false when that is not known
+    // (nothing is waited for then, nor on a stream being captured).
+    bool wait(cudaStream_t s) const;
+};
+
 // One point set's search structure (the reference's Octree + permutation +
 // morton_codes, src/types.jl:23-42 and src/types.jl:153-154).
 struct Tree {
@@ -90,6 +102,7 @@ struct Tree {
     int32_t group_cap = 32;  // query points per traversal group of the last build
     bool built = false;
     bool keep_morton = false;
+    mutable UsedStream used;
     uint64_t generation = 0;
 
     // Build results (host copies, valid after a successful build).

@@ -99,6 +99,8 @@ extern "C" OCT_API int oct_edges_count_noalloc(oct_ctx* ctx, const oct_tree* que
     int64_t* scratch = nullptr;
     e = scratch_address(c.device, &scratch);
     if (e != cudaSuccess) return oct::cuda_status(c, e, "cudaGetSymbolAddress(scan scratch)");
+    q.used.note(c.stream);
+    t.used.note(c.stream);
     if ((e = oct::count_into(q, t, exclude_self != 0, counts, c.stream)) != cudaSuccess)
         return oct::cuda_status(c, e, "edge count launch");
     oct::exclusive_scan_i32_i64(counts, offsets, q.n, scratch + kNoAllocTiles, scratch, c.stream);
