@@ -75,6 +75,12 @@ OCT_API const char* oct_status_string(int status);
 OCT_API int oct_ctx_create(int device, oct_ctx** out);
 OCT_API int oct_ctx_destroy(oct_ctx* ctx);
 
+/* Device memory of destroyed trees is kept for the next ones, at most 4 GiB
+ * per device and only while an eighth of the device's memory is free.  This
+ * gives what is held back to the device, for allocations made elsewhere in
+ * the process; the library's own allocations do so by themselves. */
+OCT_API int oct_ctx_release_memory(oct_ctx* ctx);
+
 /* Order all later work after the caller's stream (a cudaStream_t). */
 OCT_API int oct_ctx_set_stream(oct_ctx* ctx, void* stream);
 

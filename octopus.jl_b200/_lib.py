@@ -65,6 +65,7 @@ SIGNATURES = [
     ("oct_status_string", C.c_char_p, [I]),
     ("oct_ctx_create", I, [I, C.POINTER(P)]),
     ("oct_ctx_destroy", I, [P]),
+    ("oct_ctx_release_memory", I, [P]),
     ("oct_ctx_set_stream", I, [P, P]),
     ("oct_ctx_last_error", C.c_char_p, [P]),
     ("oct_synchronize", I, [P]),

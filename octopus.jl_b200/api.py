@@ -112,6 +112,25 @@ def colmajor(x: torch.Tensor) -> torch.Tensor:
     return x.t().contiguous().t()
 
 
+def release_memory(device: int | None = None) -> None:
+    """Give back the device memory that the library keeps of dropped trees (at
+    most 4 GiB per device), for allocations made elsewhere in the process;
+    this package's own allocations do so by themselves."""
+    ctx = _Context._by_device.get(torch.cuda.current_device() if device is None else device)
+    if ctx is not None:
+        ctx.check(ctx.lib.oct_ctx_release_memory(ctx.handle), "release_memory")
+
+
+def _empty(shape, dtype: torch.dtype, device: int) -> torch.Tensor:
+    """torch.empty on a CUDA device, once more after release_memory when the
+    device is out of memory."""
+    try:
+        return torch.empty(shape, dtype=dtype, device=f"cuda:{device}")
+    except torch.OutOfMemoryError:
+        release_memory(device)
+        return torch.empty(shape, dtype=dtype, device=f"cuda:{device}")
+
+
 def _ptr(x: torch.Tensor | None):
     return C.c_void_p(x.data_ptr()) if x is not None and x.numel() > 0 else C.c_void_p(0)
 
@@ -407,13 +426,12 @@ def _reserve_buffer(buf: EdgeBuffer, T, ndims, n_edges, device):
     step."""
     cap = getattr(buf, "_capacity", -1)
     if n_edges > cap:
-        dev = f"cuda:{device}"
         cap = n_edges + n_edges // 4
-        buf._capacity = cap
-        buf._snd = torch.empty(cap, dtype=torch.int32, device=dev)
-        buf._rcv = torch.empty(cap, dtype=torch.int32, device=dev)
-        buf._disp = torch.empty((cap, ndims), dtype=T, device=dev)
-        buf._dist = torch.empty((cap, 1), dtype=T, device=dev)
+        buf._snd = _empty(cap, torch.int32, device)
+        buf._rcv = _empty(cap, torch.int32, device)
+        buf._disp = _empty((cap, ndims), T, device)
+        buf._dist = _empty((cap, 1), T, device)
+        buf._capacity = cap  # (last: an allocation that fails leaves the old capacity)
 
 
 def _resize_buffer(buf: EdgeBuffer, T, ndims, n_edges, device):
@@ -552,8 +570,8 @@ def materialize_all_neighbors_(tns: TNS) -> TNS:
         ctx, qtree, ttree, excl, n = got
         if n > 2**31 - 1:
             raise OctopusError(f"materialize_all_neighbors!: {n} neighbors exceed the Int32 offsets")
-        buf.flat = torch.empty(n, dtype=torch.int32, device=dev)
-        buf.offsets = torch.empty(nq + 1, dtype=torch.int32, device=dev)
+        buf.flat = _empty(n, torch.int32, tns.device)
+        buf.offsets = _empty(nq + 1, torch.int32, tns.device)
         ctx.check(ctx.lib.oct_csr_fill(ctx.handle, qtree.handle, ttree.handle, excl, _ptr(buf.offsets),
                                        _ptr(buf.flat), n), "materialize_all_neighbors!")
         buf.materialized = True
@@ -590,11 +608,10 @@ class _EdgesDiff(torch.autograd.Function):
             lc, qtree, ttree, excl, n_edges = got
             if n_edges > 2**31 - 1:
                 raise OctopusError(f"build_edges_diff: {n_edges} edges exceed the Int32 edge count")
-        dev = f"cuda:{tns.device}"
-        snd = torch.empty(n_edges, dtype=torch.int32, device=dev)
-        rcv = torch.empty(n_edges, dtype=torch.int32, device=dev)
-        disp_rows = torch.empty((n_edges, tns.ndims), dtype=tns.T, device=dev)
-        dist = torch.empty((1, n_edges), dtype=tns.T, device=dev)
+        snd = _empty(n_edges, torch.int32, tns.device)
+        rcv = _empty(n_edges, torch.int32, tns.device)
+        disp_rows = _empty((n_edges, tns.ndims), tns.T, tns.device)
+        dist = _empty((1, n_edges), tns.T, tns.device)
         if n_edges > 0:
             lc.check(lc.lib.oct_edges_fill(lc.handle, qtree.handle, ttree.handle, excl, _ptr(snd), _ptr(rcv),
                                            _ptr(disp_rows), _ptr(dist), n_edges), "build_edges_diff")
@@ -629,8 +646,7 @@ class _EdgesDiff(torch.autograd.Function):
         tns = ctx.tns
         d, n = ctx.coords_shape
         T = tns.T
-        dev = f"cuda:{tns.device}"
-        grad = torch.empty((n, d), dtype=T, device=dev)
+        grad = _empty((n, d), T, tns.device)
         dd = None if g_disp is None else g_disp.t().contiguous()
         dn = None if g_dist is None else g_dist.reshape(-1).contiguous()
         lc = tns._ctx
@@ -675,9 +691,8 @@ class _EdgesDiffPair(torch.autograd.Function):
         tns = ctx.tns
         (d, nq), (_, nt) = ctx.shapes
         T = tns.T
-        dev = f"cuda:{tns.device}"
-        gq = torch.empty((nq, d), dtype=T, device=dev)
-        gt = torch.empty((nt, d), dtype=T, device=dev)
+        gq = _empty((nq, d), T, tns.device)
+        gt = _empty((nt, d), T, tns.device)
         dd = None if g_disp is None else g_disp.t().contiguous()
         dn = None if g_dist is None else g_dist.reshape(-1).contiguous()
         snd, rcv, disp, dist = ctx.saved_tensors
@@ -729,11 +744,11 @@ def _zsort_rows(tns: TNS, set_id: int, x: torch.Tensor, direction: int) -> torch
         raise DimensionMismatch(f"perm length {n} does not match last axis {x.shape[-1]}")
     if x.dim() == 1:
         xin = x.contiguous()
-        out = torch.empty_like(xin)
+        out = _empty(xin.shape, x.dtype, x.device.index)
         row = xin.element_size()
     else:
         xin = x.t().contiguous()  # (N, F): each point's F values contiguous
-        out = torch.empty((x.shape[1], x.shape[0]), dtype=x.dtype, device=x.device).t()
+        out = _empty((x.shape[1], x.shape[0]), x.dtype, x.device.index).t()
         row = x.shape[0] * xin.element_size()
     if n == 0 or row == 0:
         return out

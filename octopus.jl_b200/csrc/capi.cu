@@ -26,9 +26,14 @@ namespace {
 // stream or thread takes it next finds no work on it; the others are freed,
 // which waits for their work.  Nothing here waits for the whole device: that
 // would invalidate any capture in progress.  At most kPoolBytes are held per
-// device; the rest is freed, everything is when the device's last context is
-// destroyed or an allocation fails.
+// device, and above kPoolSmall nothing is added while less than 1 / kPoolFree of
+// its memory is free (asking costs 70 us, half of a small tree's build); the
+// rest is freed, everything is when the caller asks for it
+// (oct_ctx_release_memory), the device's last context is destroyed or an
+// allocation fails.
 constexpr size_t kPoolBytes = 4ULL << 30;
+constexpr size_t kPoolSmall = 64ULL << 20;
+constexpr size_t kPoolFree = 8;
 constexpr int kPoolDevices = 64;
 
 struct BlockPool {
@@ -64,7 +69,7 @@ cudaError_t block_alloc(size_t least, size_t want, DevBuf& b) {
     if (pool) {
         std::lock_guard<std::mutex> lock(pool->mu);
         const auto it = pool->blocks.lower_bound(least);
-        if (it != pool->blocks.end() && it->first <= 2 * want + 65536) {
+        if (it != pool->blocks.end() && it->first <= want + want / 4 + 65536) {
             b.p = it->second;
             b.bytes = it->first;
             pool->held -= it->first;
@@ -142,6 +147,21 @@ cudaError_t ensure(DevBuf& b, size_t bytes) {
 }
 
 void release(DevBuf& b, bool idle) { block_free(b, idle); }
+
+bool memory_to_spare(size_t bytes) {
+    if (BlockPool* pool = pool_of_current_device()) {
+        std::lock_guard<std::mutex> lock(pool->mu);
+        if (pool->held + bytes <= kPoolSmall) return true;
+    }
+    size_t free = 0, total = 0;
+    if (cudaMemGetInfo(&free, &total) == cudaSuccess) return free >= total / kPoolFree;
+    (void)cudaGetLastError();
+    return false;
+}
+
+void pool_release() {
+    if (BlockPool* pool = pool_of_current_device()) pool->trim();
+}
 
 void pool_context(int delta) {
     BlockPool* pool = pool_of_current_device();
@@ -323,17 +343,19 @@ struct DeviceGuard {
 
 void release_tree(oct::Tree& t, const oct::Ctx* owner) {
     // its buffers may go to another tree, on another stream
-    const bool idle = owner && t.used.wait(owner->stream);
+    bool idle = owner && t.used.wait(owner->stream);
     using oct::release;
     // the caller's own kernels may be reading the views, on any stream
     for (auto* b : {&t.morton, &t.v_first, &t.v_last, &t.v_children, &t.v_bmin, &t.v_bmax, &t.v_perm})
         release(*b, false);
-    for (auto* b : {&t.b_coff, &t.b_cparam, &t.b_cbounds, &t.b_eoff})
-        release(*b, idle);
-    for (auto* b : {&t.keys[0], &t.keys[1], &t.vals[0], &t.vals[1], &t.hist, &t.sort_tmp, &t.look, &t.spts, &t.spts_tmp, &t.tnode, &t.nrange,
+    auto blocks = {&t.b_coff, &t.b_cparam, &t.b_cbounds, &t.b_eoff,
+                    &t.keys[0], &t.keys[1], &t.vals[0], &t.vals[1], &t.hist, &t.sort_tmp, &t.look, &t.spts, &t.spts_tmp, &t.tnode, &t.nrange,
                     &t.link, &t.fchild, &t.arrive, &t.dpts, &t.dstart, &t.dnode, &t.rbox, &t.chunk, &t.bvh, &t.bvh_arrive, &t.lohi, &t.blockcnt, &t.blockoff, &t.scan_tmp, &t.partials, &t.hdr,
-                    &t.iperm, &t.rflag, &t.rcnt, &t.roff, &t.mkeys, &t.mvals, &t.mkeys2, &t.mvals2})
-        release(*b, idle);
+                    &t.iperm, &t.rflag, &t.rcnt, &t.roff, &t.mkeys, &t.mvals, &t.mkeys2, &t.mvals2};
+    size_t bytes = 0;
+    for (auto* b : blocks) bytes += b->bytes;
+    idle = idle && oct::memory_to_spare(bytes);
+    for (auto* b : blocks) release(*b, idle);
     oct::header_free(t.hdr_host, idle);
     t.hdr_host = nullptr;
 }
@@ -397,6 +419,13 @@ OCT_API int oct_ctx_destroy(oct_ctx* ctx) {
     for (auto e : ctx->c.event_pool) cudaEventDestroy(e);
     oct::pool_context(-1);
     delete ctx;
+    return OCT_OK;
+}
+
+OCT_API int oct_ctx_release_memory(oct_ctx* ctx) {
+    if (!ctx) return OCT_ERR_ARGUMENT;
+    DeviceGuard g(ctx->c.device);
+    oct::pool_release();
     return OCT_OK;
 }
 

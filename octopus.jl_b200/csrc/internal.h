@@ -21,6 +21,8 @@ struct DevBuf {
 
 cudaError_t ensure(DevBuf& b, size_t bytes);
 void release(DevBuf& b, bool idle);  // idle: the work that used it is known to be done
+bool memory_to_spare(size_t bytes);  // whether so much more may be kept: the current device is not nearly full
+void pool_release();                 // frees what the current device's pool holds
 // A tree's pinned header block, and the number of contexts on the current
 // device (the device's pool is emptied with the last).
 cudaError_t header_alloc(OctHeader** h);
