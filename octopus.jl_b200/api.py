@@ -802,6 +802,18 @@ def apply_zsort_(tns: TNS, set_id: int, user_array: torch.Tensor) -> torch.Tenso
     return apply_zsort(tns, set_id, user_array)
 
 
+def _cloud_radii(radii, n_clouds: int, T: torch.dtype) -> np.ndarray:
+    """One radius per cloud, rounded to the element type like
+    set_search_radius! (src/api.jl:26)."""
+    radii = np.ascontiguousarray(np.asarray(radii, dtype=np.float64))
+    if len(radii) != n_clouds or n_clouds == 0:
+        raise DimensionMismatch("sizes and radii need one entry per cloud")
+    if radii.size != n_clouds:
+        raise TypeError(f"radii of shape {radii.shape}: each cloud needs a single radius")
+    with np.errstate(over="ignore"):
+        return radii.reshape(-1).astype(np.float32 if T == torch.float32 else np.float64).astype(np.float64)
+
+
 class BatchedSearch:
     """Many independent point clouds searched in one pass (no counterpart in
     the reference, which needs one TNS per radius, src/api.jl:24-29).
@@ -831,12 +843,7 @@ class BatchedSearch:
         if not coords.is_cuda:
             raise ArgumentError("coords must be a CUDA tensor: this backend runs on the GPU only")
         sizes = np.asarray(sizes, dtype=np.int64)
-        radii = np.ascontiguousarray(np.asarray(radii, dtype=np.float64))
-        if len(sizes) != len(radii) or len(sizes) == 0:
-            raise DimensionMismatch("sizes and radii need one entry per cloud")
-        # radii in the element type, like set_search_radius! (src/api.jl:26)
-        with np.errstate(over="ignore"):
-            radii = radii.astype(np.float32 if self.T == torch.float32 else np.float64).astype(np.float64)
+        radii = _cloud_radii(radii, len(sizes), self.T)
         coff = np.zeros(len(sizes) + 1, np.int64)
         coff[1:] = np.cumsum(sizes)
         self.coords = colmajor(coords)
