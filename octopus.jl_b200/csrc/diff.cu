@@ -396,7 +396,8 @@ __global__ void __launch_bounds__(kTwinWarps * 32) k_adjoint_twins(
         }
     }
     double acc[3] = {0.0, 0.0, 0.0};
-    for (int k = sg.x + sub; k < sg.y; k += kTwinLanes) {
+    // (unsigned: with up to 2^31 - 1 edges the step past the last may need bit 31)
+    for (uint32_t k = (uint32_t)sg.x + sub; k < (uint32_t)sg.y; k += kTwinLanes) {
         const int32_t j1 = snd[k];
         if (j1 < 1 || j1 > (int32_t)n) {
             bad |= kAdjBadIndex;
