@@ -380,7 +380,10 @@ __global__ void __launch_bounds__(kTwinWarps * 32) k_adjoint_twins(
     pdl_trigger();
     const int lane = threadIdx.x & 31, sub = lane & (kTwinLanes - 1);
     const int64_t w0 = ((int64_t)blockIdx.x * kTwinWarps + (threadIdx.x >> 5)) * kTwinGroups;
-    if (w0 >= n || (__ldcg(status) & (kAdjUngrouped | kAdjBadIndex))) return;  // warp-uniform
+    // Other blocks set bits while this one starts, so one lane's reading decides
+    // for the warp (its shuffles below need every lane).
+    const int known = __shfl_sync(0xffffffffu, __ldcg(status), 0);
+    if (w0 >= n || (known & (kAdjUngrouped | kAdjBadIndex))) return;  // warp-uniform
     int bad = 0, p = -1;
     int2 sg = make_int2(0, 0);
     {
