@@ -243,12 +243,11 @@ __global__ void __launch_bounds__(kThreads) k_encode(const T* __restrict__ coord
 // ------------------------------------------------------------ 4. gather --
 // A permutation entry outside [0, n) can only come from a sort whose
 // look-back wait ran out (DF_TIMEOUT is then set already): it is skipped, so
-// neither the coordinate read nor the inverse-permutation store leaves its
-// array.
+// that the coordinate read stays inside its array.
 template <class T, int D>
 __global__ void __launch_bounds__(kThreads) k_gather(const T* __restrict__ coords, const int32_t* __restrict__ perm,
                                                      int64_t n, SPt<T, D>* __restrict__ spts,
-                                                     int32_t* __restrict__ iperm, int* __restrict__ status) {
+                                                     int* __restrict__ status) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int32_t j = perm ? perm[k] : (int32_t)k;
@@ -261,7 +260,6 @@ __global__ void __launch_bounds__(kThreads) k_gather(const T* __restrict__ coord
     for (int d = 0; d < D; ++d) p.x[d] = coords[(int64_t)D * j + d];
     p.idx = j;
     spts[k] = p;
-    iperm[j] = (int32_t)k;
 }
 
 // ---------------------------------------------------------- 5. topology --
@@ -1591,22 +1589,26 @@ void guard_check(Ctx& ctx, const DevBuf& b, size_t bytes, OctHeader* hdr) {
 // Bounds, visiting order, chunks and box hierarchy (sections 6 and 7) of the
 // tree whose topology was just launched; `nodes` bounds its node count.
 template <class T, int D>
-void launch_layout(Ctx& ctx, Tree& t, int64_t n, int64_t node_cap, int64_t chunk_cap, int64_t nodes, int gmax,
-                   T inv_r) {
+void launch_layout(Ctx& ctx, Tree& t, const void* skeys, int64_t n, int64_t node_cap, int64_t chunk_cap, int64_t nodes,
+                   int gmax, T inv_r) {
     OctHeader* hdr = t.hdr.as<OctHeader>();
+    // Each run's first leaf, by visiting position, in the key buffer that does
+    // not hold the sorted keys (4 or 8 bytes per point).
+    int32_t* dnode = t.keys[skeys == t.keys[0].p ? 1 : 0].as<int32_t>();
     {
         PhaseTimer pt_(ctx, PH_REFIT);
         // a grid that fills the device; warps take further nodes in turn
         const int64_t blocks = std::min<int64_t>(div_up(nodes, kThreads), 2 * kLayoutWave);
         launch_pdl(k_layout<T, D>, blocks, kThreads, 0, ctx.stream, node_cap, n, t.tnode.as<TNode<T, D>>(),
             t.nrange.as<int2>(), t.link.as<NodeLink>(), t.spts.as<SPt<T, D>>(), t.dpts.as<SPt<T, D>>(),
-            t.dstart.as<uint8_t>(), t.dnode.as<int32_t>(), t.rbox.as<BoxNode<T, D>>(), gmax, inv_r, hdr, t.batch());
+            t.dstart.as<uint8_t>(), dnode, t.rbox.as<BoxNode<T, D>>(), gmax, inv_r, hdr, t.batch());
     }
     PhaseTimer pt_(ctx, PH_GROUPS);
     const int span_blocks = div_up(n, kSpan * kSpansPerBlock);
     const int64_t fold_blocks = std::min<int64_t>(div_up(nodes, kThreads), 148 * 16);
     launch_pdl(k_fold_chunks<T, D>, span_blocks + fold_blocks, kThreads, 0, ctx.stream, span_blocks, n, node_cap,
-        t.tnode.as<TNode<T, D>>(), t.link.as<NodeLink>(), t.arrive.as<int32_t>(), t.dpts.as<SPt<T, D>>(), t.dstart.as<uint8_t>(), t.dnode.as<int32_t>(), t.rbox.as<BoxNode<T, D>>(), chunk_cap,
+        t.tnode.as<TNode<T, D>>(), t.link.as<NodeLink>(), t.arrive.as<int32_t>(), t.dpts.as<SPt<T, D>>(),
+        t.dstart.as<uint8_t>(), dnode, t.rbox.as<BoxNode<T, D>>(), chunk_cap,
         t.search_layout<T, D>(), t.bvh_arrive.as<int32_t>(), inv_r, hdr, t.batch());
     ctx.kernel_launches += 2;
 }
@@ -1622,14 +1624,13 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
     T o[3] = {T(0), T(0), T(0)};
     for (int d = 0; d < D; ++d) o[d] = (T)t.origin[d];
 
-    if ((err = ensure(t.spts, (size_t)n * sizeof(SPt<T, D>))) || (err = ensure(t.iperm, (size_t)n * 4)))
-        return cuda_status(ctx, err, "allocating points");
+    if ((err = ensure(t.spts, (size_t)n * sizeof(SPt<T, D>)))) return cuda_status(ctx, err, "allocating points");
+    t.iperm_valid = false;
     int32_t lev[kBvhLevels];
     int64_t bvh_nodes = 0;
     t.bvh_levels(n, lev, &bvh_nodes);
     const int n_arrive = (int)(bvh_nodes - lev[0]);
-    if ((err = ensure(t.dpts, (size_t)n * sizeof(SPt<T, D>))) || (err = ensure(t.dstart, (size_t)n)) ||
-        (err = ensure(t.dnode, (size_t)n * 4)) ||
+    if ((err = ensure_g(ctx, t.dpts, (size_t)n * sizeof(SPt<T, D>))) || (err = ensure(t.dstart, (size_t)n)) ||
         (err = ensure(t.bvh, (size_t)bvh_nodes * sizeof(BoxNode<T, D>))) ||
         (err = ensure(t.bvh_arrive, (size_t)n_arrive * 4)))
         return cuda_status(ctx, err, "allocating the search layout");
@@ -1643,17 +1644,13 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
         const int passes = t.sort_passes;
         if ((err = ensure_g(ctx, t.keys[0], (size_t)n * sizeof(K))) ||
             (err = ensure_g(ctx, t.keys[1], (size_t)n * sizeof(K))) || (err = ensure_g(ctx, t.vals[0], (size_t)n * 4)) ||
-            (err = ensure_g(ctx, t.spts, (size_t)n * sizeof(SPt<T, D>))) ||
-            (err = ensure_g(ctx, t.spts_tmp, (size_t)n * sizeof(SPt<T, D>))) ||
-            (err = ensure_g(ctx, t.iperm, (size_t)n * 4)) ||
-            (err = ensure(t.vals[1], (size_t)n * 4)))  // the next refit-mode merge writes here
+            (err = ensure_g(ctx, t.spts, (size_t)n * sizeof(SPt<T, D>))))
             return cuda_status(ctx, err, "allocating sort buffers");
         for (int b = 0; b < 2; ++b)
             if ((err = guard_fill(ctx, t.keys[b], (size_t)n * sizeof(K)))) return cuda_status(ctx, err, "sort guards");
         if ((err = guard_fill(ctx, t.vals[0], (size_t)n * 4)) ||
             (err = guard_fill(ctx, t.spts, (size_t)n * sizeof(SPt<T, D>))) ||
-            (err = guard_fill(ctx, t.spts_tmp, (size_t)n * sizeof(SPt<T, D>))) ||
-            (err = guard_fill(ctx, t.iperm, (size_t)n * 4)))
+            (err = guard_fill(ctx, t.dpts, (size_t)n * sizeof(SPt<T, D>))))
             return cuda_status(ctx, err, "sort guards");
         if (passes == 0) {
             // Every point in one cell: keys all equal, the input order stands.
@@ -1661,9 +1658,8 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
             k_encode<T, D, K><<<div_up(n, kThreads), kThreads, 0, s>>>(coords, n, o[0], o[1], o[2], inv_cs,
                                                                         t.keys[0].as<K>(), bt);
             k_gather<T, D><<<div_up(n, kThreads), kThreads, 0, s>>>(coords, nullptr, n, t.spts.as<SPt<T, D>>(),
-                                                                    t.iperm.as<int32_t>(), &hdr->status);
+                                                                    &hdr->status);
             ctx.kernel_launches += 2;
-            t.iperm_valid = true;
             perm = nullptr;
         } else {
             if ((err = ensure(t.look, onesweep_words(n, passes) * 4)))
@@ -1679,11 +1675,10 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
             PhaseTimer pt_(ctx, PH_SORT);
             // the inverse permutation is left to its first user (ensure_iperm)
             err = point_sort<T, D, K>(coords, ep, n, passes, t.keys[0].as<K>(), t.keys[1].as<K>(),
-                                      t.spts.as<SPt<T, D>>(), t.spts_tmp.as<SPt<T, D>>(), t.vals[0].as<int32_t>(),
+                                      t.spts.as<SPt<T, D>>(), t.dpts.as<SPt<T, D>>(), t.vals[0].as<int32_t>(),
                                       nullptr, t.look.as<uint32_t>(), &hdr->status, sms, ctx.wait_limit,
                                       ctx.withhold_tile, s, &ctx.kernel_launches);
             if (err) return cuda_status(ctx, err, "key sort launch");
-            t.iperm_valid = false;
             perm = t.vals[0].as<int32_t>();
             if (!bt.n_clouds) sorted = 0;
         }
@@ -1701,9 +1696,8 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
             {
                 PhaseTimer pt_(ctx, PH_GATHER);
                 k_gather<T, D><<<div_up(n, kThreads), kThreads, 0, s>>>(coords, vp, n, t.spts.as<SPt<T, D>>(),
-                                                                    t.iperm.as<int32_t>(), &hdr->status);
+                                                                    &hdr->status);
                 ctx.kernel_launches += 1;
-                t.iperm_valid = true;
             }
             {
                 PhaseTimer pt_(ctx, PH_REFIT);
@@ -1712,8 +1706,7 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
                     t.bvh_arrive.as<int32_t>(), n_arrive, t.asc_key, hdr);
                 ctx.kernel_launches += 1;
             }
-            // the chunk array's capacity is that of the build that made it
-            launch_layout<T, D>(ctx, t, n, t.capacity, t.n_groups, t.n_nodes, t.group_cap, inv_cs);
+            launch_layout<T, D>(ctx, t, skeys, n, t.capacity, t.chunk_cap, t.n_nodes, t.group_cap, inv_cs);
             if ((err = cudaGetLastError())) return cuda_status(ctx, err, "bounds refit");
             t.last_path = 2;
             t.sorted_buf = sorted;
@@ -1730,7 +1723,8 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
         const int64_t nchunks = div_up(mmax, kChunk);
         int width = 64;
         while (width < mmax && width < kChunk) width <<= 1;
-        if ((err = ensure(t.mkeys2, (size_t)mmax * sizeof(K))) || (err = ensure(t.mvals2, (size_t)mmax * 4)))
+        if ((err = ensure(t.mkeys2, (size_t)mmax * sizeof(K))) || (err = ensure(t.mvals2, (size_t)mmax * 4)) ||
+            (err = ensure(t.vals[1 - prev], (size_t)n * 4)))
             return cuda_status(ctx, err, "allocating changed keys");
         K* mk = t.mkeys.as<K>();
         int32_t* mv = t.mvals.as<int32_t>();
@@ -1751,7 +1745,6 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
                 t.rflag.as<uint8_t>(), t.roff.as<int64_t>(), mk, mv, t.mkeys2.as<K>(), t.mvals2.as<int32_t>(), coords,
                 ok, ov, t.spts.as<SPt<T, D>>());
             ctx.kernel_launches += 1;
-            t.iperm_valid = false;
         }
         skeys = ok;
         perm = ov;
@@ -1759,11 +1752,11 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
         t.last_path = 1;
     }
 
-    // --- topology + refit (retried once with the exact node count on overflow)
+    // --- topology + refit (retried with the exact node or chunk count on overflow)
     const int nblocks = div_up(n, kMarkTile);
     t.n_mark_blocks = nblocks;
     const int64_t nbc = (int64_t)NLEV * nblocks;
-    if ((err = ensure(t.lohi, (size_t)n * 2)) || (err = ensure(t.blockcnt, (size_t)nbc * 4)) ||
+    if ((err = ensure(t.blockcnt, (size_t)nbc * 4)) ||
         (err = ensure(t.blockoff, (size_t)(nbc + 1) * 8)) ||
         (err = ensure(t.scan_tmp, (size_t)scan_tmp_elems(nbc) * 8)))
         return cuda_status(ctx, err, "allocating topology scratch");
@@ -1775,51 +1768,58 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
     // Query points per traversal group (a tuned shape; 32 by default).
     const int gmax = ctx.tuning_for(t.ndims, t.dtype, n, t.nbrs_hint).group_cap;
     t.group_cap = gmax;
-    for (int attempt = 0; attempt < 3; ++attempt) {
+    // Two chunks per gmax points (32: n / 16; uniform, clustered, lattice, line
+    // and sphere sets have n / 20 to n / 32) and one per cloud; a set that has
+    // more is laid out again with its own count.
+    t.chunk_cap = std::max(t.chunk_cap, 2 * n / gmax + t.n_clouds + 64);
+    for (int attempt = 0; attempt < 4; ++attempt) {
         ctx.last_attempts = attempt + 1;
         const int64_t cap = t.capacity;
-        const size_t gcap = (size_t)(cap + n / gmax + 2);
+        const size_t gcap = (size_t)t.chunk_cap;
+        const size_t lohi_at = ((size_t)cap * 4 + 15) / 16 * 16;  // behind the first child ids
+        const size_t rbytes =
+            std::max({(size_t)cap * sizeof(BoxNode<T, D>), (size_t)n * 4, lohi_at + (size_t)n * 2});
         if ((err = ensure_g(ctx, t.tnode, (size_t)cap * sizeof(TNode<T, D>))) ||
             (err = ensure_g(ctx, t.nrange, (size_t)cap * 8)) || (err = ensure_g(ctx, t.link, (size_t)cap * sizeof(NodeLink))) ||
-            (err = ensure_g(ctx, t.arrive, (size_t)cap * 4)) || (err = ensure_g(ctx, t.fchild, (size_t)cap * 4)) ||
+            (err = ensure_g(ctx, t.arrive, (size_t)cap * 4)) ||
             (err = ensure(t.scan_tmp, (size_t)scan_tmp_elems(nbc) * 8)) ||
-            (err = ensure_g(ctx, t.rbox, (size_t)cap * sizeof(BoxNode<T, D>))) ||
+            (err = ensure_g(ctx, t.rbox, rbytes)) ||
             (err = ensure_g(ctx, t.chunk, gcap * sizeof(BoxNode<T, D>))))
             return cuda_status(ctx, err, "allocating node arrays");
         if ((err = guard_fill(ctx, t.tnode, (size_t)cap * sizeof(TNode<T, D>))) ||
             (err = guard_fill(ctx, t.nrange, (size_t)cap * 8)) || (err = guard_fill(ctx, t.link, (size_t)cap * sizeof(NodeLink))) ||
-            (err = guard_fill(ctx, t.arrive, (size_t)cap * 4)) || (err = guard_fill(ctx, t.fchild, (size_t)cap * 4)) ||
-            (err = guard_fill(ctx, t.rbox, (size_t)cap * sizeof(BoxNode<T, D>))) ||
+            (err = guard_fill(ctx, t.arrive, (size_t)cap * 4)) ||
+            (err = guard_fill(ctx, t.rbox, rbytes)) ||
             (err = guard_fill(ctx, t.chunk, gcap * sizeof(BoxNode<T, D>))))
             return cuda_status(ctx, err, "node array guards");
         {
         PhaseTimer pt_(ctx, PH_TOPOLOGY);
-        launch_pdl(k_mark<D, K>, nblocks, kThreads, 0, s, skeys, n, t.lohi.as<uint16_t>(), t.blockcnt.as<int32_t>(),
+        int32_t* fchild = t.rbox.as<int32_t>();
+        uint16_t* lohi = reinterpret_cast<uint16_t*>(t.rbox.as<unsigned char>() + lohi_at);
+        launch_pdl(k_mark<D, K>, nblocks, kThreads, 0, s, skeys, n, lohi, t.blockcnt.as<int32_t>(),
             nblocks, t.dstart.as<uint8_t>(), t.bvh_arrive.as<int32_t>(), n_arrive, hdr, bt);
         ctx.kernel_launches += exclusive_scan_i32_i64(t.blockcnt.as<int32_t>(), t.blockoff.as<int64_t>(), nbc,
                                                       &hdr->n_nodes, t.scan_tmp.as<int64_t>(), s);
-        launch_pdl(k_emit_ids<D>, nblocks, kThreads, 0, s, n, t.lohi.as<uint16_t>(), t.blockoff.as<int64_t>(), nblocks,
-            cap, t.fchild.as<int32_t>(), t.nrange.as<int2>(), t.arrive.as<int32_t>(), hdr, bt);
-        launch_pdl(k_emit_nodes<T, D, K>, div_up(cap, kThreads), kThreads, 0, s, skeys, n, cap, t.fchild.as<int32_t>(),
+        launch_pdl(k_emit_ids<D>, nblocks, kThreads, 0, s, n, lohi, t.blockoff.as<int64_t>(), nblocks,
+            cap, fchild, t.nrange.as<int2>(), t.arrive.as<int32_t>(), hdr, bt);
+        launch_pdl(k_emit_nodes<T, D, K>, div_up(cap, kThreads), kThreads, 0, s, skeys, n, cap, fchild,
             t.tnode.as<TNode<T, D>>(), t.nrange.as<int2>(), t.link.as<NodeLink>(), t.arrive.as<int32_t>(),
             t.blockoff.as<int64_t>(), nblocks, hdr, bt);
         ctx.kernel_launches += 3;
         }
-        launch_layout<T, D>(ctx, t, n, cap, (int64_t)gcap, cap, gmax, inv_cs);
+        launch_layout<T, D>(ctx, t, skeys, n, cap, (int64_t)gcap, cap, gmax, inv_cs);
         if (ctx.guard_check) {
             guard_check(ctx, t.tnode, (size_t)cap * sizeof(TNode<T, D>), hdr);
             guard_check(ctx, t.nrange, (size_t)cap * 8, hdr);
             guard_check(ctx, t.link, (size_t)cap * sizeof(NodeLink), hdr);
             guard_check(ctx, t.arrive, (size_t)cap * 4, hdr);
-            guard_check(ctx, t.fchild, (size_t)cap * 4, hdr);
-            guard_check(ctx, t.rbox, (size_t)cap * sizeof(BoxNode<T, D>), hdr);
+            guard_check(ctx, t.rbox, rbytes, hdr);
             guard_check(ctx, t.chunk, gcap * sizeof(BoxNode<T, D>), hdr);
             if (moved == -1) {
                 for (int b = 0; b < 2; ++b) guard_check(ctx, t.keys[b], (size_t)n * sizeof(K), hdr);
                 guard_check(ctx, t.vals[0], (size_t)n * 4, hdr);
                 guard_check(ctx, t.spts, (size_t)n * sizeof(SPt<T, D>), hdr);
-                guard_check(ctx, t.spts_tmp, (size_t)n * sizeof(SPt<T, D>), hdr);
-                guard_check(ctx, t.iperm, (size_t)n * 4, hdr);
+                guard_check(ctx, t.dpts, (size_t)n * sizeof(SPt<T, D>), hdr);
             }
         }
         if ((err = cudaMemcpyAsync(t.hdr_host, hdr, sizeof(OctHeader), cudaMemcpyDeviceToHost, s)) ||
@@ -1838,6 +1838,10 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
             cudaMemcpyAsync(&hdr->status, &zero, sizeof(int), cudaMemcpyHostToDevice, s);
             continue;
         }
+        if (t.hdr_host->n_groups > t.chunk_cap) {
+            t.chunk_cap = t.hdr_host->n_groups + t.hdr_host->n_groups / 8;
+            continue;
+        }
         t.n_nodes = t.hdr_host->n_nodes;
         t.n_groups = t.hdr_host->n_groups;
         t.asc_key = t.hdr_host->asc_key;
@@ -1847,7 +1851,7 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
         t.key_bytes = (int)sizeof(K);
         return OK;
     }
-    return set_error(ctx, ERR_OVERFLOW, "tree build: node capacity retry did not converge");
+    return set_error(ctx, ERR_OVERFLOW, "tree build: node or chunk capacity retry did not converge");
 }
 
 // Refit mode: re-encodes every point at its previous sorted position and
@@ -2120,11 +2124,10 @@ int build_tree(Ctx& ctx, Tree& t, const void* coords, int64_t n, double radius) 
 }
 
 int ensure_iperm(Ctx& ctx, const Tree& t) {
-    if (t.iperm_valid || t.n == 0) return OK;
-    if (!t.perm_dev) return set_error(ctx, ERR_STATE, "inverse permutation: the tree has no sorted order");
+    if (t.iperm_valid || t.n == 0 || !t.perm_dev) return OK;
     OctHeader* hdr = t.hdr.as<OctHeader>();
     k_inverse_perm<<<(unsigned)div_up(t.n, kSortThreads), kSortThreads, 0, ctx.stream>>>(
-        t.perm_dev, t.n, t.iperm.as<int32_t>(), &hdr->status);
+        t.perm_dev, t.n, t.rbox.as<int32_t>(), &hdr->status);
     ctx.kernel_launches += 1;
     const cudaError_t err = cudaGetLastError();
     if (err) return cuda_status(ctx, err, "inverse permutation launch");

@@ -123,19 +123,15 @@ struct Tree {
     DevBuf sort_tmp;             // int64 tile sums of the histogram scan
     DevBuf look;                 // one-pass-per-digit sort: digit counts and tile look-back words
     DevBuf spts;                 // SPt<T,D>[n] in Morton order
-    DevBuf spts_tmp;             // SPt<T,D>[n]: the key sort's intermediate passes
-    DevBuf iperm;                // int32 [n]: sorted position of each original point
-    // iperm holds the inverse of the current order (a full sort leaves it to
-    // the first caller that needs it: ensure_iperm)
+    // rbox holds the inverse of the current order, the sorted position of each
+    // original point, for the first caller that needs it (ensure_iperm)
     mutable bool iperm_valid = false;
     const int32_t* perm_dev = nullptr;  // original index of each sorted position (null: identity)
     const void* skeys_dev = nullptr;    // sorted keys of the last build (key_bytes wide)
     DevBuf tnode;                // TNode<T,D>[capacity]
     DevBuf nrange;               // int2 {first,last} 0-based per node
     DevBuf link;                 // NodeLink per node: parent, children, for climbing
-    DevBuf fchild;               // int32 per node: first child id from the id pass
     DevBuf arrive;               // int32 per node, refit arrival counters
-    DevBuf lohi;                 // uint16 per position: first | last level starting here
     DevBuf blockcnt;             // int32 [(maxlev+1) * n_mark_blocks]
     DevBuf blockoff;             // int64 exclusive scan of blockcnt (+1)
     DevBuf scan_tmp;             // int64 tile sums for scans
@@ -143,13 +139,18 @@ struct Tree {
     DevBuf hdr;                  // OctHeader
     DevBuf morton;               // uint64 per original point (refit mode), filled with the views
     // Search layout (Bvh): what build_edges reads.
-    DevBuf dpts;                 // SPt<T,D>[n] in the search's visiting order
+    DevBuf dpts;                 // SPt<T,D>[n] in the search's visiting order; before, the key sort's scratch
     DevBuf dstart;               // uint8 per visiting position: point count of the chunk starting there, else 0
-    DevBuf dnode, rbox;          // a run's first leaf (int32, at its start) and its box (BoxNode<T,D> at that leaf)
+    // In turn: the topology's first child ids (int32 per node) and levels per
+    // position (uint16: first | last level starting there); a run's box
+    // (BoxNode<T,D> at its first leaf) until the chunks are made; the inverse
+    // permutation (above).
+    DevBuf rbox;
     DevBuf chunk;                // BoxNode<T,D> per chunk: box, first position, count <= group_cap
     DevBuf bvh;                  // BoxNode<T,D>: the box hierarchy's levels, one after another
     DevBuf bvh_arrive;           // int32 per node above the lowest level: children done
     int64_t n_groups = 0;        // chunks
+    int64_t chunk_cap = 0;       // capacity of the chunk array
     int32_t asc_key = 0;         // OctHeader::asc_key of the last topology
 
     // Refit mode across time steps: the previous build's sorted keys and
@@ -308,8 +309,8 @@ int edges_fill(Ctx& ctx, const Tree& q, const Tree& t, bool exclude_self, int32_
                int32_t* receivers, void* rel_disp, void* rel_dist, int64_t n_edges);
 int edges_fill_diff(Ctx& ctx, const Tree& t, int32_t* senders, int32_t* receivers, void* rel_disp, void* rel_dist,
                     int32_t* mirror, int64_t n_edges);
-// The inverse permutation of a built tree, computed on first use after a
-// full sort (the build itself does not need it).
+// The inverse permutation of a built tree (in rbox), computed on first use
+// after a build, which does not need it.
 int ensure_iperm(Ctx& ctx, const Tree& t);
 int edges_mirror_scan(Ctx& ctx, const int32_t* snd, const int32_t* rcv, int64_t m, int64_t n, const int64_t* off,
                       int32_t* mirror);

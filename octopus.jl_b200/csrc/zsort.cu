@@ -147,7 +147,7 @@ int zsort_apply(Ctx& ctx, const Tree& t, const void* in, void* out, int64_t n, i
         const int st = ensure_iperm(ctx, t);
         if (st != OK) return st;
     }
-    const int32_t* src = direction == 0 ? t.perm_dev : t.iperm.as<int32_t>();
+    const int32_t* src = direction == 0 || !t.perm_dev ? t.perm_dev : t.rbox.as<int32_t>();  // (null: identity)
     const uintptr_t a = (uintptr_t)in | (uintptr_t)out | (uintptr_t)row_bytes;
     if (a % 16 == 0) launch<uint4>(in, out, src, n, row_bytes, ctx.stream);
     else if (a % 8 == 0) launch<uint2>(in, out, src, n, row_bytes, ctx.stream);
