@@ -1673,10 +1673,9 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
             ep.inv_cs = inv_cs;
             ep.bt = bt;
             PhaseTimer pt_(ctx, PH_SORT);
-            // the inverse permutation is left to its first user (ensure_iperm)
             err = point_sort<T, D, K>(coords, ep, n, passes, t.keys[0].as<K>(), t.keys[1].as<K>(),
                                       t.spts.as<SPt<T, D>>(), t.dpts.as<SPt<T, D>>(), t.vals[0].as<int32_t>(),
-                                      nullptr, t.look.as<uint32_t>(), &hdr->status, sms, ctx.wait_limit,
+                                      t.look.as<uint32_t>(), &hdr->status, sms, ctx.wait_limit,
                                       ctx.withhold_tile, s, &ctx.kernel_launches);
             if (err) return cuda_status(ctx, err, "key sort launch");
             perm = t.vals[0].as<int32_t>();

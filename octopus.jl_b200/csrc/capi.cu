@@ -349,7 +349,7 @@ void release_tree(oct::Tree& t, const oct::Ctx* owner) {
     for (auto* b : {&t.morton, &t.v_first, &t.v_last, &t.v_children, &t.v_bmin, &t.v_bmax, &t.v_perm})
         release(*b, false);
     auto blocks = {&t.b_coff, &t.b_cparam, &t.b_cbounds, &t.b_eoff,
-                    &t.keys[0], &t.keys[1], &t.vals[0], &t.vals[1], &t.hist, &t.sort_tmp, &t.look, &t.spts, &t.tnode, &t.nrange,
+                    &t.keys[0], &t.keys[1], &t.vals[0], &t.vals[1], &t.look, &t.spts, &t.tnode, &t.nrange,
                     &t.link, &t.arrive, &t.dpts, &t.dstart, &t.rbox, &t.chunk, &t.bvh, &t.bvh_arrive, &t.blockcnt, &t.blockoff, &t.scan_tmp, &t.partials, &t.hdr,
                     &t.rflag, &t.rcnt, &t.roff, &t.mkeys, &t.mvals, &t.mkeys2, &t.mvals2};
     size_t bytes = 0;

@@ -119,8 +119,6 @@ struct Tree {
 
     // Device storage.
     DevBuf keys[2], vals[2];     // radix-sort ping-pong
-    DevBuf hist;                 // radix digit histograms (+1 total slot)
-    DevBuf sort_tmp;             // int64 tile sums of the histogram scan
     DevBuf look;                 // one-pass-per-digit sort: digit counts and tile look-back words
     DevBuf spts;                 // SPt<T,D>[n] in Morton order
     // rbox holds the inverse of the current order, the sorted position of each

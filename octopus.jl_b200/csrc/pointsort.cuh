@@ -17,8 +17,8 @@
 //                   contiguously.  The first pass encodes from the coordinates;
 //                   the last writes the sorted keys, the sorted points and the
 //                   permutation;
-//   k_inverse_perm  the inverse permutation (when asked for; the build
-//                   leaves it to the first caller that needs it).
+//   k_inverse_perm  the inverse permutation, launched by the first caller that
+//                   needs it after a build.
 //
 // Every wait is bounded (spin_limit polling rounds); one that runs out sets
 // DF_TIMEOUT, and every store still stays inside its array.
@@ -202,8 +202,7 @@ constexpr size_t point_pass_smem() { return sizeof(PointPassSmem<T, D, K, FIRST>
 template <class T, int D, class K, bool FIRST, bool LAST>
 __global__ void __launch_bounds__(kSortThreads) k_point_pass(
     const T* __restrict__ coords, EncodeParams<T> ep, const K* __restrict__ kin, const SPt<T, D>* __restrict__ pin,
-    K* __restrict__ kout, SPt<T, D>* __restrict__ pout, int32_t* __restrict__ perm, int32_t* __restrict__ iperm,
-    int64_t n, int pass, int ntiles, uint32_t* __restrict__ scratch, int* __restrict__ status, int64_t spin_limit,
+    K* __restrict__ kout, SPt<T, D>* __restrict__ pout, int32_t* __restrict__ perm, int64_t n, int pass, int ntiles, uint32_t* __restrict__ scratch, int* __restrict__ status, int64_t spin_limit,
     int withhold_tile) {
     pdl_wait();
     pdl_trigger();
@@ -381,8 +380,8 @@ __global__ void __launch_bounds__(kSortThreads) k_inverse_perm(const int32_t* __
 
 template <class T, int D, class K, bool FIRST, bool LAST>
 cudaError_t launch_point_pass(const T* coords, const EncodeParams<T>& ep, const K* kin, const SPt<T, D>* pin, K* kout,
-                              SPt<T, D>* pout, int32_t* perm, int32_t* iperm, int64_t n, int pass, int ntiles,
-                              uint32_t* scratch, int* status, int64_t spin_limit, int withhold, cudaStream_t s) {
+                              SPt<T, D>* pout, int32_t* perm, int64_t n, int pass, int ntiles, uint32_t* scratch,
+                              int* status, int64_t spin_limit, int withhold, cudaStream_t s) {
     constexpr size_t smem = point_pass_smem<T, D, K, FIRST>();
     auto kern = k_point_pass<T, D, K, FIRST, LAST>;
     static bool attr_set = false;  // per instantiation
@@ -391,20 +390,19 @@ cudaError_t launch_point_pass(const T* coords, const EncodeParams<T>& ep, const 
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
-    launch_pdl(kern, ntiles, kSortThreads, smem, s, coords, ep, kin, pin, kout, pout, perm, iperm, n, pass, ntiles,
+    launch_pdl(kern, ntiles, kSortThreads, smem, s, coords, ep, kin, pin, kout, pout, perm, n, pass, ntiles,
         scratch, status, spin_limit, withhold);
     return cudaGetLastError();
 }
 
 // Sorts the n points of `coords` by Morton key (passes 8-bit digits, 1..8):
-// on return keys_out holds the sorted keys, spts the sorted points, perm the
-// original index of each sorted position and iperm its inverse.  kt and ptmp
-// are scratch of n keys / points (used when passes > 1); `scratch` holds
-// onesweep_words(n, kOnesweepMaxPasses) words.  Launches 1 + passes kernels,
-// plus k_inverse_perm when iperm is not null.
+// on return keys_out holds the sorted keys, spts the sorted points and perm the
+// original index of each sorted position.  kt and ptmp are scratch of n keys /
+// points (used when passes > 1); `scratch` holds onesweep_words(n,
+// kOnesweepMaxPasses) words.  Launches 1 + passes kernels.
 template <class T, int D, class K>
 cudaError_t point_sort(const T* coords, const EncodeParams<T>& ep, int64_t n, int passes, K* keys_out, K* kt,
-                       SPt<T, D>* spts, SPt<T, D>* ptmp, int32_t* perm, int32_t* iperm, uint32_t* scratch, int* status,
+                       SPt<T, D>* spts, SPt<T, D>* ptmp, int32_t* perm, uint32_t* scratch, int* status,
                        int sms, int64_t spin_limit, int withhold, cudaStream_t s, int64_t* launches) {
     const int ntiles = sort_tiles(n);
     cudaError_t e = cudaMemsetAsync(scratch, 0, onesweep_words(n, passes) * 4, s);
@@ -418,27 +416,22 @@ cudaError_t point_sort(const T* coords, const EncodeParams<T>& ep, int64_t n, in
     auto kb = [&](int p) { return ((passes - 1 - p) & 1) == 0 ? keys_out : kt; };
     auto pb = [&](int p) { return ((passes - 1 - p) & 1) == 0 ? spts : ptmp; };
     if (passes == 1) {
-        if ((e = launch_point_pass<T, D, K, true, true>(coords, ep, nullptr, nullptr, keys_out, spts, perm, iperm, n, 0,
+        if ((e = launch_point_pass<T, D, K, true, true>(coords, ep, nullptr, nullptr, keys_out, spts, perm, n, 0,
                                                         ntiles, scratch, status, spin_limit, withhold, s)))
             return e;
     } else {
-        if ((e = launch_point_pass<T, D, K, true, false>(coords, ep, nullptr, nullptr, kb(0), pb(0), nullptr, nullptr,
-                                                         n, 0, ntiles, scratch, status, spin_limit, withhold, s)))
+        if ((e = launch_point_pass<T, D, K, true, false>(coords, ep, nullptr, nullptr, kb(0), pb(0), nullptr, n, 0,
+                                                         ntiles, scratch, status, spin_limit, withhold, s)))
             return e;
         for (int p = 1; p < passes - 1; ++p)
             if ((e = launch_point_pass<T, D, K, false, false>(coords, ep, kb(p - 1), pb(p - 1), kb(p), pb(p), nullptr,
-                                                              nullptr, n, p, ntiles, scratch, status, spin_limit,
+                                                              n, p, ntiles, scratch, status, spin_limit,
                                                               withhold, s)))
                 return e;
         if ((e = launch_point_pass<T, D, K, false, true>(coords, ep, kb(passes - 2), pb(passes - 2), keys_out, spts,
-                                                         perm, iperm, n, passes - 1, ntiles, scratch, status,
+                                                         perm, n, passes - 1, ntiles, scratch, status,
                                                          spin_limit, withhold, s)))
             return e;
-    }
-    if (iperm) {
-        launch_pdl(k_inverse_perm, (unsigned)((n + kSortThreads - 1) / kSortThreads), kSortThreads, 0, s, perm, n,
-            iperm, status);
-        *launches += 1;
     }
     return cudaGetLastError();
 }
