@@ -1644,7 +1644,8 @@ int run_pipeline(Ctx& ctx, Tree& t, const T* coords, int64_t n, T radius, int64_
         const int passes = t.sort_passes;
         if ((err = ensure_g(ctx, t.keys[0], (size_t)n * sizeof(K))) ||
             (err = ensure_g(ctx, t.keys[1], (size_t)n * sizeof(K))) || (err = ensure_g(ctx, t.vals[0], (size_t)n * 4)) ||
-            (err = ensure_g(ctx, t.spts, (size_t)n * sizeof(SPt<T, D>))))
+            (err = ensure_g(ctx, t.spts, (size_t)n * sizeof(SPt<T, D>))) ||
+            (t.keep_morton && (err = ensure(t.vals[1], (size_t)n * 4))))  // the next step's merge writes here
             return cuda_status(ctx, err, "allocating sort buffers");
         for (int b = 0; b < 2; ++b)
             if ((err = guard_fill(ctx, t.keys[b], (size_t)n * sizeof(K)))) return cuda_status(ctx, err, "sort guards");

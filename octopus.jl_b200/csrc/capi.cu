@@ -1,5 +1,6 @@
 // C ABI (include/octopus_b200.h): argument checks, object lifetime and error
 // reporting around the build / edge / adjoint pipelines.
+#include <chrono>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -26,20 +27,24 @@ namespace {
 // stream or thread takes it next finds no work on it; the others are freed,
 // which waits for their work.  Nothing here waits for the whole device: that
 // would invalidate any capture in progress.  At most kPoolBytes are held per
-// device, and above kPoolSmall nothing is added while less than 1 / kPoolFree of
-// its memory is free (asking costs 70 us, half of a small tree's build); the
-// rest is freed, everything is when the caller asks for it
-// (oct_ctx_release_memory), the device's last context is destroyed or an
-// allocation fails.
+// device, and no more than kPoolSmall while less than 1 / kPoolFree of its memory
+// is free.  Asking for that costs 70 us, half of a small tree's build, so an
+// answer holds for kPoolAsk and for as much as it was asked for.  The rest is
+// freed, everything is when the caller asks for it (oct_ctx_release_memory), the
+// device is found nearly full, its last context is destroyed or an allocation
+// fails.
 constexpr size_t kPoolBytes = 4ULL << 30;
 constexpr size_t kPoolSmall = 64ULL << 20;
 constexpr size_t kPoolFree = 8;
+constexpr std::chrono::milliseconds kPoolAsk{100};
 constexpr int kPoolDevices = 64;
 
 struct BlockPool {
     std::mutex mu;
     std::multimap<size_t, void*> blocks;
     size_t held = 0;
+    size_t spare = 0;  // as much could be held when the device was last asked
+    std::chrono::steady_clock::time_point asked{};
     int contexts = 0;
     std::vector<void*> headers;  // pinned host blocks of kHeaderBytes
 
@@ -48,7 +53,7 @@ struct BlockPool {
         {
             std::lock_guard<std::mutex> lock(mu);
             gone.swap(blocks);
-            held = 0;
+            held = spare = 0;
         }
         for (auto& kv : gone) cudaFree(kv.second);
     }
@@ -149,13 +154,23 @@ cudaError_t ensure(DevBuf& b, size_t bytes) {
 void release(DevBuf& b, bool idle) { block_free(b, idle); }
 
 bool memory_to_spare(size_t bytes) {
-    if (BlockPool* pool = pool_of_current_device()) {
+    BlockPool* pool = pool_of_current_device();
+    if (!pool) return false;
+    const auto now = std::chrono::steady_clock::now();
+    {
         std::lock_guard<std::mutex> lock(pool->mu);
-        if (pool->held + bytes <= kPoolSmall) return true;
+        bytes += pool->held;
+        if (bytes <= kPoolSmall || (bytes <= pool->spare && now - pool->asked < kPoolAsk)) return true;
     }
     size_t free = 0, total = 0;
-    if (cudaMemGetInfo(&free, &total) == cudaSuccess) return free >= total / kPoolFree;
+    if (cudaMemGetInfo(&free, &total) == cudaSuccess && free >= total / kPoolFree) {
+        std::lock_guard<std::mutex> lock(pool->mu);
+        pool->spare = bytes;
+        pool->asked = now;
+        return true;
+    }
     (void)cudaGetLastError();
+    pool->trim();
     return false;
 }
 
