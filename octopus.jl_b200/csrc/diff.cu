@@ -151,7 +151,7 @@ constexpr int kAdjBadOrder = 8;     // an entry of the processing order outside 
 // run of receivers starts and ends (points without edges keep the zeros the
 // caller put there), and the check that the receivers are in 1..n and
 // ascending.  Four receivers per thread.  Bound by DRAM: 4 bytes per edge in, 8
-// per point out (28.6 M edges of 2M points: 24 us; one binary search of the
+// per point out (28.6 M edges of 2M points: 42 us; one binary search of the
 // receivers per point took 69, and 10 to pair the starts).
 constexpr int kSegRun = 4;
 __global__ void __launch_bounds__(256) k_segments(const int32_t* __restrict__ rcv, int64_t m, int64_t n,

@@ -311,7 +311,7 @@ __device__ __forceinline__ unsigned pairs_fast(const double (*sx)[32], unsigned 
 // k_edges over the tree with an exact test per pair executed 100 M warp
 // instructions, this one 64 M).  Count, before and after: 1M lattice points
 // 313 -> 258 us, 2M uniform points at 14 neighbors 792 -> 663, 1M clustered 2D
-// points at 151 neighbors 373 -> 298, 200,003 Float64 points 152 -> 138, 250,007
+// points at 151 neighbors 373 -> 298, 200,003 Float64 points 152 -> 147, 250,007
 // queries against 1M points 329 -> 255.  Not faster: loading the next chunk's
 // points while this one is tested (72 registers), spans of 256 or 1024
 // positions, two or eight warps per block, two chunks of queries per warp.
@@ -717,7 +717,7 @@ __device__ __forceinline__ int kth_set_bit(unsigned m, int k) {
 // of an overflowed group (record count kOverflowMark) are left to the walking
 // fill.
 //
-// Bound by L1 (72% on a 343,000-point lattice: the gathered targets and the
+// Bound by L1 (76% on a 343,000-point lattice: the gathered targets and the
 // strided columns) and instruction issue (68%), at 3.5 to 3.8 TB/s of COO.
 // Against windows that start and end with each batch of 32 records, with the
 // query's data by shuffles and one store per value: 1M lattice points 225 ->

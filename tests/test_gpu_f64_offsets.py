@@ -91,3 +91,34 @@ def test_sets_many_radii_wide(ob, oracle_mod, log2_width):
         ob.run_(pair)
         want = oracle_mod.build_edges(oracle_mod.build_tree(x, r), q, exclude_self=False)
         assert_edges_equal(ob.build_edges(pair, iq, it), want)
+
+
+def test_time_steps_far_from_the_origin(ob, oracle_mod):
+    """Refit-mode steps (a sort, merges that do not wait for the bounds, unchanged
+    keys) whose extremes move, so that the units' origin differs between the
+    steps; the kernels derive it on the device, the search from the host's copy."""
+    rng = np.random.default_rng(1430)
+    x = points(8000, 3, 1431) + 3e6
+    r = np.float64(1 / 16)
+    tns = ob.TNS(torch.float64, 3)
+    ob.set_search_radius_(tns, r)
+    ob.set_refit_mode_(tns, True)
+    sid = ob.add_point_set_(tns, torch.from_numpy(x).cuda().t())
+    ob.set_active_search_(tns, sid, sid)
+    paths = []
+    for step in range(7):
+        if step:
+            x = x.copy()
+            if step == 4:
+                x[5] = x[5]  # nothing moves
+            else:
+                move = rng.choice(len(x), 150, replace=False)
+                x[move] += 0.02 * rng.standard_normal((150, 3))
+            if step == 5:
+                x[x[:, 0].argmin(), 0] -= 1e-4  # the origin, by less than a cell
+            ob.update_point_set_(tns, sid, torch.from_numpy(x).cuda().t())
+        ob.run_(tns)
+        paths.append(tns.trees[0].last_build()[0])
+        want = oracle_mod.build_edges(oracle_mod.build_tree(x, r), x, exclude_self=True)
+        assert_edges_equal(ob.build_edges(tns, sid, sid), want)
+    assert paths[0] == 0 and 1 in paths and paths[4] == 2
